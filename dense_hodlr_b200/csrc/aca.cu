@@ -31,6 +31,7 @@
 // are either all of size L.G (CTA c works on block c / G) or, with a CTA
 // table, of per-block size B.G starting at CTA B.g0 (sized from predicted
 // ranks so that a level's blocks finish together).
+#include "aca_post.cuh"
 #include "common.cuh"
 #include "hodlr_internal.h"
 
@@ -284,262 +285,6 @@ __device__ void residual_pass(const AcaLaunch& L, const AcaBlock& B, T* P, int l
   }
 }
 
-// ---------------------------------------------------------------- bulk-copy rings
-// With streaming on, the group levels run 16 warps per CTA, and every warp
-// streams its own contiguous part of the CTA's slice through a private ring
-// of WR_S stages in shared memory, each WR_BC panel columns x WR_ROWS rows,
-// filled by cp.async.bulk copies (one per column) that complete on the
-// stage's mbarrier.  Lane 0 refills a stage as soon as its own warp is done
-// with it: no warp waits for another.  Rows start on an even global index so
-// that every copy is 16-byte aligned (requires an even N).
-constexpr int WR_NT = 512, WR_E = 4, WR_ROWS = 32 * WR_E;
-constexpr int WR_BC = 4, WR_SMAX = 3;
-constexpr int WR_NW = WR_NT / 32;
-// ring bytes of one CTA with `stages` stages (192 KB with 3)
-constexpr size_t wring_bytes(int stages) {
-  return sizeof(double) * (size_t)WR_NW * stages * WR_BC * WR_ROWS;
-}
-
-struct WRing {
-  // [warp][stage][column u][row], WR_ROWS rows per column: a warp's stages
-  // are `stages` apart (wring_bytes(stages) in all), not WR_SMAX
-  double* buf;
-  uint64_t* full;   // [warp][stage]: the stage's copies landed (1 arrival + bytes)
-  int stages;
-  uint32_t t;       // tiles this warp has consumed (the same in all its lanes)
-};
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait on an mbarrier phase.  On giving up it raises DEV_ERR_TIMEOUT
-// and returns; once the error word is set, later waits give up at once, so a
-// failed launch ends quickly (its next group barrier fails).
-__device__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity, unsigned* err) {
-  for (uint32_t polls = 0;; ++polls) {
-    if (mbar_try(bar, parity)) return;
-    if (polls >= (1u << 20) || (polls >= 64 && *(volatile unsigned*)err)) {
-      atomicOr(err, DEV_ERR_TIMEOUT);
-      return;
-    }
-    if (polls >= 64) __nanosleep(64);
-  }
-}
-
-// Lane 0: this warp's tile number tw into its stage tw % stages -- `nc`
-// columns from l0 of P, `count` rows from row0 (count even, row0 on an even
-// global row).  The stage was last read by this warp before a __syncwarp;
-// the proxy fence orders those reads before the copies overwrite it.
-__device__ void wring_issue(WRing& R, int w, uint32_t tw, const double* P, int64_t ld, int row0,
-                            int count, int l0, int nc) {
-  const int slot = (int)(tw % (uint32_t)R.stages);
-  uint64_t* bar = R.full + w * WR_SMAX + slot;
-  const uint32_t bytes = (uint32_t)count * (uint32_t)sizeof(double);
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-               "r"(bytes * (uint32_t)nc)
-               : "memory");
-  double* dst = R.buf + ((size_t)(w * R.stages + slot) * WR_BC) * WR_ROWS;
-  for (int u = 0; u < nc; ++u)
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-            "r"(smem_addr(dst + u * WR_ROWS)),
-        "l"(P + row0 + (int64_t)(l0 + u) * ld), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
-
-// Lane 0: the same tile as wring_issue, as one 2D tensor copy of the whole
-// box (WR_ROWS rows from arena row x, WR_BC columns from column y).  Rows or
-// columns past the slice land in the stage unread (the consumer masks them);
-// past the arena they are zero-filled, and the transaction always counts the
-// full box.  x is even by construction (16-byte aligned start) and every
-// stage starts on a 128-byte boundary (the ring heads dynamic shared memory,
-// stages are 4 KB); a copy breaking either rule would be invalid, so it is
-// refused: the stage completes without data and the launch reports
-// DEV_ERR_INDEX.
-__device__ void wring_issue_tile(WRing& R, int w, uint32_t tw, const CUtensorMap* map, int x,
-                                 int y, unsigned* err) {
-  const int slot = (int)(tw % (uint32_t)R.stages);
-  uint64_t* bar = R.full + w * WR_SMAX + slot;
-  double* dst = R.buf + ((size_t)(w * R.stages + slot) * WR_BC) * WR_ROWS;
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  if ((x & 1) || (smem_addr(dst) & 127u)) {
-    atomicOr(err, DEV_ERR_INDEX);
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-    return;
-  }
-  constexpr uint32_t bytes = (uint32_t)(sizeof(double) * WR_ROWS * WR_BC);
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_addr(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_addr(bar))
-      : "memory");
-}
-
-// Lane 0, before the CTA exits: every copy this warp issued has landed.
-// In normal flow each issued tile was waited for; a wait that gave up (an
-// error raised elsewhere in the launch) can leave copies in flight, and the
-// CTA's shared memory must not be released under them.  A stage's tiles
-// complete in issue order, so waiting for the last tile of each stage (the
-// last `stages` tiles) suffices; each wait is bounded.
-__device__ void wring_drain(const WRing& R, int w) {
-  const uint32_t t0 = R.t > (uint32_t)R.stages ? R.t - (uint32_t)R.stages : 0u;
-  for (uint32_t tw = t0; tw < R.t; ++tw) {
-    uint64_t* bar = R.full + w * WR_SMAX + (int)(tw % (uint32_t)R.stages);
-    const uint32_t parity = (tw / (uint32_t)R.stages) & 1u;
-    for (uint32_t polls = 0; polls < (1u << 20) && !mbar_try(bar, parity); ++polls)
-      __nanosleep(64);
-  }
-}
-
-// residual_pass with every warp streaming its own rows through its ring.
-// gbase: the global row of P[0] (the block's first column for V, first row
-// for W).  The same arithmetic as residual_pass, element for element: the
-// residual sums in l order with separately rounded products and sums, the
-// argmax in increasing index per thread; the fused dots add their partials
-// in a GPU order, as there.
-template <int NT, int E, bool ROW>
-__device__ void residual_pass_wring(const AcaLaunch& L, const AcaBlock& B, double* P, int lo,
-                                    int hi, int k, const double* __restrict__ coef, bool dots,
-                                    double* __restrict__ dotw, int ldd, int fixed,
-                                    const double* xfix, double scale, const unsigned char* chosen,
-                                    double& bv, int& bi, int& cand, double& sq, bool& nonfinite,
-                                    const EntrySrc& S, WRing& R, int gbase) {
-  static_assert(NT == WR_NT && E == WR_E, "the warp ring's geometry");
-  constexpr int NW = NT / 32;
-  const int64_t ld = L.ld;
-  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  const double minPiv = L.minPivot;
-  const int kd = dots ? k - 1 : 0;
-  // this warp's rows: an even-sized share of the slice from an even global row
-  const int x0 = lo - ((gbase + lo) & 1);
-  int rw = (hi - x0 + NW - 1) / NW;
-  rw = (rw + 1) & ~1;
-  const int wlo = x0 + w * rw, whi = min(hi, wlo + rw);
-  if (lo >= hi || wlo >= whi) {  // no rows: zero partial dots from this warp
-    if (dots)
-      for (int l = lane; l < kd; l += 32) dotw[w * ldd + l] = 0.0;
-    return;
-  }
-  const int tpc = (k + WR_BC - 1) / WR_BC;  // tiles per chunk
-  if (lane == 0) {
-    // this warp's earlier generic stores to these rows, then the copies
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-  }
-  const CUtensorMap* map = ROW ? &L.map_v : &L.map_w;  // the arena P lies in (ring_tile)
-  bool first = true;
-  for (int jb = wlo; jb < whi; jb += WR_ROWS, first = false) {
-    const int count = (min(WR_ROWS, whi - jb) + 1) & ~1;
-    // lane 0: tile q of this chunk into the warp's stage for tile number tw
-    auto issue = [&](uint32_t tw, int q) {
-      if (L.ring_tile)
-        wring_issue_tile(R, w, tw, map, gbase + jb, q * WR_BC, L.err);
-      else
-        wring_issue(R, w, tw, P, ld, jb, count, q * WR_BC, min(WR_BC, k - q * WR_BC));
-    };
-    if (lane == 0)
-      for (int q = 0; q < tpc && q < R.stages; ++q) issue(R.t + q, q);
-    int jj[E];
-    bool ok[E];
-    double s[E], vp[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      jj[e] = jb + lane + 32 * e;
-      ok[e] = jj[e] >= lo && jj[e] < whi;
-      s[e] = 0.0;
-      vp[e] = (dots && ok[e]) ? P[jj[e] + (int64_t)(k - 1) * ld] : 0.0;
-    }
-    for (int q = 0; q < tpc; ++q) {
-      const uint32_t tw = R.t + q;
-      const int slot = (int)(tw % (uint32_t)R.stages);
-      mbar_wait_bounded(R.full + w * WR_SMAX + slot, (tw / (uint32_t)R.stages) & 1, L.err);
-      const double* tile = R.buf + ((size_t)(w * R.stages + slot) * WR_BC) * WR_ROWS;
-      const int l0 = q * WR_BC, nc = min(WR_BC, k - l0);
-      double v[WR_BC][E];
-#pragma unroll
-      for (int u = 0; u < WR_BC; ++u)
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-          v[u][e] = (u < nc && ok[e]) ? tile[u * WR_ROWS + lane + 32 * e] : 0.0;
-#pragma unroll
-      for (int u = 0; u < WR_BC; ++u) {
-        if (u >= nc) break;
-        const double cf = coef[l0 + u];
-#pragma unroll
-        for (int e = 0; e < E; ++e) s[e] = __dadd_rn(s[e], __dmul_rn(cf, v[u][e]));
-      }
-      if (dots && l0 < kd) {
-        // the tile's four column dots over the warp in one transposed
-        // reduction: after the exchanges at offsets 16 and 8, lane group
-        // q = lane / 8 holds partial sums of column q, then each group of 8
-        // lanes sums its own (6 shuffles instead of 4 x 5)
-        static_assert(WR_BC == 4, "transposed reduction of four columns");
-        double d[WR_BC];
-#pragma unroll
-        for (int u = 0; u < WR_BC; ++u) {
-          d[u] = 0.0;
-#pragma unroll
-          for (int e = 0; e < E; ++e) d[u] = fma(v[u][e], vp[e], d[u]);
-        }
-        const bool hi16 = (lane & 16) != 0, hi8 = (lane & 8) != 0;
-        const double s0 = __shfl_xor_sync(0xffffffffu, hi16 ? d[0] : d[2], 16);
-        const double s1 = __shfl_xor_sync(0xffffffffu, hi16 ? d[1] : d[3], 16);
-        const double p0 = (hi16 ? d[2] : d[0]) + s0;
-        const double p1 = (hi16 ? d[3] : d[1]) + s1;
-        const double s2 = __shfl_xor_sync(0xffffffffu, hi8 ? p0 : p1, 8);
-        double t = (hi8 ? p1 : p0) + s2;
-        t += __shfl_xor_sync(0xffffffffu, t, 4);
-        t += __shfl_xor_sync(0xffffffffu, t, 2);
-        t += __shfl_xor_sync(0xffffffffu, t, 1);
-        const int u = (hi16 ? 2 : 0) + (hi8 ? 1 : 0);  // the column this lane group summed
-        if ((lane & 7) == 0 && l0 + u < kd) {
-          if (first)
-            dotw[w * ldd + l0 + u] = t;
-          else
-            dotw[w * ldd + l0 + u] += t;
-        }
-      }
-      __syncwarp();
-      if (lane == 0 && q + R.stages < tpc) issue(tw + R.stages, q + R.stages);
-    }
-    R.t += tpc;
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      if (!ok[e]) continue;
-      const int j = jj[e];
-      double ent = ROW ? src_entry_xi(S, xfix, fixed, B.c0 + j)
-                       : src_entry_xj(S, xfix, B.r0 + j, fixed);
-      double r = __dsub_rn(ent, s[e]);
-      const double stored = ROW ? r : __dmul_rn(scale, r);
-      P[j + (int64_t)k * ld] = stored;
-      sq = fma(stored, stored, sq);
-      double a = fabs(r);
-      nonfinite |= !isfinite(r);
-      if (a > bv) {
-        bv = a;
-        bi = j;
-      }
-      if (cand == INT_MAX && a > minPiv && __ldcg(chosen + j) == 0) cand = j;
-    }
-  }
-}
-
 // Partial dots of step k-1 over this CTA's slices when they could not be
 // fused into a residual pass (a zero residual row, or the capacity limit).
 template <int NT, typename T>
@@ -585,16 +330,11 @@ __device__ double resolve_eps(Shared& sh, const AcaLaunch& L, const AcaBlock& B,
   return sqrt(swp) * sqrt(svp) / sqrt(frob2);
 }
 
-// RING: the residual passes stream their panel slices through the warps'
-// bulk-copy rings (group levels of an even N, 512 threads); the dynamic
-// shared memory then starts with the rings' wring_bytes(L.ring_stages).
 // T: the element type of the W/V panels (double).
-template <int NT, int E, bool RING, typename T>
-__global__ void __launch_bounds__(NT, (NT == 512 ? 1 : NT == 256 ? 2 : 4)) aca_kernel(const __grid_constant__ AcaLaunch L) {
-  extern __shared__ __align__(128) double dyn_all[];
+template <int NT, int E, typename T>
+__global__ void __launch_bounds__(NT, (NT == 256 ? 2 : 4)) aca_kernel(const __grid_constant__ AcaLaunch L) {
+  extern __shared__ __align__(128) double dyn[];
   __shared__ Shared sh;
-  __shared__ __align__(8) uint64_t ring_full[RING ? WR_NW * WR_SMAX : 1];
-  double* dyn = RING ? dyn_all + wring_bytes(L.ring_stages) / sizeof(double) : dyn_all;
   // dyn: row[kcap], then (unless L.dotg) per-warp dots[NT/32][kcap]
   constexpr int NW = NT / 32;
   const int b = L.cta_block ? (blockIdx.x < (unsigned)L.ncta ? L.cta_block[blockIdx.x] : L.nblocks)
@@ -633,15 +373,6 @@ __global__ void __launch_bounds__(NT, (NT == 512 ? 1 : NT == 256 ? 2 : 4)) aca_k
   double swp = st->swp, svp = st->svp;
   int near = st->near, pending = st->pending;
   bool nonfinite = false;
-  WRing ring{dyn_all, ring_full, L.ring_stages, 0};
-  if (RING) {
-    if (tid == 0) {
-      for (int q = 0; q < WR_NW * WR_SMAX; ++q)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&ring_full[q])));
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-  }
 
   const int minR = B.minRank, maxR = B.maxRank;  // -1: none (src/lowRank.cpp:149,244-247)
   if (status == ACA_RUNNING && k == 0 && maxR == 0) status = ACA_POST;  // zero columns, rank 1
@@ -692,11 +423,7 @@ __global__ void __launch_bounds__(NT, (NT == 512 ? 1 : NT == 256 ? 2 : 4)) aca_k
     }
     double bv = -1.0, sv = 0.0;
     int bi = INT_MAX, cand = INT_MAX;
-    if constexpr (RING)
-      residual_pass_wring<NT, E, true>(L, B, BV, j_lo, j_hi, k, row, fuse, dotw, ldd, gi, xi,
-                                       1.0, B.cC, bv, bi, cand, sv, nonfinite, S, ring, B.c0);
-    else
-      residual_pass<NT, E, true>(L, B, BV, j_lo, j_hi, k, row, fuse, dotw, ldd, gi, xi, 1.0,
+    residual_pass<NT, E, true>(L, B, BV, j_lo, j_hi, k, row, fuse, dotw, ldd, gi, xi, 1.0,
                                  B.cC, bv, bi, cand, sv, nonfinite, S);
     __syncthreads();
     if (fuse)  // CTA partial dots of V, warps summed in order
@@ -770,11 +497,7 @@ __global__ void __launch_bounds__(NT, (NT == 512 ? 1 : NT == 256 ? 2 : 4)) aca_k
     bi = INT_MAX;
     cand = INT_MAX;
     double sw = 0.0;
-    if constexpr (RING)
-      residual_pass_wring<NT, E, false>(L, B, BW, i_lo, i_hi, k, row, fuse, dotw, ldd, gj, xj,
-                                        piv, B.cR, bv, bi, cand, sw, nonfinite, S, ring, B.r0);
-    else
-      residual_pass<NT, E, false>(L, B, BW, i_lo, i_hi, k, row, fuse, dotw, ldd, gj, xj, piv,
+    residual_pass<NT, E, false>(L, B, BW, i_lo, i_hi, k, row, fuse, dotw, ldd, gj, xj, piv,
                                   B.cR, bv, bi, cand, sw, nonfinite, S);
     __syncthreads();
     if (fuse)
@@ -841,54 +564,9 @@ __global__ void __launch_bounds__(NT, (NT == 512 ? 1 : NT == 256 ? 2 : 4)) aca_k
     // every CTA has passed barrier 2, and W(:,k) / V(:,k) are final.
   }
 
-  // ---------------- post-processing (src/lowRank.cpp:250-277)
   int rank = k;
-  if (status == ACA_POST) {
-    if (k == 0) {
-      for (int i = i_lo + tid; i < i_hi; i += NT) BW[i] = (T)0;
-      for (int j = j_lo + tid; j < j_hi; j += NT) BV[j] = (T)0;
-      rank = 1;
-      status = ACA_DONE;
-    } else if (k >= ub - 1) {
-      const int full = (n <= m) ? n : m;
-      if (B.kcap < full) {
-        status = ACA_NEED_CAP_POST;  // the full representation needs more columns
-        rank = full;
-      } else if (n <= m) {  // W = block (m x n), V = I_n
-        for (int l = 0; l < n; ++l) {
-          double xc[3] = {0.0, 0.0, 0.0};
-          if (!S.dense) {
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-              if (d < S.kp.dim) xc[d] = __ldg(S.pts + d * S.ld + B.c0 + l);
-          }
-          for (int i = i_lo + tid; i < i_hi; i += NT)
-            BW[i + (int64_t)l * ld] = (T)src_entry_xj(S, xc, B.r0 + i, B.c0 + l);
-          for (int j = j_lo + tid; j < j_hi; j += NT)
-            BV[j + (int64_t)l * ld] = (T)((j == l) ? 1.0 : 0.0);
-        }
-        rank = n;
-        status = ACA_DONE;
-      } else {  // W = I_m, V = block^T (n x m)
-        for (int l = 0; l < m; ++l) {
-          double xr[3] = {0.0, 0.0, 0.0};
-          if (!S.dense) {
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-              if (d < S.kp.dim) xr[d] = __ldg(S.pts + d * S.ld + B.r0 + l);
-          }
-          for (int j = j_lo + tid; j < j_hi; j += NT)
-            BV[j + (int64_t)l * ld] = (T)src_entry_xi(S, xr, B.r0 + l, B.c0 + j);
-          for (int i = i_lo + tid; i < i_hi; i += NT)
-            BW[i + (int64_t)l * ld] = (T)((i == l) ? 1.0 : 0.0);
-        }
-        rank = m;
-        status = ACA_DONE;
-      }
-    } else {
-      status = ACA_DONE;
-    }
-  }
+  if (status == ACA_POST)
+    status = aca_post_process<T>(B, S, BW, BV, ld, k, i_lo, i_hi, j_lo, j_hi, NT, &rank);
   if (nonfinite) atomicOr(L.err, DEV_ERR_NONFINITE);
   // Every CTA of the group reached the same state; CTA 0 records it after a
   // last barrier, so that no CTA of the group can still be about to read the
@@ -908,133 +586,54 @@ __global__ void __launch_bounds__(NT, (NT == 512 ? 1 : NT == 256 ? 2 : 4)) aca_k
     st->svp = svp;
     st->pending = pending;
   }
-  if constexpr (RING)
-    if ((tid & 31) == 0) wring_drain(ring, tid >> 5);
 }
 
 }  // namespace
 
-// Stages of the warp rings that fit beside kcap_max row coefficients (the
-// ring's dots are always in global memory): 3, 2, or 0 (no ring).
-int aca_ring_stages(int kcap_max) {
-  for (int st = WR_SMAX; st >= 2; --st)
-    if (wring_bytes(st) + sizeof(double) * (size_t)kcap_max <= 224 * 1024) return st;
-  return 0;
-}
-
-namespace {
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
-// against the driver library); null when the driver does not provide it.
-EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
-                                         &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
-}
-
-// A 2D map over an n x kcap column-major arena (leading dimension n) whose
-// box is one ring tile: WR_ROWS rows by WR_BC columns.  The copy's start row
-// must give a 16-byte aligned address; the kernel keeps it even.
-bool panel_map(CUtensorMap* m, const double* base, int64_t n, int kcap) {
-  EncodeTiledFn f = encode_tiled();
-  if (!f || !base || ((uintptr_t)base & 15) || (n & 1) || n <= 0 || kcap <= 0) return false;
-  const cuuint64_t dim[2] = {(cuuint64_t)n, (cuuint64_t)kcap};
-  const cuuint64_t stride[1] = {(cuuint64_t)n * sizeof(double)};
-  const cuuint32_t box[2] = {(cuuint32_t)WR_ROWS, (cuuint32_t)WR_BC};
-  const cuuint32_t elem[2] = {1, 1};
-  return f(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(base), dim, stride, box,
-           elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-}  // namespace
-
-// The launch's W and V maps for one tensor copy per ring tile; false (and
-// the per-column copies) when either cannot be encoded.
-bool aca_ring_tile_maps(AcaLaunch& L, const double* W, const double* V, int64_t n, int kcap) {
-  return panel_map(&L.map_w, W, n, kcap) && panel_map(&L.map_v, V, n, kcap);
-}
-
-static size_t aca_smem(int nt, int kcap_max, bool global_dots, bool ring, bool f32) {
-  (void)f32;
-  return (ring ? wring_bytes(aca_ring_stages(kcap_max)) : 0) +
-         sizeof(double) * (size_t)(global_dots ? 1 : 1 + nt / 32) * (size_t)kcap_max;
+static size_t aca_smem(int nt, int kcap_max, bool global_dots) {
+  return sizeof(double) * (size_t)(global_dots ? 1 : 1 + nt / 32) * (size_t)kcap_max;
 }
 
 // The per-warp dot partials move to global memory once the CTA's shared
 // memory would pass 100 KB (beyond that fewer than two 256-thread CTAs fit on
-// an SM), and always with the warp rings (their stages fill shared memory).
-bool aca_dots_global(int nt, int kcap_max, bool ring, bool f32) {
-  return ring || aca_smem(nt, kcap_max, false, false, f32) > 100 * 1024;
+// an SM).
+bool aca_dots_global(int nt, int kcap_max) { return aca_smem(nt, kcap_max, false) > 100 * 1024; }
+
+size_t aca_smem_bytes(int nt, int kcap_max) {
+  return aca_smem(nt, kcap_max, aca_dots_global(nt, kcap_max));
 }
 
-size_t aca_smem_bytes(int nt, int kcap_max, bool ring, bool f32) {
-  return aca_smem(nt, kcap_max, aca_dots_global(nt, kcap_max, ring, f32), ring, f32);
-}
-
-template <typename T>
-static void* aca_fn_t(int nt, bool ring, bool narrow) {
-  if (ring) return (void*)aca_kernel<WR_NT, WR_E, true, T>;
+static const void* aca_fn(int nt, bool narrow) {
   if (nt == 256)
-    return narrow ? (void*)aca_kernel<256, 2, false, T> : (void*)aca_kernel<256, 4, false, T>;
-  return (void*)aca_kernel<128, 2, false, T>;
+    return narrow ? (const void*)aca_kernel<256, 2, double> : (const void*)aca_kernel<256, 4, double>;
+  return (const void*)aca_kernel<128, 2, double>;
 }
 
-static void* aca_fn(int nt, bool ring, bool f32, bool narrow = false) {
-  (void)f32;  // FP64 panels only
-  return aca_fn_t<double>(nt, ring, narrow);
-}
-
-// Dynamic shared memory above 48 KB.  The ring kernels (160+ KB per CTA)
-// also ask for the largest shared-memory carveout, so that the occupancy
-// query sizing their cooperative launch and the launch see the same
-// capacity; the others keep the default split and its larger L1 for their
-// per-thread panel loads.
-static int set_smem(void* fn, size_t smem, bool ring) {
-  cudaError_t e = cudaSuccess;
-  if (ring)
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-  if (e == cudaSuccess) e = smem_opt_in(fn, smem);
+// Dynamic shared memory above 48 KB; the default shared-memory carveout
+// otherwise, for its larger L1 (the panels are loaded per thread).
+static int set_smem(const void* fn, size_t smem) {
+  cudaError_t e = smem_opt_in(fn, smem);
   if (e != cudaSuccess) cudaGetLastError();  // consume it: later launch checks stay clean
   return (int)e;
 }
 
 int aca_launch(const AcaLaunch& L, int nt, int kcap_max, bool cooperative, cudaStream_t s) {
-  const bool ring = L.ring != 0, f32 = false;
-  if (ring && (nt != WR_NT || (L.ld % 2) || L.ring_stages != aca_ring_stages(kcap_max) ||
-               L.ring_stages < 2))
-    return (int)cudaErrorInvalidValue;
-  const size_t smem = aca_smem(nt, kcap_max, L.dotg != nullptr, ring, f32);
+  const size_t smem = aca_smem(nt, kcap_max, L.dotg != nullptr);
   dim3 grid(L.cta_block ? L.ncta : L.nblocks * L.G), block(nt);
   void* args[] = {(void*)&L};
-  void* fn = aca_fn(nt, ring, f32, L.narrow != 0);
-  if (int e = set_smem(fn, smem, ring)) return e;
+  const void* fn = aca_fn(nt, L.narrow != 0);
+  if (int e = set_smem(fn, smem)) return e;
   cudaError_t e = cooperative ? cudaLaunchCooperativeKernel(fn, grid, block, args, smem, s)
                               : cudaLaunchKernel(fn, grid, block, args, smem, s);
   if (e != cudaSuccess) cudaGetLastError();
   return e == cudaSuccess ? 0 : (int)e;
 }
 
-int aca_max_coresident(int nt, int kcap_max, bool ring, bool f32, int* per_sm) {
-  const size_t smem = aca_smem_bytes(nt, kcap_max, ring, f32);
-  void* fn = aca_fn(nt, ring, f32);
+int aca_max_coresident(int nt, int kcap_max, int* per_sm) {
+  const size_t smem = aca_smem_bytes(nt, kcap_max);
+  const void* fn = aca_fn(nt, false);
   *per_sm = 0;
-  if (int e = set_smem(fn, smem, ring)) return e;
+  if (int e = set_smem(fn, smem)) return e;
   int nb = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, nt, smem);
   if (e != cudaSuccess) cudaGetLastError();

@@ -6,7 +6,7 @@ namespace hodlr_impl {
 
 // Grow level L to `cap` columns, keeping the first kcap ones.
 int grow_level(hodlr_t h, Level& L, int cap) {
-  const int64_t N = h->n;
+  const int64_t N = h->ldp();
   double *W2 = nullptr, *V2 = nullptr;
   CK(dalloc(h, &W2, (size_t)(N * cap)));
   cudaError_t e = dalloc(h, &V2, (size_t)(N * cap));
@@ -47,6 +47,8 @@ void fill_block(hodlr_t h, Level& L, int q, AcaBlock& B) {
   B.g0 = 0;
   B.G = 1;
   const int p = q >> 1;
+  B.sW = B.sV = nullptr;
+  B.strW = B.strV = 0;
   B.minRank = (q & 1) ? L.bmin[p] : L.tmin[p];
   B.maxRank = (q & 1) ? L.bmax[p] : L.tmax[p];
 }
@@ -57,11 +59,16 @@ bool level_done(const Level& L) {
   return true;
 }
 
-// Run one ACA launch over `blocks` with group size G.
+// Dynamic shared memory of a group launch (one CTA an SM), beside its static
+// arrays.
+size_t group_smem_budget(int v) { return v == ACA_GROUP_8x1 ? 212 * 1024 : 224 * 1024; }
+
 // One ACA launch over `blocks`: groups of G CTAs each, or, with `groups`,
-// groups[i] CTAs for block i (a CTA table maps CTAs to blocks).
-int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_max,
-            bool ring, const std::vector<int>* groups, const Level* arena) {
+// groups[i] CTAs for block i (a CTA table maps CTAs to blocks).  variant:
+// ACA_GROUP_NONE for aca_kernel with nt threads, else of aca_group_kernel.
+// yield_at: with so many CTAs out of work the others' blocks pause (0: never).
+int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_max, int variant,
+            const std::vector<int>* groups, int yield_at) {
   const int nb = (int)blocks.size();
   if (nb == 0) return HODLR_OK;
   int ncta = nb * G;
@@ -107,7 +114,7 @@ int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_ma
   L.blocks = h->d_blocks;
   L.nblocks = nb;
   L.G = G;
-  L.ld = h->n;
+  L.ld = h->ldp();
   L.tol = h->tol;
   L.minPivot = (double)h->minPivot;
   L.kcap_max = kcap_max;
@@ -120,28 +127,58 @@ int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_ma
   L.ncta = ncta;
   L.dotg = nullptr;
   L.dotg_stride = 0;
-  L.ring = ring ? 1 : 0;
-  L.ring_stages = ring ? aca_ring_stages(kcap_max) : 0;
-  // one tensor copy per ring tile needs every block's panels in the level's
-  // arenas (fill_block: W + r0, V + c0); a map that cannot be encoded keeps
-  // the per-column copies
-  L.ring_tile = 0;
-  if (ring && h->aca_ring_tile && arena && arena->kcap == kcap_max)
-    L.ring_tile = aca_ring_tile_maps(L, arena->W, arena->V, h->n, arena->kcap) ? 1 : 0;
-  // slices of a group shorter than 768 rows: the 2-element instance (512-row
-  // chunks) leaves fewer lanes idle than the 4-element one (1024-row chunks)
-  L.narrow = 0;
-  if (!ring && nt == 256 && G > 1) {
-    int longest = 0;
-    for (auto& b : blocks) longest = std::max(longest, std::max(b.m, b.n));
-    L.narrow = (longest + G - 1) / G < 768 ? 1 : 0;
-  }
-  L.spin_limit = h->spin_limit ? h->spin_limit : HODLR_SPIN_LIMIT;
+  L.spin_limit = h->spin_limit ? h->spin_limit : variant ? HODLR_SPIN_LIMIT >> 4 : HODLR_SPIN_LIMIT;
   L.bar_extra = h->bar_unreachable ? 1u : 0u;
-  if (aca_smem_bytes(nt, kcap_max, ring, false) > 227 * 1024)
-    return fail(h, HODLR_ERR_UNSUPPORTED, "block rank above the shared-memory limit of ACA");
-  if (aca_dots_global(nt, kcap_max, ring, false)) {
-    L.dotg_stride = (int64_t)(nt / 32) * kcap_max;
+  L.narrow = 0;
+  L.ring_stages = L.stage_elems = 0;
+  L.slots = nullptr;
+  size_t smem = 0;
+  if (variant) {
+    int rows = 1;
+    for (int i = 0; i < nb; ++i) {
+      const int g = groups ? (*groups)[i] : G;
+      rows = std::max(rows, (std::max(blocks[i].m, blocks[i].n) + g - 1) / g);
+    }
+    L.ring_stages = aca_group_ring(variant, rows, kcap_max, group_smem_budget(variant), &L.stage_elems,
+                                   &smem);
+    if (!L.ring_stages) return fail(h, HODLR_ERR_STATE, "ACA ring does not fit");
+    if (ncta > h->slots_cap) {
+      dfree(h, h->slots);
+      CK(dalloc(h, &h->slots, (size_t)ncta * 128 + 128));
+      h->slots_cap = ncta;
+    }
+    L.slots = h->slots;
+    CK(cudaMemsetAsync(h->slots, 0, (size_t)ncta * 128 + 128, h->stream));
+    L.idle = reinterpret_cast<unsigned*>(h->slots + (size_t)ncta * 128);
+    L.yield_at = yield_at;
+    L.pub_stride = 16 * ((int64_t)kcap_max + 1);
+    const int64_t pneed = 2 * L.pub_stride * ncta;
+    if (pneed > h->pub_cap) {
+      dfree(h, h->pub);
+      h->pub_cap = 0;
+      CK(dalloc(h, &h->pub, (size_t)pneed));
+      CK(cudaMemsetAsync(h->pub, 0, (size_t)pneed, h->stream));
+      h->pub_cap = pneed;
+    }
+    L.pub = h->pub;
+    L.launch_tag = ++h->aca_tag;
+    L.dotg_stride = aca_group_dots(variant, rows) * kcap_max;
+  } else {
+    // slices of a group shorter than 768 rows: the 2-element instance (512-row
+    // chunks) leaves fewer lanes idle than the 4-element one (1024-row chunks)
+    if (nt == 256) {
+      int longest = 0;
+      for (int i = 0; i < nb; ++i) {
+        const int g = groups ? (*groups)[i] : G;
+        longest = std::max(longest, (std::max(blocks[i].m, blocks[i].n) + g - 1) / g);
+      }
+      L.narrow = longest < 768 ? 1 : 0;
+    }
+    if (aca_smem_bytes(nt, kcap_max) > 227 * 1024)
+      return fail(h, HODLR_ERR_UNSUPPORTED, "block rank above the shared-memory limit of ACA");
+    if (aca_dots_global(nt, kcap_max)) L.dotg_stride = (int64_t)(nt / 32) * kcap_max;
+  }
+  if (L.dotg_stride > 0) {
     const int64_t dneed = L.dotg_stride * ncta;
     if (dneed > h->dotg_cap) {
       dfree(h, h->dotg);
@@ -154,7 +191,8 @@ int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_ma
   if (groups)
     for (int g : *groups) coop |= g > 1;
   CK(cudaEventRecord(h->ev0, h->stream));
-  int rc = aca_launch(L, nt, kcap_max, coop, h->stream);
+  int rc = variant ? aca_group_launch(L, variant, smem, coop, h->stream)
+                   : aca_launch(L, nt, kcap_max, coop, h->stream);
   if (rc == (int)cudaErrorCooperativeLaunchTooLarge) return HODLR_ERR_RETRY_SMALLER;
   if (rc) return cuda_fail(h, (cudaError_t)rc, "aca_launch");
   h->nlaunch += 1;
@@ -208,19 +246,21 @@ int sync_level(hodlr_t h, Level& L, bool* done) {
                      h->stream));
   CK(cudaStreamSynchronize(h->stream));
   int need = 0;
+  bool resume = false;
   *done = true;
   for (auto& s : L.st) {
     if (s.status == ACA_ERROR) return fail(h, HODLR_ERR_TIMEOUT, "ACA group failed");
     if (s.status == ACA_NEED_CAP) need = std::max(need, L.kcap + std::max(32, L.kcap / 2));
     if (s.status == ACA_NEED_CAP_POST) need = std::max(need, s.rank);
+    resume |= s.status == ACA_PAUSED;
     if (s.status != ACA_DONE) *done = false;
   }
-  if (need > 0) {
+  if (need > 0 || resume) {
     int cap = std::min(std::max(need, L.kcap + 1), std::max(L.ub_max, L.kcap + 1));
-    int rc = grow_level(h, L, cap);
+    int rc = need > 0 ? grow_level(h, L, cap) : HODLR_OK;
     if (rc) return rc;
     for (auto& s : L.st) {
-      if (s.status == ACA_NEED_CAP) s.status = ACA_RUNNING;
+      if (s.status == ACA_NEED_CAP || s.status == ACA_PAUSED) s.status = ACA_RUNNING;
       if (s.status == ACA_NEED_CAP_POST) s.status = ACA_POST;
     }
     CK(cudaMemcpyAsync(L.d_st, L.st.data(), sizeof(AcaState) * nb, cudaMemcpyHostToDevice,
@@ -294,6 +334,203 @@ int predict_ranks(hodlr_t h) {
   return HODLR_OK;
 }
 
+// The working layout's memory goes back to the device pool, not to the
+// handle's cache: the factorization's panels are cut from it next.
+void free_aca_work(hodlr_t h) {
+  if (h->aca_work) cudaFreeAsync(h->aca_work, h->stream);
+  h->aca_work = nullptr;
+  h->aca_work_cap = 0;
+}
+
+// ---- launches of the few-block levels
+//
+// Time of a block's ACA from k0 to k columns, in us: steps of two passes.  A pass is a fixed part
+// (5 alone, 8 with an exchange over a group), the start of every further chunk
+// of the slice (its entries), and its tiles: GR 8x1 takes 16 columns of up to
+// 256 rows in 0.3 us or more and streams at 44 KB/us, 8x4 takes 4 columns of
+// up to 1024 rows in 0.3 us or more at 48 KB/us (measured on B200, one CTA an
+// SM: the rates are the SM's share of the memory rate).
+double group_time(int variant, double rows, double k0, double k, int G) {
+  const double r = std::ceil(rows / G), kh = 0.5 * (k0 + k), fixed = G > 1 ? 8.0 : 5.0;
+  double pass;
+  if (variant == ACA_GROUP_8x1) {
+    const double c = std::ceil(r / 256.0);
+    pass = fixed + 0.9 * (c - 1.0) + std::ceil(kh / 16.0) * c * std::max(0.3, r / c * 128.0 / 44e3);
+  } else {
+    const double c = std::ceil(r / 1024.0);
+    pass = fixed + 1.0 + 2.5 * (c - 1.0) +
+           std::ceil(kh / 4.0) * c * std::max(0.3, r / c * 32.0 / 48e3);
+  }
+  return 2.0 * (k - k0) * pass;
+}
+
+struct GroupJob {
+  int level, q, rows, G;
+  double k0, k, t;
+  int64_t work = 0, strW = 0, strV = 0;  // the block's slices in the working memory
+};
+
+// Share `ctas` CTAs among the jobs: always to the slowest one, as many more as
+// make it faster.  Returns the slowest job's time; < 0: more jobs than CTAs.
+double share_ctas(std::vector<GroupJob>& jobs, int ctas, int variant) {
+  if ((int)jobs.size() > ctas) return -1.0;
+  int left = ctas - (int)jobs.size();
+  auto slower = [&](int a, int b) { return jobs[a].t < jobs[b].t; };
+  std::vector<int> heap;
+  for (size_t i = 0; i < jobs.size(); ++i) {
+    jobs[i].G = 1;
+    jobs[i].t = group_time(variant, jobs[i].rows, jobs[i].k0, jobs[i].k, 1);
+    heap.push_back((int)i);
+  }
+  std::make_heap(heap.begin(), heap.end(), slower);
+  while (!heap.empty()) {
+    GroupJob& j = jobs[heap.front()];
+    int more = 0;
+    const int most = std::min(left, j.rows / 16);  // at least 16 rows a CTA
+    for (int d = 1; d <= most && !more; ++d)
+      if (group_time(variant, j.rows, j.k0, j.k, j.G + d) < j.t) more = d;
+    if (!more) break;
+    j.G += more;
+    left -= more;
+    j.t = group_time(variant, j.rows, j.k0, j.k, j.G);
+    std::pop_heap(heap.begin(), heap.end(), slower);
+    std::push_heap(heap.begin(), heap.end(), slower);
+  }
+  return heap.empty() ? 0.0 : jobs[heap.front()].t;
+}
+
+std::vector<GroupJob> group_jobs(hodlr_t h, const std::vector<int>& levels,
+                                 const std::vector<double>& rank_est) {
+  std::vector<GroupJob> jobs;
+  for (int l : levels) {
+    const Level& L = h->lv[l];
+    for (int q = 0; q < L.nblocks(); ++q) {
+      if (!L.st.empty() && L.st[q].status == ACA_DONE) continue;
+      int r0, c0, m, n;
+      block_geom(L, q, r0, c0, m, n);
+      const double k0 = L.st.empty() ? 0.0 : L.st[q].k, most = std::min(m, n);
+      const double k = std::min(most, std::max(rank_est[l], 1.25 * k0 + 4.0));
+      GroupJob j{l, q, std::max(m, n), 1, k0, std::max(k0 + 1.0, k), 0.0};
+      jobs.push_back(j);
+    }
+  }
+  return jobs;
+}
+
+// The levels still to do (uppermost first) are cut into sets of neighbours
+// whose blocks run in one launch: few-step and many-step blocks side by side
+// keep the SMs busy where one level alone waits on its exchanges or on its
+// slowest block, but a block in a crowd has fewer CTAs.  The cut minimises the
+// sum of the sets' times as group_time has them.  Returns the index of the
+// uppermost level of the deepest set, which runs first.
+int group_set_top(hodlr_t h, const std::vector<int>& levels, const std::vector<double>& rank_est) {
+  const int n = (int)levels.size();
+  std::vector<double> best((size_t)n + 1, HUGE_VAL);  // of levels [0, i)
+  std::vector<int> cut((size_t)n + 1, 0);
+  best[0] = 0.0;
+  for (int i = 1; i <= n; ++i)
+    for (int j = i - 1; j >= 0; --j) {
+      std::vector<int> set(levels.begin() + j, levels.begin() + i);
+      std::vector<GroupJob> jobs = group_jobs(h, set, rank_est);
+      const double t1 = share_ctas(jobs, h->num_sms, ACA_GROUP_8x1);
+      if (t1 < 0 && j < i - 1) break;  // more levels only add blocks
+      double t = t1 < 0 ? 0.0 : std::min(t1, share_ctas(jobs, h->num_sms, ACA_GROUP_8x4));
+      t += 60.0;  // a launch and its read-back
+      if (best[j] + t < best[i]) {
+        best[i] = best[j] + t;
+        cut[i] = j;
+      }
+    }
+  return cut[n];
+}
+
+// One launch over every unfinished block of the set's levels.
+int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<double>& rank_est) {
+  std::vector<GroupJob> jobs = group_jobs(h, set, rank_est);
+  int ctas = h->num_sms, kcap_max = 1;
+  for (int l : set) kcap_max = std::max(kcap_max, h->lv[l].kcap);
+  for (;;) {  // a cooperative launch the driver refuses is retried with half the CTAs
+    int variant = ACA_GROUP_NONE;
+    const double t1 = share_ctas(jobs, ctas, ACA_GROUP_8x1);
+    if (h->aca_ring && t1 >= 0) {
+      int rows = 1, elems = 0, ps = 0;
+      size_t bytes = 0;
+      variant = ACA_GROUP_8x4;
+      if (t1 <= share_ctas(jobs, ctas, variant)) {
+        variant = ACA_GROUP_8x1;
+        share_ctas(jobs, ctas, variant);
+      }
+      for (auto& j : jobs) rows = std::max(rows, (j.rows + j.G - 1) / j.G);
+      if (!aca_group_ring(variant, rows, kcap_max, group_smem_budget(variant), &elems, &bytes))
+        variant = ACA_GROUP_NONE;  // too many columns beside a ring
+      else if (aca_group_max_coresident(variant, bytes, &ps) || ps < 1)
+        return fail(h, HODLR_ERR_CUDA, "occupancy query failed");
+      // the slices' working layout; without memory for it the panels are
+      // loaded from the arenas per thread
+      int64_t work = 0;
+      for (auto& j : jobs) {
+        int r0, c0, m, n;
+        block_geom(h->lv[j.level], j.q, r0, c0, m, n);
+        const int kcap = h->lv[j.level].kcap;
+        j.work = work;
+        j.strW = aca_group_slice(variant, (m + j.G - 1) / j.G, kcap);
+        j.strV = aca_group_slice(variant, (n + j.G - 1) / j.G, kcap);
+        work += (j.strW + j.strV) * j.G;
+      }
+      if (variant && work > h->aca_work_cap) {
+        free_aca_work(h);
+        if (h->pool.raw_alloc((void**)&h->aca_work, sizeof(double) * (size_t)work, h->stream) ==
+            cudaSuccess) {
+          h->aca_work_cap = work;
+        } else {
+          cudaGetLastError();
+          h->aca_work = nullptr;
+          variant = ACA_GROUP_NONE;
+        }
+      }
+    }
+    if (!variant) {
+      // panels loaded per thread, several CTAs an SM: the same shares of what fits
+      int ps = 0;
+      if (aca_max_coresident(256, kcap_max, &ps))
+        return fail(h, HODLR_ERR_CUDA, "occupancy query failed");
+      const int most = std::max(1, ps) * ctas;
+      if (share_ctas(jobs, most, ACA_GROUP_8x4) < 0)
+        for (auto& j : jobs) j.G = 1;
+    }
+    std::vector<AcaBlock> bl(jobs.size());
+    std::vector<int> groups(jobs.size());
+    bool any = false;
+    for (size_t i = 0; i < jobs.size(); ++i) {
+      Level& L = h->lv[jobs[i].level];
+      fill_block(h, L, jobs[i].q, bl[i]);
+      if (variant) {
+        bl[i].sW = h->aca_work + jobs[i].work;
+        bl[i].sV = bl[i].sW + jobs[i].strW * jobs[i].G;
+        bl[i].strW = jobs[i].strW;
+        bl[i].strV = jobs[i].strV;
+      }
+      groups[i] = jobs[i].G;
+      L.G = jobs[i].G;
+      any |= jobs[i].G > 1;
+    }
+    int most = 0;
+    double slowest = 0.0;
+    for (auto& j : jobs) {
+      most += j.G;
+      slowest = std::max(slowest, j.t);
+    }
+    // ranks differ from block to block: share the CTAs anew when a third of
+    // them are out of work, where a launch takes far longer than its overhead
+    // (2D N = 262144: 107 ms against 133 with fixed shares)
+    const int yield_at = jobs.size() > 1 && slowest > 2000.0 ? std::max(1, most / 3) : 0;
+    const int rc = run_aca(h, bl, 1, any ? 256 : 128, kcap_max, variant, &groups, yield_at);
+    if (rc != HODLR_ERR_RETRY_SMALLER) return rc;
+    if (ctas == 1) return fail(h, HODLR_ERR_CUDA, "aca_launch: cooperative launch refused");
+    ctas = std::max(1, ctas / 2);
+  }
+}
+
 int do_compress(hodlr_t h) {
   if (h->compressed) return HODLR_OK;
   free_compress(h);
@@ -324,7 +561,7 @@ int do_compress(hodlr_t h) {
   };
   auto pred_or = [&](int l, int q) -> int64_t { return have_pred ? pred(l, q) + 1 : 1; };
   int per_sm = 0;
-  if (aca_max_coresident(256, 256, false, false, &per_sm))
+  if (aca_max_coresident(256, 256, &per_sm))
     return fail(h, HODLR_ERR_CUDA, "occupancy query failed");
   const int P0 = std::max(1, per_sm) * h->num_sms;
   std::vector<int> pooled_levels, group_levels;
@@ -367,51 +604,50 @@ int do_compress(hodlr_t h) {
     }
     if (all) break;
   }
-  // 2. the few-block levels, deepest first
-  int kmax_below = 0;
-  if (!pooled_levels.empty()) kmax_below = level_kmax(h->lv[pooled_levels.front()]);
-  for (auto it = group_levels.rbegin(); it != group_levels.rend(); ++it) {
-    const int l = *it;
-    Level& L = h->lv[l];
-    int guess = hint(l) ? hint(l) : std::max(64, (kmax_below * 3 + 1) / 2 + 16);
-    int rc = init_level(h, L, guess);
-    if (rc) return rc;
-    for (int round = 0; round < 64; ++round) {
-      // the group levels stream their panels through the bulk-copy ring
-      // (16-byte aligned columns need an even N) while that still leaves at
-      // least two of its one-per-SM CTAs to every block
-      const int nb = L.nblocks();
-      int ps = 0, ps_ring = 0;
-      const bool ring_fits = aca_ring_stages(L.kcap) >= 2;
-      if (aca_max_coresident(256, L.kcap, false, false, &ps) ||
-          (ring_fits && aca_max_coresident(512, L.kcap, true, false, &ps_ring)))
-        return fail(h, HODLR_ERR_CUDA, "occupancy query failed");
-      const bool ring = h->aca_ring && ring_fits && (h->n % 2 == 0) &&
-                        ps_ring * h->num_sms >= 2 * nb;
-      if (ring) ps = ps_ring;
-      // equal groups: CTAs sized by predicted work measured 2-8% slower on
-      // 3D clouds than equal groups (per-step latency, not streamed bytes,
-      // sets a block's time)
-      int G = std::max(1, std::max(1, ps) * h->num_sms / nb);
-      std::vector<AcaBlock> bl(nb);
-      for (;;) {  // a cooperative launch the driver refuses is retried with half the groups
-        L.G = G;
-        for (int q = 0; q < nb; ++q) fill_block(h, L, q, bl[q]);
-        rc = run_aca(h, bl, G, ring ? 512 : G > 1 ? 256 : 128, L.kcap, ring, nullptr, &L);
-        if (rc != HODLR_ERR_RETRY_SMALLER) break;
-        if (G == 1) return fail(h, HODLR_ERR_CUDA, "aca_launch: cooperative launch refused");
-        G = std::max(1, G / 2);
-      }
-      if (rc) return rc;
-      bool done;
-      rc = sync_level(h, L, &done);
-      if (rc) return rc;
-      if (done) break;
+  // 2. the few-block levels, in sets of neighbouring levels, deepest first:
+  // the blocks of a set run in one launch (group_sets)
+  std::vector<double> rank_est((size_t)nlev, 0.0);
+  double growth = 1.0;  // of the rank from one level to the next above it
+  int known = -1;       // the uppermost level compressed so far
+  auto note_rank = [&](int l) {
+    rank_est[l] = std::max(1, level_kmax(h->lv[l]));
+    if (known == l + 1 && rank_est[known] > 0)
+      growth = std::min(1.5, std::max(1.0, rank_est[l] / rank_est[known]));
+    known = l;
+  };
+  for (auto it = pooled_levels.rbegin(); it != pooled_levels.rend(); ++it) note_rank(*it);
+  while (!group_levels.empty()) {
+    for (auto it = group_levels.rbegin(); it != group_levels.rend(); ++it) {
+      const int l = *it;
+      const double below = l + 1 < nlev ? rank_est[l + 1] : 0.0;
+      rank_est[l] = std::min((double)h->lv[l].ub_max, below > 0 ? below * growth : 32.0);
     }
-    kmax_below = level_kmax(L);
+    const int top = group_set_top(h, group_levels, rank_est);
+    std::vector<int> set(group_levels.begin() + top, group_levels.end());
+    group_levels.resize(top);
+    for (int l : set) {
+      const double below = l + 1 < nlev ? rank_est[l + 1] : 0.0;
+      int rc = init_level(h, h->lv[l],
+                          hint(l) ? hint(l) : std::max(64, ((int)below * 3 + 1) / 2 + 16));
+      if (rc) return rc;
+    }
+    for (int round = 0; round < 256; ++round) {
+      bool all = true;
+      for (int l : set) all &= level_done(h->lv[l]);
+      if (all) break;
+      int rc = run_group_set(h, set, rank_est);
+      if (rc) return rc;
+      for (int l : set) {
+        bool done;
+        rc = sync_level(h, h->lv[l], &done);
+        if (rc) return rc;
+      }
+    }
+    for (auto it = set.rbegin(); it != set.rend(); ++it) note_rank(*it);
   }
+  free_aca_work(h);
   for (auto& L : h->lv)
-    if (!level_done(L)) return fail(h, HODLR_ERR_STATE, "ACA did not converge in 64 rounds");
+    if (!level_done(L)) return fail(h, HODLR_ERR_STATE, "ACA did not converge in its launches");
   // ranks, level widths, column offsets, algorithmic bytes
   int64_t coff = 0;
   double bytes = 0;

@@ -129,7 +129,7 @@ int do_factorize(hodlr_t h) {
   free_factor(h);  // first: a factorization that overwrote W also drops the compression
   int rc = do_compress(h);
   if (rc) return rc;
-  const int64_t N = h->n;
+  const int64_t N = h->n, ldp = h->ldp();
   CK(cudaEventRecord(h->ev0, h->stream));
   // leaves: assemble + LU
   const int nl = (int)h->leaf_min.size();
@@ -198,7 +198,7 @@ int do_factorize(hodlr_t h) {
       }
       L.y_alias = h->in_place == 1;
       if (!L.y_alias) {
-        cudaError_t ea = dalloc(h, &L.Yl, (size_t)(N * L.kmax));
+        cudaError_t ea = dalloc(h, &L.Yl, (size_t)(ldp * L.kmax));
         if (ea == cudaErrorMemoryAllocation && h->in_place == -1) {
           cudaGetLastError();
           L.y_alias = true;
@@ -220,7 +220,7 @@ int do_factorize(hodlr_t h) {
       int maxm = 0;
       for (int m : ms) maxm = std::max(maxm, m);
       dim3 grid(std::min(64, (maxm + 255) / 256), nb, std::min(L.kmax, 64));
-      y_init_kernel<<<grid, 256, 0, h->stream>>>(L.Yl, L.W, N, L.kmax, d_r0, d_m, d_rk, nb);
+      y_init_kernel<<<grid, 256, 0, h->stream>>>(L.Yl, L.W, ldp, L.kmax, d_r0, d_m, d_rk, nb);
       CK(cudaGetLastError());
       h->nlaunch += 1;
       dfree(h, d_r0);  // reused only after the stream has drained (DevPool)
@@ -240,7 +240,7 @@ int do_factorize(hodlr_t h) {
     for (auto& L : h->lv) CH = std::max(CH, std::min(L.kmax, 512));
     double *Xinv = nullptr, *Y2 = nullptr;
     CK(dalloc(h, &Xinv, (size_t)(N * sm)));
-    CK(dalloc(h, &Y2, (size_t)(N * CH)));
+    CK(dalloc(h, &Y2, (size_t)(ldp * CH)));
     CK(cudaMemsetAsync(Xinv, 0, sizeof(double) * N * sm, h->stream));
     leaf_identity_kernel<<<nl, 128, 0, h->stream>>>(Xinv, N, h->d_leaf_min, h->d_leaf_size);
     CK(cudaGetLastError());
@@ -268,7 +268,7 @@ int do_factorize(hodlr_t h) {
     for (auto& L : h->lv) {
       for (int c0 = 0; c0 < L.kmax; c0 += CH) {
         const int nc = std::min(CH, L.kmax - c0);
-        double* Yc = L.Yl + (int64_t)c0 * N;
+        double* Yc = L.Yl + (int64_t)c0 * ldp;
         std::vector<GemmProblem> probs[3];
         for (int p = 0; p < nl; ++p) {
           const int r0 = h->leaf_min[p], s = h->leaf_size[p];
@@ -276,7 +276,8 @@ int do_factorize(hodlr_t h) {
           g.M = s;
           g.N = nc;
           g.K = s;
-          g.lda = g.ldb = g.ldc = (int)N;
+          g.lda = (int)N;
+          g.ldb = g.ldc = (int)ldp;
           g.A = Xinv + r0;  // Y2 = Xinv Y
           g.B = Yc + r0;
           g.C = Y2 + r0;
@@ -312,7 +313,7 @@ int do_factorize(hodlr_t h) {
         if (e) return cuda_fail(h, (cudaError_t)e, "leaf inverse product");
         rc = check_phase(h, "factor: leaf inverse product");
         if (rc) return rc;
-        CK(cudaMemcpyAsync(Yc, Y2, sizeof(double) * N * nc, cudaMemcpyDeviceToDevice, h->stream));
+        CK(cudaMemcpyAsync(Yc, Y2, sizeof(double) * ldp * nc, cudaMemcpyDeviceToDevice, h->stream));
         h->nlaunch += 3;
       }
     }
@@ -371,10 +372,10 @@ int do_factorize(hodlr_t h) {
           t.A = L.V + mn;  // V of the bottom block lives on the top rows
           t.M = sn.kb;
           t.K = sp - mn + 1;
-          t.lda = (int)N;
+          t.lda = (int)ldp;
           t.B = A.Yl + mn;
           t.N = ncols_t;
-          t.ldb = (int)N;
+          t.ldb = (int)ldp;
           t.C = h->Z + sn.z_off + (int64_t)A.coff * sd + (h->sm_form ? sn.kt : 0);
           t.ldc = sd;
           tn.push_back(t);
@@ -384,10 +385,10 @@ int do_factorize(hodlr_t h) {
           b.A = L.V + sp + 1;  // V of the top block lives on the bottom rows
           b.M = sn.kt;
           b.K = mx - sp;
-          b.lda = (int)N;
+          b.lda = (int)ldp;
           b.B = A.Yl + sp + 1;
           b.N = ncols_b;
-          b.ldb = (int)N;
+          b.ldb = (int)ldp;
           b.C = h->Z + sn.z_off + (int64_t)A.coff * sd + (h->sm_form ? 0 : sn.kb);
           b.ldc = sd;
           tn.push_back(b);
@@ -456,9 +457,9 @@ int do_factorize(hodlr_t h) {
           if (sn.kt > 0) {
             GemmProblem t{};
             t.C = A.Yl + mn;
-            t.ldc = (int)N;
+            t.ldc = (int)ldp;
             t.A = L.Yl + mn;
-            t.lda = (int)N;
+            t.lda = (int)ldp;
             t.M = sp - mn + 1;
             t.K = sn.kt;
             t.B = h->Z + sn.z_off + (h->sm_form ? 0 : sn.kb) + (int64_t)A.coff * sd;
@@ -469,9 +470,9 @@ int do_factorize(hodlr_t h) {
           if (sn.kb > 0) {
             GemmProblem b{};
             b.C = A.Yl + sp + 1;
-            b.ldc = (int)N;
+            b.ldc = (int)ldp;
             b.A = L.Yl + sp + 1;
-            b.lda = (int)N;
+            b.lda = (int)ldp;
             b.M = mx - sp;
             b.K = sn.kb;
             b.B = h->Z + sn.z_off + (h->sm_form ? sn.kt : 0) + (int64_t)A.coff * sd;

@@ -238,7 +238,6 @@ int init_common(hodlr_t h) {
   const char* acs = getenv("HODLR_ACA_STREAMING");
   if (acs && acs[0] >= '0' && acs[0] <= '2' && acs[1] == 0) {
     h->aca_ring = acs[0] != '0';
-    h->aca_ring_tile = acs[0] == '2';
   }
   CK(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
   h->stream = h->own_stream;

@@ -17,9 +17,9 @@
 //
 // HBM layout (N = matrix size, column-major, leading dimension N):
 //   pts        dim x N coordinates (SoA)            or A  N x N dense input
-//   W_l, V_l   N x kcap_l per inner level l: the blocks of a level tile the
+//   W_l, V_l   N x kcap_l (leading dimension ldp: N rounded up to even) per inner level l: the blocks of a level tile the
 //              rows (W) and the columns (V) of the matrix exactly once
-//   Y_l        N x kmax_l per level (its own allocation, or the first kmax_l
+//   Y_l        N x kmax_l (ldp) per level (its own allocation, or the first kmax_l
 //              columns of W_l, overwritten): K^-1 U of the level's nodes
 //              (topDiagSoln_LR / bottDiagSoln_LR) after the factorization
 //   leaf LU    sum over leaves of s^2, plus a row permutation (N ints)
@@ -45,11 +45,16 @@
 #include "rank_mlp.h"
 
 int aca_launch(const AcaLaunch& L, int nt, int kcap_max, bool cooperative, cudaStream_t s);
-int aca_max_coresident(int nt, int kcap_max, bool ring, bool f32, int* per_sm);
-bool aca_dots_global(int nt, int kcap_max, bool ring, bool f32);
-size_t aca_smem_bytes(int nt, int kcap_max, bool ring, bool f32);
-int aca_ring_stages(int kcap_max);
-bool aca_ring_tile_maps(AcaLaunch& L, const double* W, const double* V, int64_t n, int kcap);
+int aca_max_coresident(int nt, int kcap_max, int* per_sm);
+bool aca_dots_global(int nt, int kcap_max);
+size_t aca_smem_bytes(int nt, int kcap_max);
+// aca_group_kernel, by sum warps x rows a thread (aca_group.cu)
+enum { ACA_GROUP_NONE = 0, ACA_GROUP_8x1, ACA_GROUP_8x4 };
+int64_t aca_group_dots(int v, int rows);
+int64_t aca_group_slice(int v, int per, int kcap);
+int aca_group_ring(int v, int rows, int kcap, size_t budget, int* stage_elems, size_t* bytes);
+int aca_group_max_coresident(int v, size_t smem, int* per_sm);
+int aca_group_launch(const AcaLaunch& L, int v, size_t smem, bool cooperative, cudaStream_t s);
 
 namespace hodlr_impl {
 
@@ -224,6 +229,9 @@ struct hodlr_handle_s {
   double model_l = 0.0;
   std::vector<int> pred;
   int n = 0, leaf = 30, dim = 0;
+  // leading dimension of the W, V and K^-1 U panels: n rounded up to even, so
+  // that every column starts on a 16-byte boundary
+  int64_t ldp() const { return ((int64_t)n + 1) & ~(int64_t)1; }
   bool dense = false;
   hx_kparams kp{};
   double* d_pts = nullptr;
@@ -233,12 +241,9 @@ struct hodlr_handle_s {
   std::vector<hodlr_impl::Level> lv;
   std::vector<int> cap_hint;  // initial W/V columns per level (0 = default)
   int gemm_prec = HODLR_GEMM_FP64;  // arithmetic of the Woodbury products
-  // group-level ACA panels through the warps' rings (per-thread loads: 3.59
-  // TB/s on the sphere shape at N = 262144, 2.38 on the 2D cloud) ...
+  // group levels in aca_group_kernel (panels through the CTAs' rings); false:
+  // aca_kernel (panels loaded per thread), the same bits
   bool aca_ring = true;
-  // ... each ring tile one 2D tensor copy (4.87 and 3.30 TB/s) rather than
-  // one bulk copy per column (4.28 and 2.85 TB/s); the same bits every way
-  bool aca_ring_tile = true;
   // factorization form (hodlr_set_solver_form): false recLU's Schur systems
   // [bottom; top], true recSM's perturbI systems [top; bottom]
   bool sm_form = false;
@@ -289,6 +294,13 @@ struct hodlr_handle_s {
   int64_t part_cap = 0;
   unsigned* bar = nullptr;
   int bar_cap = 0;
+  unsigned char* slots = nullptr;  // exchange slots of aca_group_kernel, 128 bytes a CTA
+  int slots_cap = 0;
+  unsigned char* pub = nullptr;    // its published rows, zeroed when allocated
+  int64_t pub_cap = 0;
+  double* aca_work = nullptr;      // its blocks' slices while a compression runs
+  int64_t aca_work_cap = 0;
+  unsigned aca_tag = 0;            // number of its last launch: no tag is used twice
   AcaBlock* d_blocks = nullptr;
   int blocks_cap = 0;
   unsigned* d_err = nullptr;
@@ -360,15 +372,15 @@ EntrySrc make_src(hodlr_t h);
 int grow_level(hodlr_t h, Level& L, int cap);
 void fill_block(hodlr_t h, Level& L, int q, AcaBlock& B);
 bool level_done(const Level& L);
-int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_max,
-            bool ring = false, const std::vector<int>* groups = nullptr,
-            const Level* arena = nullptr);
+int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_max, int variant = 0,
+            const std::vector<int>* groups = nullptr, int yield_at = 0);
 int init_level(hodlr_t h, Level& L, int cap);
 int sync_level(hodlr_t h, Level& L, bool* done);
 int level_kmax(const Level& L);
 std::vector<int4> block_geoms(hodlr_t h);
 int block_features_dev(hodlr_t h, const std::vector<int4>& geom, double l, float* d_F);
 int predict_ranks(hodlr_t h);
+void free_aca_work(hodlr_t h);
 int do_compress(hodlr_t h);
 int upload_plan(hodlr_t h, std::vector<GemmProblem>& probs, bool split, DevPlan& out,
                 const char* what = "grouped GEMM");

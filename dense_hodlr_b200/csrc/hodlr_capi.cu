@@ -268,6 +268,9 @@ void hodlr_destroy(hodlr_t h) {
   dfree(h, h->gm_part);
   dfree(h, h->part);
   dfree(h, h->bar);
+  dfree(h, h->slots);
+  dfree(h, h->pub);
+  free_aca_work(h);
   dfree(h, h->d_blocks);
   dfree(h, h->d_cta);
   dfree(h, h->dotg);
@@ -488,7 +491,6 @@ int hodlr_set_checked(hodlr_t h, int on) {
 int hodlr_set_aca_streaming(hodlr_t h, int on) {
   if (!h || on < 0 || on > 2) return HODLR_ERR_ARG;
   h->aca_ring = on != 0;
-  h->aca_ring_tile = on == 2;
   return HODLR_OK;
 }
 
@@ -808,7 +810,7 @@ int hodlr_get_lowrank(hodlr_t h, int block, double* W, double* V) {
   int r0, c0, m, n;
   block_geom(L, q, r0, c0, m, n);
   const int r = L.st[q].rank;
-  const int64_t N = h->n;
+  const int64_t N = h->ldp();
   if (W) CK(copy2d(h, W, sizeof(double) * m, L.W + r0, sizeof(double) * N, sizeof(double) * m, r, cudaMemcpyDeviceToHost));
   if (V) CK(copy2d(h, V, sizeof(double) * n, L.V + c0, sizeof(double) * N, sizeof(double) * n, r, cudaMemcpyDeviceToHost));
   return HODLR_OK;

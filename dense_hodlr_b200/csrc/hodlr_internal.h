@@ -1,7 +1,6 @@
 // Internal structures shared by the kernels and the host orchestration.
 #pragma once
 
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -28,6 +27,7 @@ enum {
   ACA_NEED_CAP = 3,  // loop paused: more columns of W/V are needed
   ACA_ERROR = 4,
   ACA_NEED_CAP_POST = 5,  // loop done; the full-rank form needs more columns
+  ACA_PAUSED = 6,         // loop paused for another share of the CTAs
 };
 
 // One off-diagonal block.  W and V point at the block's first row inside the
@@ -47,6 +47,10 @@ struct AcaBlock {
   int kcap;           // columns available in W and V
   int level;
   int g0, G;          // with a CTA table: first CTA of this block's group, group size
+  // aca_group_kernel: the block's slices of W and V in the launch's working
+  // layout, doubles from one CTA's to the next
+  double *sW, *sV;
+  int64_t strW, strV;
   int minRank, maxRank;  // the node's rank bounds for this block (-1: none)
 };
 
@@ -75,17 +79,21 @@ struct AcaLaunch {
   int ncta;              // CTAs of the launch when cta_block is set
   double* dotg;          // per-CTA per-warp dot partials in global memory (large ranks), or null
   int64_t dotg_stride;   // doubles per CTA in dotg (NT/32 * kcap_max)
-  int ring;              // 1: panel slices streamed by per-warp bulk-copy rings (512
-                         //    threads, even ld)
-  int ring_stages;       // stages of each warp's ring (aca_ring_stages(kcap_max))
-  int narrow;            // 1 (256 threads, no ring): 2 elements per thread, 512-row chunks
+  int narrow;            // 1 (aca_kernel with 256 threads): 2 elements per thread, 512-row chunks
   unsigned spin_limit;   // polls of a group barrier before it gives up (DEV_ERR_TIMEOUT)
   unsigned bar_extra;    // arrivals a group barrier waits for beyond its G CTAs (0; 1 makes
                          // every barrier unreachable, to exercise the timeout path)
-  int ring_tile;         // 1 (with ring): each ring tile is one 2D tensor copy through
-                         // map_w / map_v instead of one bulk copy per column
-  // 2D maps over the level's W and V arenas (rows: N, columns: the level's
-  // kcap, row stride ld), box WR_ROWS rows x WR_BC columns; set when ring_tile
-  alignas(64) CUtensorMap map_w;
-  alignas(64) CUtensorMap map_v;
+  // aca_group_kernel: ring stages, doubles of a stage (GR_TC columns of the
+  // largest chunk), and the exchange slots (128 bytes a CTA, zeroed before launch)
+  int ring_stages, stage_elems;
+  unsigned char* slots;
+  // rows published for the next pass: two per CTA of pub_stride bytes (16 a
+  // column), tagged with this launch's number and the exchange's
+  unsigned char* pub;
+  int64_t pub_stride;
+  unsigned launch_tag;
+  // CTAs of the launch that ran out of work so far (zeroed before launch); once
+  // there are yield_at (0: never) the blocks still running pause
+  unsigned* idle;
+  int yield_at;
 };

@@ -6,7 +6,7 @@
 namespace hodlr_impl {
 
 int build_solve_plans(hodlr_t h, int nrhs) {
-  const int64_t N = h->n;
+  const int64_t N = h->n, ldp = h->ldp();
   int64_t zs_tot = 0;
   for (auto& L : h->lv) {
     int64_t t = 0;
@@ -43,7 +43,7 @@ int build_solve_plans(hodlr_t h, int nrhs) {
       a.A = L.V + mn;
       a.M = sn[p].kb;
       a.K = sp - mn + 1;
-      a.lda = (int)N;
+      a.lda = (int)ldp;
       a.B = h->X + mn;
       a.N = nrhs;
       a.ldb = (int)N;
@@ -54,7 +54,7 @@ int build_solve_plans(hodlr_t h, int nrhs) {
       b.A = L.V + sp + 1;
       b.M = sn[p].kt;
       b.K = mx - sp;
-      b.lda = (int)N;
+      b.lda = (int)ldp;
       b.B = h->X + sp + 1;
       b.N = nrhs;
       b.ldb = (int)N;
@@ -65,7 +65,7 @@ int build_solve_plans(hodlr_t h, int nrhs) {
       c.C = h->X + mn;
       c.ldc = (int)N;
       c.A = L.Yl + mn;
-      c.lda = (int)N;
+      c.lda = (int)ldp;
       c.M = sp - mn + 1;
       c.K = sn[p].kt;
       c.B = h->zs + sn[p].r_off + (h->sm_form ? 0 : sn[p].kb);
@@ -76,7 +76,7 @@ int build_solve_plans(hodlr_t h, int nrhs) {
       d.C = h->X + sp + 1;
       d.ldc = (int)N;
       d.A = L.Yl + sp + 1;
-      d.lda = (int)N;
+      d.lda = (int)ldp;
       d.M = mx - sp;
       d.K = sn[p].kb;
       d.B = h->zs + sn[p].r_off + (h->sm_form ? sn[p].kt : 0);

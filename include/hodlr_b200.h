@@ -345,15 +345,13 @@ int hodlr_gemm_device(int precision, int mode, int m, int n, int k, const double
 int hodlr_set_factor_in_place(hodlr_t h, int mode);
 
 /* How the ACA of the few-block top levels reads its W/V panel slices (no
- * counterpart in the reference): on = 2 (default) streams them through
- * per-warp shared-memory rings (used when N is even), each ring tile of 128
- * rows x 4 columns filled by one 2D tensor copy; 1 fills the tiles with one
- * bulk copy per panel column; 0 loads the panels per thread.  Measured ACA
- * time at N = 262144, modes 2 / 1 / 0: 0.188 / 0.218 / 0.260 s (2D Matern
- * cloud, tol 1e-8), 9.0 / 10.3 / 12.3 s (sphere, tol 1e-10).  Pivots, ranks
- * and W/V are the same in every mode; the setting applies from the next
- * compression.  HODLR_ACA_STREAMING=0, 1 or 2 in the environment sets the
- * mode of every new handle. */
+ * counterpart in the reference): on = 2 (default) or 1 streams them through
+ * a shared-memory ring per CTA, one bulk copy per panel column of a tile; 0
+ * loads the panels per thread.  Measured ACA time, streamed / per thread:
+ * 0.015 / 0.090 s (2D Matern cloud, N = 20011, tol 1e-8), 0.133 / 0.260 s
+ * (N = 262144).  Pivots, ranks and W/V are the same in every mode; the
+ * setting applies from the next compression.  HODLR_ACA_STREAMING=0, 1 or 2
+ * in the environment sets the mode of every new handle. */
 int hodlr_set_aca_streaming(hodlr_t h, int on);
 
 /* Bounded device waits (no counterpart in the reference).  The CTAs of one
