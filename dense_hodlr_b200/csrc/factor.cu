@@ -69,7 +69,8 @@ __global__ void y_init_kernel(double* Y, const double* W, int64_t ld, int kmax, 
 
 // log|det| pieces of the factorization: per leaf LU (column-major s x s,
 // final row permutation perm) and per capacitance LU (sd x sd, LAPACK-style
-// swaps piv): out = (sum_i log|u_ii|, #u_ii < 0, permutation parity).
+// swaps piv): out = (sum_i log|u_ii|, #u_ii < 0, permutation parity).  The
+// stored diagonal is that of the inverted triangles, 1 / u_ii.
 __global__ void leaf_logdet_kernel(const double* lu, const int64_t* lu_off, const int* leaf_min,
                                    const int* leaf_size, const int* perm, double* out) {
   if (threadIdx.x != 0) return;
@@ -80,7 +81,7 @@ __global__ void leaf_logdet_kernel(const double* lu, const int64_t* lu_off, cons
   int neg = 0;
   for (int i = 0; i < s; ++i) {
     const double d = g[(int64_t)i * s + i];
-    sum += log(fabs(d));
+    sum -= log(fabs(d));
     neg += d < 0.0;
   }
   unsigned char seen[160];
@@ -107,7 +108,7 @@ __global__ void schur_logdet_kernel(const SchurNode* nodes, const double* S, con
   int neg = 0, swaps = 0;
   for (int i = 0; i < n; ++i) {
     const double d = a[(int64_t)i * n + i];
-    sum += log(fabs(d));
+    sum -= log(fabs(d));
     neg += d < 0.0;
     swaps += p[i] != i;
   }
@@ -324,6 +325,17 @@ int do_factorize(hodlr_t h) {
     dfree(h, d_probs);
     dfree(h, d_tiles);
   }
+  {  // the solves multiply by inverted diagonal triangles (skinny.cu)
+    LeafSolveLaunch S{};
+    S.leaf_size = h->d_leaf_size;
+    S.lu_off = h->d_lu_off;
+    S.lu = h->d_lu;
+    int e = tri_invert_leaves_launch(S, nl, h->smax, h->stream);
+    if (e) return cuda_fail(h, (cudaError_t)e, "leaf triangles");
+    h->nlaunch += 1;
+    rc = check_phase(h, "factor: leaf triangles");
+    if (rc) return rc;
+  }
   // levels bottom-up
   for (int l = (int)h->lv.size() - 1; l >= 0; --l) {
     Level& L = h->lv[l];
@@ -349,6 +361,7 @@ int do_factorize(hodlr_t h) {
     }
     CK(dalloc(h, &L.S, (size_t)s_tot));
     CK(dalloc(h, &L.piv, (size_t)p_tot));
+    CK(dalloc(h, &L.perm, (size_t)p_tot));
     CK(dalloc(h, &L.d_nodes, (size_t)nn));
     CK(h2d_async(h, L.d_nodes, L.nodes.data(), sizeof(SchurNode) * nn));
     if (z_tot > h->z_cap) {
@@ -489,6 +502,11 @@ int do_factorize(hodlr_t h) {
       rc2 = check_phase(h, "factor: Y updates");
       if (rc2) return rc2;
     }
+    e = tri_invert_nodes_launch(S, L.perm, nn, L.max_sd, h->stream);
+    if (e) return cuda_fail(h, (cudaError_t)e, "capacitance triangles");
+    h->nlaunch += 1;
+    rc2 = check_phase(h, "factor: capacitance triangles");
+    if (rc2) return rc2;
   }
   CK(cudaEventRecord(h->ev1, h->stream));
   CK(cudaEventSynchronize(h->ev1));

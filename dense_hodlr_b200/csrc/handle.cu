@@ -61,7 +61,10 @@ void free_factor(hodlr_t h) {
     dfree(h, L.S);
     dfree(h, L.piv);
     dfree(h, L.d_nodes);
-    dfree(h, L.d_snodes);
+    dfree(h, L.perm);
+    dfree(h, L.d_caps);
+    dfree(h, L.d_stn);
+    dfree(h, L.d_snn);
     free_plan(h, L.tn);
     free_plan(h, L.nn);
     free_plan(h, L.stn);

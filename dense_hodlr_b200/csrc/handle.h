@@ -43,6 +43,7 @@
 #include "kmatvec.h"
 #include "lu.h"
 #include "rank_mlp.h"
+#include "skinny.h"
 
 int aca_launch(const AcaLaunch& L, int nt, int kcap_max, bool cooperative, cudaStream_t s);
 int aca_max_coresident(int nt, int kcap_max, int* per_sm);
@@ -97,8 +98,11 @@ struct Level {
   DevPlan tn, nn;          // factor GEMMs
   int solve_nrhs = -1;     // nrhs the solve plans were built for
   DevPlan stn, snn;        // solve GEMMs
-  SchurNode* d_snodes = nullptr;  // solve: r_off into the solve buffer
-  int64_t zs_elems = 0;
+  int* perm = nullptr;            // capacitance interchanges as permutations
+  CapNode* d_caps = nullptr;      // solve: the capacitance systems
+  TnItem* d_stn = nullptr;        // solve of few right-hand sides: V^T X, X -= Y y
+  NnItem* d_snn = nullptr;
+  int nstn = 0, nsnn = 0;
 };
 
 inline void block_geom(const Level& L, int q, int& r0, int& c0, int& m, int& n) {
@@ -204,7 +208,7 @@ struct hodlr_handle_s {
   cudaGraphExec_t sg_exec = nullptr;
   int sg_nrhs = -1;
   cudaStream_t sg_stream = nullptr;
-  const void* sg_key[4] = {nullptr, nullptr, nullptr, nullptr};
+  const void* sg_key[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   long sg_gen = -1;
   long long sg_launches = 0;
   bool sg_off = false;  // capture refused once: direct launches from then on
@@ -290,6 +294,10 @@ struct hodlr_handle_s {
   int gm_m = 0, gm_cols = 0;
   double* zs = nullptr;  // solve Schur right-hand sides
   int64_t zs_cap = 0;
+  double* spart = nullptr;  // solve: V^T X sums by chunk of rows
+  int64_t spart_cap = 0;
+  double* cap_big = nullptr;  // solve: capacitance systems beyond shared memory
+  int64_t cap_big_cap = 0;
   double* part = nullptr;
   int64_t part_cap = 0;
   unsigned* bar = nullptr;

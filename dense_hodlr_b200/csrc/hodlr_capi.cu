@@ -257,6 +257,8 @@ void hodlr_destroy(hodlr_t h) {
   dfree(h, h->Z);
   dfree(h, h->X);
   dfree(h, h->zs);
+  dfree(h, h->spart);
+  dfree(h, h->cap_big);
   dfree(h, h->ir_b);
   dfree(h, h->ir_x);
   dfree(h, h->ir_y);

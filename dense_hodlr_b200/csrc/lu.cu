@@ -6,13 +6,13 @@
 //                     of storeLRinTree (src/HODLR_Matrix.cpp:303-312) and
 //                     PartialPivLU(leafMatrix) (src/HODLR_Matrix.cpp:625).
 //  leaf_solve_kernel  applies the leaf LU to a tile of a wide panel: the
-//                     leafLU.solve of recLU_Factorize / recLU_Solve
-//                     (src/HODLR_Matrix.cpp:626,703).
+//                     leafLU.solve of recLU_Factorize (src/HODLR_Matrix.cpp:626).
 //  schur_form_kernel  builds S = [[I, V_b^T K_t^-1 U_t], [V_t^T K_b^-1 U_b, I]]
 //                     (src/HODLR_Matrix.cpp:663-673) from the level product Z.
 //  schur_lu_kernel    blocked partial-pivot LU of each node's S in place
 //                     (SchurLU = PartialPivLU(S), src/HODLR_Matrix.cpp:675).
-//  schur_solve_kernel y = S^-1 rhs by the stored LU (src/HODLR_Matrix.cpp:682,746).
+//  schur_solve_kernel y = S^-1 Z by the stored LU (src/HODLR_Matrix.cpp:682).
+// The right-hand sides of a solve go through skinny.cu.
 // Pivoting takes the first maximum |a| of the column, as PartialPivLU does.
 #include <algorithm>
 #include <vector>
@@ -628,129 +628,27 @@ __global__ void __launch_bounds__(256) big_rhs_update_kernel(SchurLaunch L, BigN
   }
 }
 
-// x <- U^-1 L^-1 x for `ncol` columns in shared memory (x[c*ldx+i]) with the
-// packed LU of an n x n matrix in global memory (column-major, ld n): the
-// capacitance matrices, up to a few thousand rows, with few columns per CTA.
-// Diagonal blocks of GB rows: one warp per column substitutes with the
-// block's row of A in registers (lane = row) and each solved value broadcast
-// by a shuffle, so the sequential chain is shuffles and FMAs, not memory
-// loads.  Rows outside the block: one thread per row loads its GB entries of
-// A once and updates every column.  The forward sweep performs exactly the
-// operations of a row-by-row substitution, in the same order (ascending
-// column); the backward sweep subtracts within a diagonal block in
-// descending column order.
-constexpr int GB = 32;
-
-__device__ void lu_solve_global(const double* __restrict__ a, int n, double* x, int ldx,
-                                int ncol) {
-  const int tid = threadIdx.x, NT = blockDim.x;
-  const int lane = tid & 31, wid = tid >> 5, NW = NT >> 5;
-  for (int b0 = 0; b0 < n; b0 += GB) {  // forward, unit lower
-    const int nb = min(GB, n - b0), be = b0 + nb;
-    if (wid < ncol) {
-      double ar[GB];  // A(b0 + lane, b0 + p), p < lane
-#pragma unroll
-      for (int p = 0; p < GB; ++p)
-        ar[p] = (p < lane && lane < nb) ? __ldg(a + (int64_t)(b0 + p) * n + b0 + lane) : 0.0;
-      for (int c = wid; c < ncol; c += NW) {
-        double* xc = x + c * ldx + b0;
-        double t = lane < nb ? xc[lane] : 0.0;
-#pragma unroll
-        for (int p = 0; p < GB - 1; ++p) {
-          const double xp = __shfl_sync(0xffffffffu, t, p);
-          if (p < lane) t = fma(-ar[p], xp, t);
-        }
-        if (lane < nb) xc[lane] = t;
-      }
-    }
-    __syncthreads();
-    for (int r = be + tid; r < n; r += NT) {
-      double ar[GB];  // A(r, b0 + p)
-#pragma unroll
-      for (int p = 0; p < GB; ++p) ar[p] = p < nb ? __ldg(a + (int64_t)(b0 + p) * n + r) : 0.0;
-      for (int c = 0; c < ncol; ++c) {
-        double* xc = x + c * ldx;
-        double t = xc[r];
-#pragma unroll
-        for (int p = 0; p < GB; ++p)
-          if (p < nb) t = fma(-ar[p], xc[b0 + p], t);
-        xc[r] = t;
-      }
-    }
-    __syncthreads();
-  }
-  for (int be = n; be > 0; be -= GB) {  // backward, upper
-    const int b0 = max(0, be - GB), nb = be - b0;
-    if (wid < ncol) {
-      double ar[GB];  // A(b0 + lane, b0 + p), p > lane
-#pragma unroll
-      for (int p = 0; p < GB; ++p)
-        ar[p] = (lane < p && p < nb) ? __ldg(a + (int64_t)(b0 + p) * n + b0 + lane) : 0.0;
-      const double ad = lane < nb ? __ldg(a + (int64_t)(b0 + lane) * n + b0 + lane) : 1.0;
-      for (int c = wid; c < ncol; c += NW) {
-        double* xc = x + c * ldx + b0;
-        double t = lane < nb ? xc[lane] : 0.0;
-#pragma unroll
-        for (int p = GB - 1; p >= 0; --p) {
-          if (p >= nb) continue;  // the same for every lane
-          if (lane == p) t = t / ad;
-          const double xp = __shfl_sync(0xffffffffu, t, p);
-          if (lane < p) t = fma(-ar[p], xp, t);
-        }
-        if (lane < nb) xc[lane] = t;
-      }
-    }
-    __syncthreads();
-    for (int r = tid; r < b0; r += NT) {
-      double ar[GB];  // A(r, b0 + p)
-#pragma unroll
-      for (int p = 0; p < GB; ++p) ar[p] = p < nb ? __ldg(a + (int64_t)(b0 + p) * n + r) : 0.0;
-      for (int c = 0; c < ncol; ++c) {
-        double* xc = x + c * ldx;
-        double t = xc[r];
-#pragma unroll
-        for (int p = 0; p < GB; ++p)
-          if (p < nb) t = fma(-ar[p], xc[b0 + p], t);
-        xc[r] = t;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// y = S^-1 rhs for `ncols` right-hand sides stored in R (ld sd) at r_off
-// (ncols < 0: N.coff columns); one CTA per (node, tile of STC columns).
-// WARP_SUBST selects lu_solve_global, whose short sequential chains suit the
-// solve (one CTA per node, latency-bound at the top levels); the ancestor
-// columns of the factorization (many CTAs per node, throughput-bound) keep
-// the 32-register blocked tile solve.
+// y = S^-1 Z for the ancestor columns (N.coff, at r_off, ld sd) of the nodes
+// with sd < skip_sd; one CTA per (node, tile of tc columns).
 constexpr int STC = 16;
 
-// tc columns per CTA (STC, or fewer where a column tile would not fit in
-// shared memory); in_smem == false: the columns are solved in place in
-// global memory (capacitance matrices too large for even one column).
-template <bool WARP_SUBST>
-__global__ void __launch_bounds__(256) schur_solve_kernel(SchurLaunch L, int ncols, int tc,
-                                                          bool in_smem, int skip_sd) {
-  extern __shared__ double xs_smem[];
+__global__ void __launch_bounds__(256) schur_solve_kernel(SchurLaunch L, int tc, int skip_sd) {
+  extern __shared__ double xs[];
   const int node = blockIdx.y;
   const SchurNode N = L.nodes[node];
   const int n = N.kb + N.kt;
   if (n >= skip_sd) return;  // left to the blocked solve
-  const int cols = ncols < 0 ? N.coff : ncols;
+  const int cols = N.coff;
   const int c0 = blockIdx.x * tc;
   if (c0 >= cols) return;
   const int nc = min(tc, cols - c0);
   const double* a = L.S + N.s_off;
   const int* piv = L.piv + N.p_off;
   double* R = L.R + N.r_off;
-  const int ldx = in_smem ? (n | 1) : n;
-  double* xs = in_smem ? xs_smem : R + (int64_t)c0 * n;
-  if (in_smem) {
-    for (int e = threadIdx.x; e < n * nc; e += blockDim.x) {
-      int i = e % n, c = e / n;
-      xs[c * ldx + i] = R[(int64_t)(c0 + c) * n + i];
-    }
+  const int ldx = n | 1;
+  for (int e = threadIdx.x; e < n * nc; e += blockDim.x) {
+    int i = e % n, c = e / n;
+    xs[c * ldx + i] = R[(int64_t)(c0 + c) * n + i];
   }
   __syncthreads();
   for (int c = threadIdx.x; c < nc; c += blockDim.x) {
@@ -769,15 +667,10 @@ __global__ void __launch_bounds__(256) schur_solve_kernel(SchurLaunch L, int nco
     }
   }
   __syncthreads();
-  if (WARP_SUBST)
-    lu_solve_global(a, n, xs, ldx, nc);
-  else
-    lu_solve_tile(GlobalLU{a, n}, n, xs, ldx, nc);
-  if (in_smem) {
-    for (int e = threadIdx.x; e < n * nc; e += blockDim.x) {
-      int i = e % n, c = e / n;
-      R[(int64_t)(c0 + c) * n + i] = xs[c * ldx + i];
-    }
+  lu_solve_tile(GlobalLU{a, n}, n, xs, ldx, nc);
+  for (int e = threadIdx.x; e < n * nc; e += blockDim.x) {
+    int i = e % n, c = e / n;
+    R[(int64_t)(c0 + c) * n + i] = xs[c * ldx + i];
   }
 }
 
@@ -905,9 +798,9 @@ int schur_solve_factor_launch(const SchurLaunch& L, int nnodes, const int* sd, i
     const size_t col_bytes = sizeof(double) * (size_t)(small_max | 1);
     const int tc = (int)std::max<size_t>(1, std::min<size_t>(STC, 200 * 1024 / col_bytes));
     const size_t smem = col_bytes * tc;
-    LCK(smem_opt_in((const void*)schur_solve_kernel<false>, smem));
-    schur_solve_kernel<false><<<dim3((coff + tc - 1) / tc, nnodes), 256, smem, s>>>(
-        L, -1, tc, true, SCHUR_BIG_SOLVE_SD);
+    LCK(smem_opt_in((const void*)schur_solve_kernel, smem));
+    schur_solve_kernel<<<dim3((coff + tc - 1) / tc, nnodes), 256, smem, s>>>(L, tc,
+                                                                             SCHUR_BIG_SOLVE_SD);
     LCK(cudaGetLastError());
     ++*launches;
   }
@@ -944,27 +837,6 @@ int schur_solve_factor_launch(const SchurLaunch& L, int nnodes, const int* sd, i
       }
       *launches += 1 + (j0 > 0);
     }
-  }
-  return (int)cudaGetLastError();
-}
-
-int schur_solve_launch(const SchurLaunch& L, int nnodes, int ncols, int max_cols, int max_sd,
-                       cudaStream_t s) {
-  if (nnodes == 0 || max_cols <= 0) return 0;
-  // columns per CTA: STC, fewer when a tile of them would exceed the
-  // shared-memory budget, none (in place in global memory) past one column
-  const size_t col_bytes = sizeof(double) * (size_t)(max_sd | 1);
-  constexpr size_t kBudget = 200 * 1024;
-  const int tc = (int)std::max<size_t>(1, std::min<size_t>(STC, kBudget / col_bytes));
-  const bool in_smem = col_bytes <= kBudget;
-  const size_t smem = in_smem ? col_bytes * tc : 0;
-  const dim3 grid((max_cols + tc - 1) / tc, nnodes);
-  if (ncols >= 0) {
-    LCK(smem_opt_in((const void*)schur_solve_kernel<true>, smem));
-    schur_solve_kernel<true><<<grid, 256, smem, s>>>(L, ncols, tc, in_smem, INT_MAX);
-  } else {
-    LCK(smem_opt_in((const void*)schur_solve_kernel<false>, smem));
-    schur_solve_kernel<false><<<grid, 256, smem, s>>>(L, ncols, tc, in_smem, INT_MAX);
   }
   return (int)cudaGetLastError();
 }

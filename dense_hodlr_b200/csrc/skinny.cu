@@ -1,0 +1,671 @@
+// The direct solve for a few right-hand sides: every kernel reads its matrix
+// once, as operand fragments of mma.m8n8k4.f64 loaded straight from global
+// memory, with the right-hand sides as the 8 columns of the other operand.
+//
+// What bounds them: the bytes of V, K^-1 U and the LUs (each entry is used
+// once per solve), and at the top of the tree the chain of block steps of a
+// triangular solve.  The 64-wide GEMM tiles these products ran through before
+// did 8 to 64 times the work of 8 or 1 columns, and the substitutions ran a
+// 32-step chain of shuffles per 32 rows in one CTA.
+//
+//  * Triangular solves multiply by inverted 64 x 64 diagonal triangles (formed
+//    once per factorization, in place), so a block step is two small products
+//    instead of a substitution: n / 64 steps each way.
+//  * Large capacitance systems run on a cluster of up to 8 CTAs: block rows
+//    dealt out cyclically, a solved block written to every CTA's shared memory.
+//  * V^T X is split over rows into items; their sums are added by the
+//    capacitance solve that reads them, in a fixed order.
+//
+// Measured on B200, a repeated direct solve end to end, 64-wide tiles and
+// one-CTA substitutions -> these kernels: N = 262144 2D, 8 columns 7.59 -> 2.44
+// ms (its panels' 3.2 GB at the copy rate: 0.49 ms); N = 30001 2D, 1 column 1.81
+// -> 0.90; sphere 16384 5.4 -> 1.2 ms; 40000-point cube 10.4 -> 3.6 ms; 1D 4096
+// 0.35 -> 0.09 ms.  What is left is the chain of the top capacitance solves
+// (2 n / 64 cluster steps of about 2 us) and, at 262144, the panels' reads.
+#include "skinny.h"
+
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int NB = TRI_NB;
+constexpr int SK_NT = 256;  // 8 warps
+
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// ------------------------------------------- inverted diagonal triangles
+// One CTA per diagonal block: threads 0..63 invert the unit lower triangle (a
+// column each), threads 64..127 the upper one, both by substitution in
+// registers over a copy in shared memory.  `m` rows of the block exist; the
+// rest is the identity.
+__device__ void invert_block(double* a, int ld, int m, double (*t)[NB + 2]) {
+  const int tid = threadIdx.x;
+  for (int e = tid; e < NB * NB; e += blockDim.x) {
+    const int i = e % NB, j = e / NB;
+    t[i][j] = i < m && j < m ? a[(int64_t)j * ld + i] : i == j ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  const int j = tid & (NB - 1);
+  if (tid < NB) t[tid][NB] = 1.0 / t[tid][tid];
+  __syncthreads();
+  double x[NB];
+  if (tid < NB) {
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      double v = i == j ? 1.0 : 0.0;
+#pragma unroll
+      for (int p = 0; p < i; ++p) v = fma(-t[i][p], x[p], v);
+      x[i] = v;
+    }
+  } else {
+#pragma unroll
+    for (int i = NB - 1; i >= 0; --i) {
+      double v = i == j ? 1.0 : 0.0;
+#pragma unroll
+      for (int p = NB - 1; p > i; --p) v = fma(-t[i][p], x[p], v);
+      x[i] = v * t[i][NB];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+    if (tid < NB ? i > j : i <= j) t[i][j] = x[i];
+  __syncthreads();
+  for (int e = tid; e < NB * NB; e += blockDim.x) {
+    const int i = e % NB, q = e / NB;
+    if (i < m && q < m) a[(int64_t)q * ld + i] = t[i][q];
+  }
+}
+
+__global__ void __launch_bounds__(2 * NB) invert_leaves_kernel(LeafSolveLaunch L) {
+  __shared__ double t[NB][NB + 2];
+  const int s = L.leaf_size[blockIdx.x], b0 = blockIdx.y * NB;
+  if (b0 >= s) return;
+  double* a = const_cast<double*>(L.lu) + L.lu_off[blockIdx.x];
+  invert_block(a + (int64_t)b0 * s + b0, s, min(NB, s - b0), t);
+}
+
+__global__ void __launch_bounds__(2 * NB) invert_nodes_kernel(SchurLaunch L, int* perm) {
+  __shared__ double t[NB][NB + 2];
+  const SchurNode N = L.nodes[blockIdx.x];
+  const int n = N.kb + N.kt, b0 = (int)(blockIdx.y - 1) * NB;
+  if (blockIdx.y == 0) {  // the interchanges, in order, as a permutation
+    int* p = perm + N.p_off;
+    const int* piv = L.piv + N.p_off;
+    // a chain of swaps: in shared memory where both arrays fit
+    constexpr int FIT = (int)(sizeof(t) / sizeof(int) / 2);
+    int* sp = reinterpret_cast<int*>(&t[0][0]);
+    const bool fit = n <= FIT;
+    int* q = fit ? sp : p;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      q[i] = i;
+      if (fit) sp[FIT + i] = piv[i];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int i = 0; i < n; ++i) {
+        const int r = fit ? sp[FIT + i] : piv[i];
+        if (r < i || r >= n) {  // not an LU interchange: skip and report
+          atomicOr(L.err, DEV_ERR_INDEX | DEV_ERR_AT_SOLVE_PIV);
+          continue;
+        }
+        const int v = q[i];
+        q[i] = q[r];
+        q[r] = v;
+      }
+    __syncthreads();
+    if (fit)
+      for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = sp[i];
+    return;
+  }
+  if (b0 >= n) return;
+  invert_block(L.S + N.s_off + (int64_t)b0 * n + b0, n, min(NB, n - b0), t);
+}
+
+// --------------------------------------------------- blocked triangular solve
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// D (8 x 8 NT tile) = A (8 x 64, fragments av) times a 64-row block of x, the
+// 16 MMAs of a tile in independent chains of 4.
+template <int NT>
+__device__ __forceinline__ void block_product(const double (&av)[NB / 4],
+                                              const double* const (&x)[NT],
+                                              double (&out)[NT][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int u = 0; u < NT; ++u) {
+    double acc[4][2];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[c][0] = acc[c][1] = 0.0;
+#pragma unroll
+    for (int k = 0; k < NB / 4; ++k) dmma(acc[k & 3], av[k], x[u][(4 * k + t) * 8 + g]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) out[u][e] = (acc[0][e] + acc[1][e]) + (acc[2][e] + acc[3][e]);
+  }
+}
+
+// x <- U^-1 L^-1 x with the packed LU `a` (n x n, inverted diagonal triangles)
+// in global memory.  The CTAs of a cluster (CL; otherwise one CTA) own block
+// rows rank, rank + size, ...: own[u][q][r][c] is column c of column tile u,
+// row r of owned block q.  Step b: its owner forms D_b x_b, one 8-row tile a
+// warp, and writes it to every CTA's xb[b mod 3]; all subtract A(b', b) x_b from
+// their blocks still to be solved.
+//
+// The chain is wait, update of the next block, its product, write: the owner
+// of the next step does those first and everybody else's updates overlap it.
+// A CTA arrives for step b + 1 once its updates of step b - 1 are done, so the
+// buffer of step b - 1 is free when step b + 2 is written: three buffers.  The
+// matrix fragments of both products are loaded before the wait.
+template <int NT, bool CL>
+__device__ void tri_solve(const double* __restrict__ a, int n, double* own, int own_blocks,
+                          double (*xb)[NT][NB][8]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  int rank = 0, size = 1;
+  if (CL) {
+    rank = (int)cg::this_cluster().block_rank();
+    size = (int)cg::this_cluster().num_blocks();
+  }
+  const int nb = (n + NB - 1) / NB;
+  auto ox = [&](int u, int q) { return own + ((int64_t)u * own_blocks + q) * NB * 8; };
+  double dv[NB / 4];
+  auto load_diag = [&](int dir, int b) {
+    const int row = 8 * w + g, gr = b * NB + row;
+#pragma unroll
+    for (int k = 0; k < NB / 4; ++k) {
+      const int col = 4 * k + t;
+      double v = dir == 0 && col == row ? 1.0 : 0.0;
+      if ((dir == 0 ? col < row : col >= row) && gr < n && b * NB + col < n)
+        v = __ldg(a + (int64_t)(b * NB + col) * n + gr);
+      dv[k] = v;
+    }
+  };
+  double av[NB / 4];
+  auto load_tile = [&](int q, int r8, int b) {
+    const int gr = (q * size + rank) * NB + 8 * r8 + g;
+#pragma unroll
+    for (int k = 0; k < NB / 4; ++k) {
+      const int col = b * NB + 4 * k + t;
+      av[k] = gr < n && col < n ? __ldg(a + (int64_t)col * n + gr) : 0.0;
+    }
+  };
+  // x_b = D_b x_b of this CTA's block b, to all CTAs' buffers
+  auto solve_block = [&](int b, int buf) {
+    const int q = CL ? b / size : b;
+    __syncthreads();  // the block's updates, by all warps
+    const double* x[NT];
+    double y[NT][2];
+#pragma unroll
+    for (int u = 0; u < NT; ++u) x[u] = ox(u, q);
+    block_product<NT>(dv, x, y);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+      const double2 v = make_double2(y[u][0], y[u][1]);
+      *reinterpret_cast<double2*>(ox(u, q) + (8 * w + g) * 8 + 2 * t) = v;
+      double* to = &xb[buf][u][8 * w + g][2 * t];
+      if (CL)
+        for (int r = 0; r < size; ++r)
+          *reinterpret_cast<double2*>(cg::this_cluster().map_shared_rank(to, r)) = v;
+      else
+        *reinterpret_cast<double2*>(to) = v;
+    }
+  };
+#pragma unroll 1
+  for (int dir = 0; dir < 2; ++dir) {  // forward with L, backward with U
+    auto block_of = [&](int step) { return dir == 0 ? step : nb - 1 - step; };
+    auto mine = [&](int step) { return step < nb && (!CL || block_of(step) % size == rank); };
+    if (mine(0)) {
+      load_diag(dir, block_of(0));
+      solve_block(block_of(0), 0);
+    }
+    if (CL) cluster_arrive();
+#pragma unroll 1
+    for (int step = 0; step < nb; ++step) {
+      const int b = block_of(step), buf = step % 3;
+      // the owned blocks behind step b (nearest first), in 8-row tiles over warps
+      int q0, q1;
+      if (dir == 0) {
+        q0 = (b + 1 - rank + size - 1) / size;
+        q1 = (nb - rank + size - 1) / size;
+      } else {
+        q0 = 0;
+        q1 = b > rank ? (b - rank + size - 1) / size : 0;
+      }
+      q0 = max(q0, 0);
+      const bool next = mine(step + 1);
+      if (q0 < q1) load_tile(dir == 0 ? q0 : q1 - 1, w, b);
+      if (next) load_diag(dir, block_of(step + 1));
+      if (CL) {
+        cluster_wait();
+        if (!next && step + 1 < nb) cluster_arrive();
+      } else {
+        __syncthreads();
+      }
+      const double* xs[NT];
+#pragma unroll
+      for (int u = 0; u < NT; ++u) xs[u] = &xb[buf][u][0][0];
+#pragma unroll 1
+      for (int i = 0; i < q1 - q0; ++i) {  // a warp takes tile w of every block
+        const int q = dir == 0 ? q0 + i : q1 - 1 - i;
+        double y[NT][2];
+        block_product<NT>(av, xs, y);
+        if (i + 1 < q1 - q0) load_tile(dir == 0 ? q + 1 : q - 1, w, b);
+#pragma unroll
+        for (int u = 0; u < NT; ++u) {
+          double2* x = reinterpret_cast<double2*>(ox(u, q) + (8 * w + g) * 8 + 2 * t);
+          double2 v = *x;
+          v.x -= y[u][0];
+          v.y -= y[u][1];
+          *x = v;
+        }
+        if (i == 0 && next) {
+          solve_block(block_of(step + 1), (step + 1) % 3);
+          if (CL) cluster_arrive();
+        }
+      }
+    }
+    // everybody's updates before the other direction's first block
+    if (CL)
+      cg::this_cluster().sync();
+    else
+      __syncthreads();
+  }
+}
+
+// ------------------------------------------------------------------ leaves
+// One CTA per leaf and 8 NT columns, the leaf's rows in shared memory.
+template <int NT>
+__global__ void __launch_bounds__(SK_NT) leaf_apply_kernel(LeafSolveLaunch L) {
+  extern __shared__ __align__(16) double dyn[];
+  const int leaf = blockIdx.x, c0 = blockIdx.y * 8 * NT;
+  const int r0 = L.leaf_min[leaf], s = L.leaf_size[leaf], nb = (s + NB - 1) / NB;
+  double* own = dyn;
+  auto xb = reinterpret_cast<double(*)[NT][NB][8]>(dyn + (size_t)NT * nb * NB * 8);  // 3 buffers
+  const int* perm = L.perm + r0;
+  for (int e = threadIdx.x; e < 8 * NT * nb * NB; e += SK_NT) {
+    const int i = e % (nb * NB), c = e / (nb * NB);
+    double v = 0.0;
+    if (i < s && c0 + c < L.ncols) {
+      const int pi = perm[i];
+      if (pi < 0 || pi >= s) {  // never written by a valid leaf LU: skip and report
+        if (L.err) atomicOr(L.err, DEV_ERR_INDEX | DEV_ERR_AT_LEAF_PERM);
+      } else {
+        v = L.X[(int64_t)(c0 + c) * L.ldx + r0 + pi];
+      }
+    }
+    own[((int64_t)(c >> 3) * nb * NB + i) * 8 + (c & 7)] = v;
+  }
+  __syncthreads();
+  tri_solve<NT, false>(L.lu + L.lu_off[leaf], s, own, nb, xb);
+  for (int e = threadIdx.x; e < 8 * NT * nb * NB; e += SK_NT) {
+    const int i = e % (nb * NB), c = e / (nb * NB);
+    if (i < s && c0 + c < L.ncols)
+      L.X[(int64_t)(c0 + c) * L.ldx + r0 + i] = own[((int64_t)(c >> 3) * nb * NB + i) * 8 + (c & 7)];
+  }
+}
+
+// ------------------------------------------------------------ capacitances
+// PARTS: r row-summed from the V^T X chunks, y row-major; otherwise r and y
+// column-major (n x nrhs at the node's z).  Cluster `size` CTAs per (node,
+// column tile); grid.x = node * size + rank.
+template <int NT, bool PARTS, bool CL>
+__global__ void __launch_bounds__(SK_NT) cap_solve_kernel(CapLaunch L, int nrhs, int own_max,
+                                                          unsigned* err) {
+  extern __shared__ __align__(16) double dyn[];
+  int rank = 0, size = 1;
+  if (CL) {
+    rank = (int)cg::this_cluster().block_rank();
+    size = (int)cg::this_cluster().num_blocks();
+  }
+  const CapNode N = L.nodes[blockIdx.x / size];
+  const int n = N.n, nb = (n + NB - 1) / NB, c0 = blockIdx.y * 8 * NT;
+  constexpr int NCP = 8 * NT;
+  const int ob = (nb - rank + size - 1) / size;  // owned blocks
+  // the owned rows: in shared memory, or (one CTA, more rows than fit) in L.big
+  const size_t mine = (size_t)NT * own_max * NB * 8;
+  double* own = L.big ? L.big + (blockIdx.y * gridDim.x + blockIdx.x) * mine : dyn;
+  auto xb = reinterpret_cast<double(*)[NT][NB][8]>(L.big ? dyn : dyn + mine);
+  const int* perm = L.perm + N.p_off;
+  for (int e = threadIdx.x; e < NCP * ob * NB; e += SK_NT) {
+    const int c = PARTS ? e % NCP : e / (ob * NB), lr = PARTS ? e / NCP : e % (ob * NB);
+    const int i = ((lr / NB) * size + rank) * NB + lr % NB;
+    double v = 0.0;
+    if (i < n) {
+      const int q = __ldg(perm + i);
+      if (q < 0 || q >= n) {
+        atomicOr(err, DEV_ERR_INDEX | DEV_ERR_AT_SOLVE_PIV);
+      } else if (PARTS) {
+        const int h = q >= N.off[0] && q < N.off[0] + N.m[0] ? 0 : 1;
+        const double* p = L.part + N.part[h] + (int64_t)(q - N.off[h]) * NCP + c;
+        const int64_t st = (int64_t)N.m[h] * NCP;
+#pragma unroll 16
+        for (int k = 0; k < N.chunks[h]; ++k) v += __ldg(p + k * st);
+      } else if (c0 + c < nrhs) {
+        v = L.z[N.z + (int64_t)(c0 + c) * n + q];
+      }
+    }
+    own[((int64_t)(c >> 3) * own_max * NB + lr) * 8 + (c & 7)] = v;
+  }
+  // column-major right-hand sides are overwritten by other CTAs of the cluster
+  if (CL)
+    cg::this_cluster().sync();
+  else
+    __syncthreads();
+  tri_solve<NT, CL>(L.S + N.s_off, n, own, own_max, xb);
+  for (int e = threadIdx.x; e < NCP * ob * NB; e += SK_NT) {
+    const int c = PARTS ? e % NCP : e / (ob * NB), lr = PARTS ? e / NCP : e % (ob * NB);
+    const int i = ((lr / NB) * size + rank) * NB + lr % NB;
+    if (i >= n) continue;
+    const double v = own[((int64_t)(c >> 3) * own_max * NB + lr) * 8 + (c & 7)];
+    if (PARTS)
+      L.z[N.z + (int64_t)i * NCP + c] = v;
+    else if (c0 + c < nrhs)
+      L.z[N.z + (int64_t)(c0 + c) * n + i] = v;
+  }
+}
+
+// ------------------------------------------------------------------ V^T X
+// One CTA per item: at most 128 columns of V, any number of rows, TN_ROWS at a
+// time.  A fragments are 8 columns of V by 4 row pairs: a lane loads rows 2t,
+// 2t + 1 of column g (16 bytes) and feeds them to two MMAs, the right-hand
+// sides with the same rows from shared memory.  Warps share the columns (16
+// each), or, when there are few, the rows, added in warp order.  Few, long
+// items keep the sums short that the capacitance solve adds up (a 504-row item
+// of all 357 columns left it 293 of them at N = 262144).
+constexpr int TN_PITCH = TN_ROWS + 8 + 8;  // a multiple of 8, odd in units of 64 bytes
+static_assert((TN_PITCH / 8) % 2 == 1, "column tiles must not share banks");
+
+template <int NT>
+__global__ void __launch_bounds__(SK_NT) skinny_tn_kernel(const TnItem* __restrict__ items,
+                                                          const double* __restrict__ X,
+                                                          int64_t ldx, int nrhs, int64_t ldv,
+                                                          double* __restrict__ part) {
+  extern __shared__ __align__(16) double dyn[];
+  constexpr int NCP = 8 * NT;
+  double* xs = dyn;                        // [NCP][TN_PITCH]
+  double* red = dyn + NCP * TN_PITCH;      // [8 warps][2][NT][32][2]
+  const TnItem it = items[blockIdx.x];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int cw = (it.M + 15) / 16;                             // 16-column groups, at most 8
+  const int mw = cw > 4 ? 8 : cw > 2 ? 4 : cw, rw = 8 / mw;    // warps over columns, over rows
+  const int wm = w % mw, wr = w / mw, m0 = 16 * wm;
+  const bool ok0 = m0 + g < it.M, ok1 = m0 + 8 + g < it.M;
+  double acc[2][NT][2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int u = 0; u < NT; ++u) acc[q][u][0] = acc[q][u][1] = 0.0;
+  for (int r0 = it.row0; r0 < it.row0 + it.rows;) {
+    const int base = r0 & ~1, end = min(it.row0 + it.rows, base + TN_ROWS);
+    const int lo = r0 - base, hi = end - base, span = (hi + 7) & ~7;
+    r0 = end;
+    __syncthreads();  // the last piece has been read
+    for (int e = threadIdx.x; e < NCP * span; e += SK_NT) {
+      const int c = e / span, i = e - c * span;
+      xs[c * TN_PITCH + i] =
+          c < nrhs && i >= lo && i < hi ? X[(int64_t)c * ldx + base + i] : 0.0;
+    }
+    __syncthreads();
+    if (m0 >= it.M) continue;
+    const double* v0 = it.V + (int64_t)(ok0 ? m0 + g : 0) * ldv + base + 2 * t;
+    const double* v1 = it.V + (int64_t)(ok1 ? m0 + 8 + g : 0) * ldv + base + 2 * t;
+    constexpr int U = 4;
+    for (int i0 = 8 * U * wr; i0 < span; i0 += 8 * U * rw) {
+      double2 a[2][U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + 8 * u, r = i + 2 * t;
+        double2 x = make_double2(0.0, 0.0), y = x;
+        if (r < hi) {  // the pair's second row may be padding: in the panel's storage
+          x = *reinterpret_cast<const double2*>(v0 + i);
+          y = *reinterpret_cast<const double2*>(v1 + i);
+        }
+        // rows outside the item may hold anything
+        const bool in0 = r >= lo && r < hi, in1 = r + 1 < hi;
+        a[0][u] = make_double2(ok0 && in0 ? x.x : 0.0, ok0 && in1 ? x.y : 0.0);
+        a[1][u] = make_double2(ok1 && in0 ? y.x : 0.0, ok1 && in1 ? y.y : 0.0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + 8 * u;
+        if (i >= span) break;
+#pragma unroll
+        for (int v = 0; v < NT; ++v) {
+          const double2 b =
+              *reinterpret_cast<const double2*>(xs + (8 * v + g) * TN_PITCH + i + 2 * t);
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            dmma(acc[q][v], a[q][u].x, b.x);
+            dmma(acc[q][v], a[q][u].y, b.y);
+          }
+        }
+      }
+    }
+  }
+  if (rw > 1) {  // the rows' shares, warps in order
+    auto slot = [&](int ww, int q, int v) {
+      return reinterpret_cast<double2*>(red + ((((ww * 2 + q) * NT + v) * 32) + lane) * 2);
+    };
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int v = 0; v < NT; ++v) *slot(w, q, v) = make_double2(acc[q][v][0], acc[q][v][1]);
+    __syncthreads();
+    if (wr == 0)
+      for (int r = 1; r < rw; ++r)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+          for (int v = 0; v < NT; ++v) {
+            const double2 o = *slot(wm + r * mw, q, v);
+            acc[q][v][0] += o.x;
+            acc[q][v][1] += o.y;
+          }
+  }
+  if (wr == 0)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int m = m0 + 8 * q + g;
+      if (m < it.M)
+#pragma unroll
+        for (int v = 0; v < NT; ++v)
+          *reinterpret_cast<double2*>(part + it.out + (int64_t)m * NCP + 8 * v + 2 * t) =
+              make_double2(acc[q][v][0], acc[q][v][1]);
+    }
+}
+
+// --------------------------------------------------------------- X -= Y y
+// One CTA per 128 rows (8 warps of 16).  A fragments are 8 row pairs by 4
+// columns: a lane loads rows 2g, 2g + 1 of column t (16 bytes; a column's
+// piece is a full 128-byte line) for two MMAs; y in shared memory, NN_K rows
+// at a time.
+constexpr int NN_K = 256;
+
+template <int NT>
+__global__ void __launch_bounds__(SK_NT) skinny_nn_kernel(const NnItem* __restrict__ items,
+                                                          double* __restrict__ X, int64_t ldx,
+                                                          int nrhs, int64_t ldy,
+                                                          const double* __restrict__ z) {
+  __shared__ __align__(16) double ys[NT][NN_K][8];
+  constexpr int NCP = 8 * NT;
+  const NnItem it = items[blockIdx.x];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int base = it.row0 & ~1;
+  const int r = base + 16 * w + 2 * g;  // this lane's row pair
+  const bool in0 = r >= it.row0 && r < it.row0 + it.rows, in1 = r + 1 < it.row0 + it.rows;
+  const bool load = r < it.row0 + it.rows;
+  double acc[2][NT][2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int v = 0; v < NT; ++v) acc[q][v][0] = acc[q][v][1] = 0.0;
+  for (int kb = 0; kb < it.K; kb += NN_K) {
+    const int kn = min(NN_K, it.K - kb), k4 = (kn + 3) & ~3;
+    __syncthreads();
+    for (int e = threadIdx.x; e < k4 * NCP; e += SK_NT) {
+      const int k = e / NCP, c = e % NCP;
+      ys[c >> 3][k][c & 7] = k < kn ? z[it.z + (int64_t)(kb + k) * NCP + c] : 0.0;
+    }
+    __syncthreads();
+    constexpr int U = 8;
+    for (int k0 = 0; k0 < k4; k0 += 4 * U) {
+      double2 a[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = k0 + 4 * u + t;
+        a[u] = load && k < kn
+                   ? *reinterpret_cast<const double2*>(it.Y + (int64_t)(kb + k) * ldy + r)
+                   : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (k0 + 4 * u >= k4) break;
+#pragma unroll
+        for (int v = 0; v < NT; ++v) {
+          const double b = ys[v][k0 + 4 * u + t][g];
+          dmma(acc[0][v], a[u].x, b);
+          dmma(acc[1][v], a[u].y, b);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < NT; ++v)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int c = 8 * v + 2 * t + q;
+      if (c >= nrhs) continue;
+      double* x = X + (int64_t)c * ldx + r;
+      if (in0) x[0] -= acc[0][v][q];
+      if (in1) x[1] -= acc[1][v][q];
+    }
+}
+
+#define LCK(call)                             \
+  do {                                        \
+    cudaError_t e__ = (call);                 \
+    if (e__ != cudaSuccess) return (int)e__;  \
+  } while (0)
+
+constexpr size_t kCapSmem = 200 * 1024;
+
+template <int NT, bool PARTS>
+int cap_launch(const CapLaunch& L, int nnodes, int nrhs, int max_sd, unsigned* err,
+               cudaStream_t s) {
+  const int nb = (max_sd + NB - 1) / NB;
+  auto smem_of = [&](int c) {
+    return sizeof(double) * 8 * NB * NT * (size_t)((nb + c - 1) / c + 3);
+  };
+  // CTAs of a cluster: at least two block rows each, and as few nodes as leave
+  // SMs over; more where the rows would not fit
+  int size = 1;
+  while (size < 8 && (smem_of(size) > kCapSmem || (nb >= 4 * size && nnodes * size < 148))) size *= 2;
+  if (L.big) size = 1;
+  const size_t smem = L.big ? sizeof(double) * 8 * NB * NT * 3 : smem_of(size);
+  if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
+  const dim3 grid(nnodes * size, (nrhs + 8 * NT - 1) / (8 * NT));
+  const int own = (nb + size - 1) / size;
+  if (size == 1) {
+    LCK(smem_opt_in((const void*)cap_solve_kernel<NT, PARTS, false>, smem));
+    cap_solve_kernel<NT, PARTS, false><<<grid, SK_NT, smem, s>>>(L, nrhs, own, err);
+    return (int)cudaGetLastError();
+  }
+  LCK(smem_opt_in((const void*)cap_solve_kernel<NT, PARTS, true>, smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(SK_NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = size;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, cap_solve_kernel<NT, PARTS, true>, L, nrhs, own, err);
+}
+
+}  // namespace
+
+int64_t cap_big_elems(int nnodes, int nrhs, int max_sd) {
+  const int nt = skinny_tiles(nrhs), nb = (max_sd + NB - 1) / NB;
+  if (sizeof(double) * 8 * NB * nt * (size_t)((nb + 7) / 8 + 3) <= kCapSmem) return 0;
+  return (int64_t)nnodes * ((nrhs + 8 * nt - 1) / (8 * nt)) * nt * nb * NB * 8;
+}
+
+int tri_invert_leaves_launch(const LeafSolveLaunch& L, int nleaves, int smax, cudaStream_t s) {
+  if (nleaves == 0) return 0;
+  invert_leaves_kernel<<<dim3(nleaves, (smax + NB - 1) / NB), 2 * NB, 0, s>>>(L);
+  return (int)cudaGetLastError();
+}
+
+int tri_invert_nodes_launch(const SchurLaunch& L, int* perm, int nnodes, int max_sd,
+                            cudaStream_t s) {
+  if (nnodes == 0) return 0;
+  invert_nodes_kernel<<<dim3(nnodes, 1 + (max_sd + NB - 1) / NB), 2 * NB, 0, s>>>(L, perm);
+  return (int)cudaGetLastError();
+}
+
+int leaf_apply_launch(const LeafSolveLaunch& L, int nleaves, int smax, cudaStream_t s) {
+  if (L.ncols <= 0 || nleaves == 0) return 0;
+  const int nt = skinny_tiles(L.ncols), nb = (smax + NB - 1) / NB;
+  const size_t smem = sizeof(double) * 8 * NB * nt * (size_t)(nb + 3);
+  const dim3 grid(nleaves, (L.ncols + 8 * nt - 1) / (8 * nt));
+  if (nt == 1) {
+    LCK(smem_opt_in((const void*)leaf_apply_kernel<1>, smem));
+    leaf_apply_kernel<1><<<grid, SK_NT, smem, s>>>(L);
+  } else {
+    LCK(smem_opt_in((const void*)leaf_apply_kernel<2>, smem));
+    leaf_apply_kernel<2><<<grid, SK_NT, smem, s>>>(L);
+  }
+  return (int)cudaGetLastError();
+}
+
+int skinny_tn_launch(const TnItem* items, int count, const double* X, int64_t ldx, int nrhs,
+                     int64_t ldv, double* part, cudaStream_t s) {
+  if (count == 0) return 0;
+  const int nt = skinny_tiles(nrhs);
+  const size_t smem = sizeof(double) * ((size_t)8 * nt * TN_PITCH + 8 * 2 * nt * 64);
+  if (nt == 1) {
+    LCK(smem_opt_in((const void*)skinny_tn_kernel<1>, smem));
+    skinny_tn_kernel<1><<<count, SK_NT, smem, s>>>(items, X, ldx, nrhs, ldv, part);
+  } else {
+    LCK(smem_opt_in((const void*)skinny_tn_kernel<2>, smem));
+    skinny_tn_kernel<2><<<count, SK_NT, smem, s>>>(items, X, ldx, nrhs, ldv, part);
+  }
+  return (int)cudaGetLastError();
+}
+
+int skinny_nn_launch(const NnItem* items, int count, double* X, int64_t ldx, int nrhs, int64_t ldy,
+                     const double* z, cudaStream_t s) {
+  if (count == 0) return 0;
+  if (skinny_tiles(nrhs) == 1)
+    skinny_nn_kernel<1><<<count, SK_NT, 0, s>>>(items, X, ldx, nrhs, ldy, z);
+  else
+    skinny_nn_kernel<2><<<count, SK_NT, 0, s>>>(items, X, ldx, nrhs, ldy, z);
+  return (int)cudaGetLastError();
+}
+
+int cap_solve_launch(const CapLaunch& L, int nnodes, int nrhs, int max_sd, bool parts,
+                     unsigned* err, cudaStream_t s) {
+  if (nnodes == 0 || nrhs <= 0) return 0;
+  if (skinny_tiles(nrhs) == 1)
+    return parts ? cap_launch<1, true>(L, nnodes, nrhs, max_sd, err, s)
+                 : cap_launch<1, false>(L, nnodes, nrhs, max_sd, err, s);
+  return parts ? cap_launch<2, true>(L, nnodes, nrhs, max_sd, err, s)
+               : cap_launch<2, false>(L, nnodes, nrhs, max_sd, err, s);
+}

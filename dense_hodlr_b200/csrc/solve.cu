@@ -5,36 +5,133 @@
 
 namespace hodlr_impl {
 
+// Few FP64 right-hand sides run through the row-major kernels of skinny.cu;
+// more, and the tensor-core precisions, through the grouped GEMMs.
+static bool few_rhs(hodlr_t h, int nrhs) {
+  return h->gemm_prec == HODLR_GEMM_FP64 && nrhs <= SKINNY_MAX;
+}
+
+// V^T X and X updates of a level as items of skinny.cu, and its capacitance
+// nodes; *z and *part become the workspace elements they use.
+static int build_few(hodlr_t h, Level& L, int nrhs, int64_t* z, int64_t* part) {
+  const int nn = (int)L.nmin.size(), ncp = 8 * skinny_tiles(nrhs);
+  // rows of an item: about four CTAs an SM over the level's rows and blocks of
+  // TN_COLS columns, a multiple of 8
+  int64_t row_blocks = 0;
+  for (int p = 0; p < nn; ++p)
+    row_blocks +=
+        (int64_t)(L.nsplit[p] - L.nmin[p] + 1) * ((L.nodes[p].kb + TN_COLS - 1) / TN_COLS) +
+        (int64_t)(L.nmax[p] - L.nsplit[p]) * ((L.nodes[p].kt + TN_COLS - 1) / TN_COLS);
+  const int chunk = (int)std::max<int64_t>(64, (row_blocks / (4 * h->num_sms) + 7) / 8 * 8);
+  std::vector<TnItem> tn;
+  std::vector<NnItem> up;
+  std::vector<CapNode> caps((size_t)nn);
+  *z = *part = 0;
+  for (int p = 0; p < nn; ++p) {
+    const SchurNode& sn = L.nodes[p];
+    const int sd = sn.kb + sn.kt;
+    CapNode& c = caps[p];
+    c = CapNode{};
+    c.n = sd;
+    c.s_off = sn.s_off;
+    c.p_off = sn.p_off;
+    c.z = *z;
+    // V of the bottom block lives on the top rows, V of the top block on the bottom ones
+    const int lo[2] = {L.nmin[p], L.nsplit[p] + 1}, hi[2] = {L.nsplit[p] + 1, L.nmax[p] + 1};
+    const int m[2] = {sn.kb, sn.kt}, off[2] = {h->sm_form ? sn.kt : 0, h->sm_form ? 0 : sn.kb};
+    for (int q = 0; q < 2; ++q) {
+      const int rows = hi[q] - lo[q], nch = m[q] > 0 ? (rows + chunk - 1) / chunk : 0;
+      const int per = nch ? ((rows + nch - 1) / nch + 7) / 8 * 8 : 0;
+      c.off[q] = off[q];
+      c.m[q] = m[q];
+      c.part[q] = *part;
+      for (int r = 0; nch && r < rows; r += per) {
+        for (int c0 = 0; c0 < m[q]; c0 += TN_COLS)
+          tn.push_back({L.V + (int64_t)c0 * h->ldp(), lo[q] + r, std::min(per, rows - r),
+                        std::min(TN_COLS, m[q] - c0), 0, *part + (int64_t)c0 * ncp});
+        *part += (int64_t)m[q] * ncp;
+        ++c.chunks[q];
+      }
+      // the half's own U columns: K^-1 U of the top block on the top rows
+      const int k = q == 0 ? sn.kt : sn.kb;
+      const int64_t zy = *z + (int64_t)(q == 0 ? (h->sm_form ? 0 : sn.kb) : (h->sm_form ? sn.kt : 0)) * ncp;
+      for (int r = lo[q]; k > 0 && r < hi[q];) {
+        const int end = std::min(hi[q], (r & ~1) + 128);
+        up.push_back({L.Yl, r, end - r, k, 0, zy});
+        r = end;
+      }
+    }
+    *z += (int64_t)sd * ncp;
+  }
+  dfree(h, L.d_stn);
+  dfree(h, L.d_snn);
+  dfree(h, L.d_caps);
+  CK(dalloc(h, &L.d_stn, tn.size()));
+  CK(dalloc(h, &L.d_snn, up.size()));
+  CK(dalloc(h, &L.d_caps, caps.size()));
+  CK(h2d_async(h, L.d_stn, tn.data(), sizeof(TnItem) * tn.size()));
+  CK(h2d_async(h, L.d_snn, up.data(), sizeof(NnItem) * up.size()));
+  CK(h2d_async(h, L.d_caps, caps.data(), sizeof(CapNode) * caps.size()));
+  L.nstn = (int)tn.size();
+  L.nsnn = (int)up.size();
+  return HODLR_OK;
+}
+
 int build_solve_plans(hodlr_t h, int nrhs) {
   const int64_t N = h->n, ldp = h->ldp();
-  int64_t zs_tot = 0;
+  const bool few = few_rhs(h, nrhs);
+  int64_t zs_tot = 0, big = 0;
   for (auto& L : h->lv) {
     int64_t t = 0;
-    for (auto& sn : L.nodes) t += (int64_t)(sn.kb + sn.kt) * nrhs;
+    for (auto& sn : L.nodes)
+      t += (int64_t)(sn.kb + sn.kt) * (few ? 8 * skinny_tiles(nrhs) : nrhs);
     zs_tot = std::max(zs_tot, t);
+    big = std::max(big, cap_big_elems((int)L.nodes.size(), nrhs, L.max_sd));
   }
   if (zs_tot > h->zs_cap) {
     dfree(h, h->zs);
     CK(dalloc(h, &h->zs, (size_t)zs_tot));
     h->zs_cap = zs_tot;
+    for (auto& L : h->lv) L.solve_nrhs = -1;  // the GEMM plans point into it
+  }
+  if (big > h->cap_big_cap) {
+    dfree(h, h->cap_big);
+    CK(dalloc(h, &h->cap_big, (size_t)big));
+    h->cap_big_cap = big;
   }
   if (nrhs > h->x_cols) {
     dfree(h, h->X);
     CK(dalloc(h, &h->X, (size_t)(N * nrhs)));
     h->x_cols = nrhs;
+    for (auto& L : h->lv) L.solve_nrhs = -1;  // the GEMM plans point into it
   }
+  int64_t part_tot = 0;
   for (auto& L : h->lv) {
     if (L.solve_nrhs == nrhs) continue;
+    if (few) {
+      int64_t z = 0, part = 0;
+      int rc = build_few(h, L, nrhs, &z, &part);
+      if (rc) return rc;
+      part_tot = std::max(part_tot, part);
+      L.solve_nrhs = nrhs;
+      continue;
+    }
     const int nn = (int)L.nmin.size();
     std::vector<SchurNode> sn = L.nodes;
+    std::vector<CapNode> caps((size_t)nn);
     int64_t off = 0;
-    for (auto& s : sn) {
-      s.r_off = off;
-      off += (int64_t)(s.kb + s.kt) * nrhs;
+    for (int p = 0; p < nn; ++p) {
+      sn[p].r_off = off;
+      caps[p] = CapNode{};
+      caps[p].n = sn[p].kb + sn[p].kt;
+      caps[p].s_off = sn[p].s_off;
+      caps[p].p_off = sn[p].p_off;
+      caps[p].z = off;
+      off += (int64_t)caps[p].n * nrhs;
     }
-    dfree(h, L.d_snodes);
-    CK(dalloc(h, &L.d_snodes, (size_t)nn));
-    CK(h2d_async(h, L.d_snodes, sn.data(), sizeof(SchurNode) * nn));
+    dfree(h, L.d_caps);
+    CK(dalloc(h, &L.d_caps, (size_t)nn));
+    CK(h2d_async(h, L.d_caps, caps.data(), sizeof(CapNode) * nn));
     std::vector<GemmProblem> tn, up;
     for (int p = 0; p < nn; ++p) {
       const int sd = sn[p].kb + sn[p].kt;
@@ -90,6 +187,11 @@ int build_solve_plans(hodlr_t h, int nrhs) {
     if (rc) return rc;
     L.solve_nrhs = nrhs;
   }
+  if (part_tot > h->spart_cap) {
+    dfree(h, h->spart);
+    CK(dalloc(h, &h->spart, (size_t)part_tot));
+    h->spart_cap = part_tot;
+  }
   return HODLR_OK;
 }
 
@@ -106,39 +208,50 @@ int solve_in_place(hodlr_t h, int nrhs) {
   S.ldx = N;
   S.ncols = nrhs;
   S.err = h->d_err;
-  int e = leaf_solve_launch(S, (int)h->leaf_min.size(), h->smax, h->stream);
-  if (e) return cuda_fail(h, (cudaError_t)e, "leaf_solve");
+  int e = leaf_apply_launch(S, (int)h->leaf_min.size(), h->smax, h->stream);
+  if (e) return cuda_fail(h, (cudaError_t)e, "leaf_apply");
   h->nlaunch += 1;
   int rc = check_phase(h, "solve: leaves");
   if (rc) return rc;
+  const bool few = few_rhs(h, nrhs);
   for (int l = (int)h->lv.size() - 1; l >= 0; --l) {
     Level& L = h->lv[l];
     const int nn = (int)L.nmin.size();
-    e = run_tn(h, L.stn);
-    if (e) return cuda_fail(h, (cudaError_t)e, "solve gemm_tn");
+    if (few) {
+      e = skinny_tn_launch(L.d_stn, L.nstn, h->X, N, nrhs, h->ldp(), h->spart, h->stream);
+      h->nlaunch += 1;
+    } else {
+      e = run_tn(h, L.stn);
+    }
+    if (e) return cuda_fail(h, (cudaError_t)e, "solve V^T X");
     rc = check_phase(h, "solve: V^T X products");
     if (!rc && h->checked)
       for (const auto& sn : L.nodes) {
         const int64_t sd = sn.kb + sn.kt;
         rc = check_extent(h, L.S + sn.s_off, sizeof(double) * sd * sd, "capacitance LU", "solve");
-        if (!rc) rc = check_extent(h, L.piv + sn.p_off, sizeof(int) * sd, "pivots", "solve");
+        if (!rc) rc = check_extent(h, L.perm + sn.p_off, sizeof(int) * sd, "permutation", "solve");
         if (rc) break;
       }
     if (rc) return rc;
-    SchurLaunch SL;
-    SL.nodes = L.d_snodes;
-    SL.S = L.S;
-    SL.Z = nullptr;
-    SL.R = h->zs;
-    SL.piv = L.piv;
-    SL.err = h->d_err;
-    e = schur_solve_launch(SL, nn, nrhs, nrhs, L.max_sd, h->stream);
-    if (e) return cuda_fail(h, (cudaError_t)e, "solve schur");
+    CapLaunch CL;
+    CL.nodes = L.d_caps;
+    CL.S = L.S;
+    CL.perm = L.perm;
+    CL.part = h->spart;
+    CL.z = h->zs;
+    CL.big = cap_big_elems(nn, nrhs, L.max_sd) ? h->cap_big : nullptr;
+    e = cap_solve_launch(CL, nn, nrhs, L.max_sd, few, h->d_err, h->stream);
+    if (e) return cuda_fail(h, (cudaError_t)e, "solve capacitance");
     h->nlaunch += 1;
     rc = check_phase(h, "solve: capacitance");
     if (rc) return rc;
-    e = run_nn(h, L.snn);
-    if (e) return cuda_fail(h, (cudaError_t)e, "solve gemm_nn");
+    if (few) {
+      e = skinny_nn_launch(L.d_snn, L.nsnn, h->X, N, nrhs, h->ldp(), h->zs, h->stream);
+      h->nlaunch += 1;
+    } else {
+      e = run_nn(h, L.snn);
+    }
+    if (e) return cuda_fail(h, (cudaError_t)e, "solve X update");
     rc = check_phase(h, "solve: X updates");
     if (rc) return rc;
   }
@@ -150,10 +263,11 @@ int solve_in_place(hodlr_t h, int nrhs) {
 // are the same (one launch instead of ~4 per level).
 int solve_fast(hodlr_t h, int nrhs) {
   if (h->sg_off || h->checked) return solve_in_place(h, nrhs);
-  const void* key[4] = {h->X, h->zs, h->ws, (const void*)(intptr_t)(h->gemm_prec + 1)};
+  const void* key[6] = {h->X, h->zs, h->ws, (const void*)(intptr_t)(h->gemm_prec + 1), h->spart,
+                        h->cap_big};
   bool same = h->sg_exec && h->sg_nrhs == nrhs && h->sg_stream == h->stream &&
               h->sg_gen == h->factor_gen;
-  for (int i = 0; i < 4 && same; ++i) same = key[i] == h->sg_key[i];
+  for (int i = 0; i < 6 && same; ++i) same = key[i] == h->sg_key[i];
   if (!same) {
     drop_solve_graph(h);
     const long long before = h->nlaunch;
@@ -179,7 +293,7 @@ int solve_fast(hodlr_t h, int nrhs) {
     h->sg_nrhs = nrhs;
     h->sg_stream = h->stream;
     h->sg_gen = h->factor_gen;
-    for (int i = 0; i < 4; ++i) h->sg_key[i] = key[i];
+    for (int i = 0; i < 6; ++i) h->sg_key[i] = key[i];
     h->sg_launches = h->nlaunch - before;
     h->nlaunch = before;
   }
