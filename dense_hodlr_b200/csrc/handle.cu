@@ -117,7 +117,7 @@ int ensure_ws(hodlr_t h, int64_t elems) {
 // h2d_async is free again.
 static cudaError_t drained(hodlr_t h, cudaError_t e) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (e == cudaSuccess) h->pin_used = 0;
+  if (e == cudaSuccess) h->pin_cur = h->pin_used = 0;
   return e;
 }
 cudaError_t h2d(hodlr_t h, void* dst, const void* src, size_t bytes) {
@@ -127,36 +127,135 @@ cudaError_t d2h(hodlr_t h, void* dst, const void* src, size_t bytes) {
   return drained(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream));
 }
 
+// Pinned staging blocks, shared by all handles of the process.  Pinning and
+// unpinning memory costs milliseconds (8 MB: 5 to 8 ms, now and then 100), more
+// than a 4096-point system takes to solve, so a destroyed handle's blocks wait
+// here, at most PIN_KEEP bytes, for the next handle; hodlr_trim_device_memory
+// frees them.  A block belongs to one handle at a time and changes hands only
+// after its stream has drained.  Measured on B200, a new system built, factored
+// and solved once, blocks pinned per handle -> kept: N = 1024 13.4 -> 2.0 ms,
+// N = 4096 13.2 -> 2.9 ms.
+static std::mutex g_pin_mu;
+static std::vector<PinBlock> g_pins;
+static size_t g_pin_bytes = 0;
+constexpr size_t PIN_BLOCK = (size_t)1 << 20;
+constexpr size_t PIN_HANDLE = (size_t)8 << 20;  // a handle waits instead of going on
+constexpr size_t PIN_KEEP = (size_t)64 << 20;
+
+static cudaError_t take_pin(size_t need, PinBlock* out) {
+  {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    size_t best = g_pins.size();  // the smallest that fits
+    for (size_t i = 0; i < g_pins.size(); ++i)
+      if (g_pins[i].bytes >= need && (best == g_pins.size() || g_pins[i].bytes < g_pins[best].bytes))
+        best = i;
+    if (best < g_pins.size()) {
+      *out = g_pins[best];
+      g_pins[best] = g_pins.back();
+      g_pins.pop_back();
+      g_pin_bytes -= out->bytes;
+      return cudaSuccess;
+    }
+  }
+  PinBlock b;
+  b.bytes = (need + PIN_BLOCK - 1) / PIN_BLOCK * PIN_BLOCK;
+  // any thread's next device may use it; and a failure is not left behind
+  const cudaError_t e = cudaHostAlloc((void**)&b.p, b.bytes, cudaHostAllocPortable);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return e;
+  }
+  *out = b;
+  return cudaSuccess;
+}
+
+static void give_pin(const PinBlock& b) {
+  {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    if (g_pin_bytes + b.bytes <= PIN_KEEP) {
+      g_pins.push_back(b);
+      g_pin_bytes += b.bytes;
+      return;
+    }
+  }
+  cudaFreeHost(b.p);
+}
+
+void release_pins(hodlr_t h) {
+  for (auto& b : h->pins) give_pin(b);
+  h->pins.clear();
+  h->pin_cur = h->pin_used = 0;
+}
+
+void trim_pins() {
+  std::vector<PinBlock> all;
+  {
+    std::lock_guard<std::mutex> lk(g_pin_mu);
+    all.swap(g_pins);
+    g_pin_bytes = 0;
+  }
+  for (auto& b : all) cudaFreeHost(b.p);
+}
+
 // A pageable cudaMemcpyAsync to the device synchronises the stream before it
 // starts, so the host would wait for every queued kernel before planning the
 // next launches.  These uploads go through pinned staging memory instead:
-// the host copies the bytes there and queues the copy.  The staging area is
-// reused once the stream has drained (any of the calls above), or here when
-// it is full.
+// the host copies the bytes there and queues the copy.  The blocks are filled
+// one after the other and reused once the stream has drained (any of the calls
+// above), or here when a handle has filled PIN_HANDLE bytes.
 cudaError_t h2d_async(hodlr_t h, void* dst, const void* src, size_t bytes) {
   if (bytes == 0) return cudaSuccess;
   const size_t need = (bytes + 255) & ~(size_t)255;
-  if (h->pin_used + need > h->pin_cap) {
-    cudaError_t e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return e;
+  while (h->pin_cur < h->pins.size() && h->pin_used + need > h->pins[h->pin_cur].bytes) {
+    ++h->pin_cur;
     h->pin_used = 0;
-    if (need > h->pin_cap) {
-      if (h->pin) cudaFreeHost(h->pin);
-      h->pin = nullptr;
-      h->pin_cap = 0;
-      const size_t cap = std::max(need, (size_t)8 << 20);
-      e = cudaMallocHost((void**)&h->pin, cap);
-      if (e != cudaSuccess) {
-        h->pin = nullptr;
-        return e;
-      }
-      h->pin_cap = cap;
+  }
+  if (h->pin_cur == h->pins.size()) {
+    size_t have = 0;
+    for (auto& b : h->pins) have += b.bytes;
+    if (have && have + need > PIN_HANDLE) {
+      const cudaError_t e = cudaStreamSynchronize(h->stream);
+      if (e != cudaSuccess) return e;
+      h->pin_cur = h->pin_used = 0;
+      while (h->pin_cur < h->pins.size() && need > h->pins[h->pin_cur].bytes) ++h->pin_cur;
+      if (h->pin_cur == h->pins.size()) release_pins(h);  // one too small: take a larger one
+    }
+    if (h->pin_cur == h->pins.size()) {
+      PinBlock b;
+      const cudaError_t e = take_pin(need, &b);
+      if (e != cudaSuccess) return e;
+      h->pins.push_back(b);
     }
   }
-  char* p = h->pin + h->pin_used;
+  char* p = h->pins[h->pin_cur].p + h->pin_used;
   memcpy(p, src, bytes);
   h->pin_used += need;
   return cudaMemcpyAsync(dst, p, bytes, cudaMemcpyHostToDevice, h->stream);
+}
+
+// A[i][j] <-> A[j][i], 32 x 32 tiles swapped in pairs: one read and one write of
+// the matrix at device bandwidth, where the host's strided pass over a row-major
+// matrix took 17 ms at n = 2001.
+__global__ void __launch_bounds__(256) transpose_square_kernel(double* A, int n) {
+  __shared__ double up[32][33], lo[32][33];
+  const int r = blockIdx.y * 32, c = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
+  if (c < r) return;
+  for (int k = ty; k < 32; k += 8) {
+    if (r + k < n && c + tx < n) up[k][tx] = A[(int64_t)(r + k) * n + c + tx];
+    if (c + k < n && r + tx < n) lo[k][tx] = A[(int64_t)(c + k) * n + r + tx];
+  }
+  __syncthreads();
+  for (int k = ty; k < 32; k += 8) {
+    if (r + k < n && c + tx < n) A[(int64_t)(r + k) * n + c + tx] = lo[tx][k];
+    if (c != r && c + k < n && r + tx < n) A[(int64_t)(c + k) * n + r + tx] = up[tx][k];
+  }
+}
+
+cudaError_t transpose_square(double* A, int n, cudaStream_t s) {
+  const int t = (n + 31) / 32;
+  if (t > 65535) return cudaErrorInvalidValue;
+  transpose_square_kernel<<<dim3(t, t), dim3(32, 8), 0, s>>>(A, n);
+  return cudaGetLastError();
 }
 cudaError_t copy2d(hodlr_t h, void* dst, size_t dpitch, const void* src, size_t spitch,
                    size_t width, size_t rows, cudaMemcpyKind kind) {

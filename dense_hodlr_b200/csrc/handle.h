@@ -59,6 +59,11 @@ int aca_group_launch(const AcaLaunch& L, int v, size_t smem, bool cooperative, c
 
 namespace hodlr_impl {
 
+struct PinBlock {  // pinned host staging memory
+  char* p = nullptr;
+  size_t bytes = 0;
+};
+
 struct DevPlan {  // a grouped GEMM uploaded to the device
   GemmProblem* probs = nullptr;
   int4* tiles = nullptr;
@@ -273,8 +278,8 @@ struct hodlr_handle_s {
   int in_place = -1;
   bool w_consumed = false;  // some level's W holds K^-1 U: recompress before refactoring
   // pinned host staging of uploads that do not wait for the stream (h2d_async)
-  char* pin = nullptr;
-  size_t pin_cap = 0, pin_used = 0;
+  std::vector<hodlr_impl::PinBlock> pins;
+  size_t pin_cur = 0, pin_used = 0;  // the block being filled and how far
   double* ws = nullptr;  // GEMM split-K / kmatvec workspace
   int64_t ws_cap = 0;
   double* Z = nullptr;  // per-level Schur right-hand sides (factor)
@@ -365,6 +370,12 @@ cudaError_t h2d(hodlr_t h, void* dst, const void* src, size_t bytes);
 // Upload without waiting: src is copied into the handle's pinned staging
 // memory at once (src may be reused on return) and the copy is queued.
 cudaError_t h2d_async(hodlr_t h, void* dst, const void* src, size_t bytes);
+// The handle's staging blocks back to the library's pool; its stream has drained.
+void release_pins(hodlr_t h);
+// The free staging blocks back to the system.
+void trim_pins();
+// Device side of a row-major upload: the n x n matrix at A transposed in place.
+cudaError_t transpose_square(double* A, int n, cudaStream_t s);
 cudaError_t d2h(hodlr_t h, void* dst, const void* src, size_t bytes);
 cudaError_t copy2d(hodlr_t h, void* dst, size_t dpitch, const void* src, size_t spitch,
                    size_t width, size_t rows, cudaMemcpyKind kind);

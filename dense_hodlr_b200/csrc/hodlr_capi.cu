@@ -34,7 +34,8 @@ int hodlr_create_kernel(hodlr_t* out, int n, int dim, const double* pts,
   return HODLR_OK;
 }
 
-int hodlr_create_dense(hodlr_t* out, int n, const double* A, int lda, int leaf_size) {
+static int create_dense(hodlr_t* out, int n, const double* A, int lda, int leaf_size,
+                        bool rows) {
   if (!out || n <= 0 || !A || lda < n || leaf_size < 1) return HODLR_ERR_ARG;
   *out = nullptr;
   hodlr_t h = new hodlr_handle_s();
@@ -48,6 +49,7 @@ int hodlr_create_dense(hodlr_t* out, int n, const double* A, int lda, int leaf_s
     if (e == cudaSuccess)
       e = copy2d(h, h->d_A, sizeof(double) * n, A, sizeof(double) * lda, sizeof(double) * n, n,
                  cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && rows) e = transpose_square(h->d_A, n, h->stream);
     if (e != cudaSuccess) rc = cuda_fail(h, e, "matrix upload");
   }
   if (rc) {
@@ -56,6 +58,14 @@ int hodlr_create_dense(hodlr_t* out, int n, const double* A, int lda, int leaf_s
   }
   *out = h;
   return HODLR_OK;
+}
+
+int hodlr_create_dense(hodlr_t* out, int n, const double* A, int lda, int leaf_size) {
+  return create_dense(out, n, A, lda, leaf_size, false);
+}
+
+int hodlr_create_dense_rows(hodlr_t* out, int n, const double* A, int lda, int leaf_size) {
+  return create_dense(out, n, A, lda, leaf_size, true);
 }
 
 int hodlr_create_dense_device(hodlr_t* out, int n, int leaf_size, double** dA, int64_t* ld) {
@@ -285,8 +295,10 @@ void hodlr_destroy(hodlr_t h) {
   dfree(h, h->d_err);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
-  if (h->stream) cudaStreamSynchronize(h->stream);
-  if (h->pin) cudaFreeHost(h->pin);
+  if (h->stream && cudaStreamSynchronize(h->stream) == cudaSuccess)
+    release_pins(h);
+  else
+    for (auto& b : h->pins) cudaFreeHost(b.p);  // copies of unknown state: not for others
   h->pool.release_all(h->stream);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   delete h;
@@ -450,6 +462,7 @@ int hodlr_trim_device_memory(void) {
   cudaMemPool_t mp = device_pool();
   if (!mp) return HODLR_ERR_CUDA;
   if (cudaDeviceSynchronize() != cudaSuccess) return HODLR_ERR_CUDA;
+  trim_pins();
   return cudaMemPoolTrimTo(mp, 0) == cudaSuccess ? HODLR_OK : HODLR_ERR_CUDA;
 }
 

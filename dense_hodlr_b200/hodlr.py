@@ -97,16 +97,20 @@ class HODLR_Matrix:
         lib = _L.lib()
         h = ctypes.c_void_p()
         if len(args) >= 1 and isinstance(args[0], np.ndarray) and args[0].ndim == 2:
-            A = np.asfortranarray(args[0], dtype=np.float64)
+            A = np.asarray(args[0], dtype=np.float64)
+            # a row-major matrix goes up as it is and is transposed on the device
+            by_rows = A.flags.c_contiguous and not A.flags.f_contiguous
+            if not by_rows:
+                A = np.asfortranarray(A)
             if A.shape[0] != A.shape[1]:
                 raise HODLRError(_L.ERR_ARG, "matrix must be square")
             leaf = int(args[1]) if len(args) > 1 else (leaf or 30)
             if len(args) > 2:
                 LR_Method = args[2]
             self.n = A.shape[0]
-            rc = lib.hodlr_create_dense(ctypes.byref(h), self.n,
-                                        A.ctypes.data_as(ctypes.POINTER(ctypes.c_double)),
-                                        self.n, int(leaf))
+            create = lib.hodlr_create_dense_rows if by_rows else lib.hodlr_create_dense
+            rc = create(ctypes.byref(h), self.n,
+                        A.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), self.n, int(leaf))
             _check(None, rc)
         else:
             if len(args) >= 1 and isinstance(args[0], kernelMatrix):

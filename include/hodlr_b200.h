@@ -62,6 +62,9 @@ int hodlr_create_kernel(hodlr_t* out, int n, int dim, const double* pts,
  *              std::string LR_Method = "partialPiv_ACA")           (:76)
  * A is n x n column-major host memory with leading dimension lda, copied. */
 int hodlr_create_dense(hodlr_t* out, int n, const double* A, int lda, int leaf_size);
+/* The same from n x n row-major host memory, lda values from row to row;
+ * transposed on the device. */
+int hodlr_create_dense_rows(hodlr_t* out, int n, const double* A, int lda, int leaf_size);
 
 /* HODLR_Matrix(int, int, double (*)(int,int,void*), void*, int)     (:162)
  * in its device-functor form: a dense handle whose n x n column-major FP64
@@ -191,8 +194,8 @@ int hodlr_set_capacity_hint(hodlr_t h, const int* caps, int nlevels);
 
 /* Device memory of all handles on the current device comes from one
  * stream-ordered pool owned by the library; memory that hodlr_destroy frees
- * stays reserved there for the next handle.  This returns it to the driver
- * (after a device synchronise).  No reference counterpart: the reference
+ * stays reserved there for the next handle, and so do up to 64 MB of pinned
+ * host staging memory.  This returns both (after a device synchronise).  No reference counterpart: the reference
  * allocates host memory per object. */
 int hodlr_trim_device_memory(void);
 
