@@ -84,12 +84,12 @@ def profiled_figure(name, key):
 # FP64 FLOPs of the symmetric full-kernel product (kmatvec.cu / kfast.cuh),
 # FMA counted as 2, as the kernel executes them: one Matern-3/2 entry in 2D is
 # the distance (2 sub + 2 fma from the floor), the square root from the
-# hardware seed (2 mul + 3 fma), Tang's exp (1 clamp, 1 fma + 1 sub for the
-# index, 2 fma for the reduction, 3 fma + 1 mul for the polynomial, 1 fma for
-# the table scale) and (1+s)e^-s (1 fma): 13 FMAs + 7 other = 33 FLOPs,
+# hardware seed (2 mul + 3 fma), Tang's exp (1 add + 2 sub for the index and the
+# remainder, 2 fma for the polynomial, 1 mul + 1 fma for the table scale) and
+# 1+s with its product (1 fma + 1 mul): 9 FMAs + 9 other = 27 FLOPs,
 # evaluated once per entry pair, plus 2 * nrhs FMAs (row and column products,
 # inside mma.m8n8k4.f64 for 8 right-hand sides) per evaluated entry.
-KMV_EVAL_FLOPS = 33
+KMV_EVAL_FLOPS = 27
 
 
 def sym_slices(n):

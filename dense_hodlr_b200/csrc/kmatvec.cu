@@ -5,7 +5,9 @@
 //
 // Bound by the FP64 units: the distance, square root and Tang exp from
 // kfast.cuh (specialised per kernel family at compile time, no dispatch) and
-// two products per right-hand side and evaluated entry.  Four forms:
+// two products per right-hand side and evaluated entry; and by everything else
+// that a scheduler issues, since an FP64 instruction holds it for two cycles.
+// Four forms:
 //   kmatvec_kernel          row by row (dense input, the no-alloc entry, up to
 //                           16 right-hand sides); column ranges split over
 //                           gridDim.y, partial sums added in a fixed order;
@@ -23,18 +25,25 @@ namespace {
 constexpr int KT = 128;
 constexpr int RPT = 2;  // rows per thread
 
-__constant__ double c_tang[HX_TANG_TABLE_SIZE] = HX_TANG_TABLE_INIT;
+// Tables of the exponential.  The 2048-entry table saves a polynomial term; the
+// kernels that load few other things hide its bank conflicts (N = 50001, 3D, one
+// vector: 2048 entries 1.60 ms, 256 entries in 8 copies 1.75, in 16 copies 1.79).
+// The row-by-row and forest forms have short column loops: the small table there.
+using ExpG = ExpTab<8, 8>;
+using ExpS = ExpTab<11, 1>;
 
 template <int NR, int KTYPE, int DIM>
 __global__ void __launch_bounds__(KT) kmatvec_kernel(KmatvecLaunch L) {
   __shared__ double xs[DIM > 0 ? DIM : 1][KT];
   __shared__ double vs[NR][KT];
-  __shared__ double tab[HX_TANG_TABLE_SIZE];
+  __shared__ double tab[ExpG::DOUBLES];
   const int n = L.n;
   const int nsplit = gridDim.y;
   const int per = ((n + nsplit - 1) / nsplit + KT - 1) / KT * KT;
   const int jb = blockIdx.y * per, je = min(n, jb + per);
-  for (int i = threadIdx.x; i < HX_TANG_TABLE_SIZE; i += blockDim.x) tab[i] = c_tang[i];
+  if (DIM > 0) ExpG::fill(tab);
+  const ExpG ex(tab);
+  const double cs = hx_point_scale<KTYPE>(L.src.kp.a, ExpG::UNIT);
   int row[RPT];
   bool live[RPT];
   double xi[RPT][DIM > 0 ? DIM : 1];
@@ -44,18 +53,17 @@ __global__ void __launch_bounds__(KT) kmatvec_kernel(KmatvecLaunch L) {
     row[q] = blockIdx.x * (KT * RPT) + q * KT + threadIdx.x;
     live[q] = row[q] < n;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) xi[q][d] = live[q] ? L.src.pts[d * L.src.ld + row[q]] : 0.0;
+    for (int d = 0; d < DIM; ++d) xi[q][d] = live[q] ? cs * L.src.pts[d * L.src.ld + row[q]] : 0.0;
 #pragma unroll
     for (int c = 0; c < NR; ++c) acc[q][c] = 0.0;
   }
-  const double a = L.src.kp.a;
   for (int j0 = jb; j0 < je; j0 += KT) {
     const int jn = min(KT, je - j0);
     __syncthreads();
     if (threadIdx.x < jn) {
       const int j = j0 + threadIdx.x;
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) xs[d][threadIdx.x] = L.src.pts[d * L.src.ld + j];
+      for (int d = 0; d < DIM; ++d) xs[d][threadIdx.x] = cs * L.src.pts[d * L.src.ld + j];
 #pragma unroll
       for (int c = 0; c < NR; ++c)
         vs[c][threadIdx.x] = c < L.nrhs ? L.X[(int64_t)c * L.ldx + j] : 0.0;
@@ -70,13 +78,13 @@ __global__ void __launch_bounds__(KT) kmatvec_kernel(KmatvecLaunch L) {
           kij = live[q] ? L.src.A[(int64_t)(j0 + t) * L.src.ld + row[q]] : 0.0;
         } else {
           // off-diagonal formula everywhere; the diagonal is corrected below
-          double r2 = 0.0;
+          double r2 = HX_R2_FLOOR;
 #pragma unroll
           for (int d = 0; d < DIM; ++d) {
             double dd = xi[q][d] - xs[d][t];
             r2 = fma(dd, dd, r2);
           }
-          kij = hx_kernel_r2_fast_t<KTYPE>(a, r2, tab);
+          kij = hx_kernel_unit<KTYPE>(r2, ex);
         }
 #pragma unroll
         for (int c = 0; c < NR; ++c) acc[q][c] = fma(kij, vs[c][t], acc[q][c]);
@@ -162,15 +170,19 @@ void launch_type(const KmatvecLaunch& L, dim3 grid, cudaStream_t s) {
 // per group) and accumulated into the workspace.
 constexpr int ST = 256;  // tile edge (rows = columns)
 constexpr int SG = 32;   // rotation group
-// 1 to 4 right-hand sides (more go to kmatvec_sym_mma_kernel): 2 rows per
-// thread, 128 threads
-template <int NR>
+// 1 to 4 right-hand sides (more go to kmatvec_sym_mma_kernel).  An FP64
+// instruction takes its scheduler two issue cycles and every other one takes one
+// (measured: N = 32768, 2 x FP64 + others = 39.4 of the 41.6 cycles per entry and
+// warp), so the loads, shuffles and index arithmetic of a column are shared by
+// as many rows as registers allow: up to 4 rows a thread for one vector
+// (N = 50001, 3D: 2 rows 1.68 ms, 4 rows 1.60), 2 for more.
+template <int NR, int ROWS>
 struct SymCfg {
   static_assert(NR == 1 || NR == 4, "the FMA form serves 1 to 4 right-hand sides");
-  static constexpr int RPT = 2;
+  static constexpr int RPT = ROWS;
   static constexpr int NT = ST / RPT;
   static constexpr int NW = NT / 32;
-  static constexpr int MINB = 3;
+  static constexpr int MINB = ROWS == 4 ? 6 : 3;
 };
 
 template <int NR>
@@ -178,15 +190,16 @@ struct SymPad {  // row stride of the staged X tile: an odd number of 16-byte un
   static constexpr int VS = NR == 1 ? 1 : NR + 2;
 };
 
-template <int NR, int KTYPE, int DIM>
-__global__ void __launch_bounds__(SymCfg<NR>::NT, SymCfg<NR>::MINB)
+template <int NR, int ROWS, int KTYPE, int DIM>
+__global__ void __launch_bounds__(SymCfg<NR, ROWS>::NT, SymCfg<NR, ROWS>::MINB)
     kmatvec_sym_kernel(KmatvecLaunch L, int S, int tps) {
-  constexpr int SYM_RPT = SymCfg<NR>::RPT, SYM_NT = SymCfg<NR>::NT, SYM_NW = SymCfg<NR>::NW;
+  using Cfg = SymCfg<NR, ROWS>;
+  constexpr int SYM_RPT = Cfg::RPT, SYM_NT = Cfg::NT, SYM_NW = Cfg::NW;
   constexpr int VS = SymPad<NR>::VS;
   __shared__ double xs[DIM][ST];
   __shared__ __align__(16) double vs[ST][VS];
   __shared__ __align__(16) double colw[2][SYM_NW][SG][VS];
-  __shared__ double tab[HX_TANG_TABLE_SIZE];
+  __shared__ double tab[ExpS::DOUBLES];
   const int n = L.n;
   const int nT = (n + ST - 1) / ST;
   int a, b;
@@ -207,8 +220,9 @@ __global__ void __launch_bounds__(SymCfg<NR>::NT, SymCfg<NR>::MINB)
   const int ia0 = a * tps, ia1 = min(nT, ia0 + tps);
   const int jb1 = min(nT, b * tps + tps);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < HX_TANG_TABLE_SIZE; i += blockDim.x) tab[i] = c_tang[i];
-  const double cs = hx_point_scale<KTYPE>(L.src.kp.a);  // coordinates scaled once
+  ExpS::fill(tab);
+  const ExpS ex(tab);
+  const double cs = hx_point_scale<KTYPE>(L.src.kp.a, ExpS::UNIT);  // coordinates scaled once
   const int64_t slice = (int64_t)L.nrhs * n;
   double* __restrict__ wsA = L.ws + (int64_t)a * slice;  // column sums (rows of split b)
   double* __restrict__ wsB = L.ws + (int64_t)b * slice;  // row sums (rows of split a)
@@ -257,7 +271,7 @@ __global__ void __launch_bounds__(SymCfg<NR>::NT, SymCfg<NR>::MINB)
               const double dd = xi[q][d] - xs[d][t];
               r2 = fma(dd, dd, r2);
             }
-            const double k = hx_kernel_unit_t<KTYPE>(r2, tab);
+            const double k = hx_kernel_unit<KTYPE>(r2, ex);
 #pragma unroll
             for (int c = 0; c < NR; ++c) acc[q][c] = fma(k, vs[t][c], acc[q][c]);
           }
@@ -293,7 +307,7 @@ __global__ void __launch_bounds__(SymCfg<NR>::NT, SymCfg<NR>::MINB)
               const double dd = xi[q][d] - xj[d];
               r2 = fma(dd, dd, r2);
             }
-            const double k = hx_kernel_unit_t<KTYPE>(r2, tab);
+            const double k = hx_kernel_unit<KTYPE>(r2, ex);
 #pragma unroll
             for (int c = 0; c < NR; ++c) {
               acc[q][c] = fma(k, vj[c], acc[q][c]);
@@ -355,11 +369,10 @@ __global__ void __launch_bounds__(SymCfg<NR>::NT, SymCfg<NR>::MINB)
 //               K[t][g], K[t+4][g], the transpose, which goes through a
 //               per-warp shared-memory buffer (two 8-byte stores, one 16-byte
 //               load per lane).
-// The chunks are software-pipelined: the column MMAs of chunk c - 1 (its
-// transpose written and warp-synchronised in the previous step) are issued
-// beside the entries of chunk c, so their dependent chain hides under the
-// entry arithmetic; two transpose buffers suffice because a step reads the
-// previous buffer before its own warp barrier.  Each warp's column sums of a
+// The column sums of a chunk follow its entries and not the next chunk's: holding
+// them back a chunk cost 16 registers and, with that, constants moved into
+// registers anew for every entry (N = 131072: 21.2 -> 20.4 ms).  Two transpose
+// buffers, so that one warp barrier a chunk is enough.  Column sums of a
 // chunk are stored per warp; after every 32 columns the CTA adds the eight
 // warps' sums in warp order into the workspace slice, so every (slice, row)
 // still has one writer in a fixed order.  The FP64 work per entry is the
@@ -385,8 +398,8 @@ struct MmaSmem {
   static constexpr int VS = XS + DIM * ST;            // [8][MMA_VSP] X_J by rhs
   static constexpr int TR = VS + 8 * MMA_VSP;         // [8 warps][2][4 row chunks][64]
   static constexpr int CW = TR + 8 * 2 * 4 * 64;      // [2][8 warps][8 rhs][34]
-  static constexpr int TAB = CW + 2 * 8 * 8 * 34;     // [HX_TANG_TABLE_SIZE]
-  static constexpr size_t BYTES = (size_t)(TAB + HX_TANG_TABLE_SIZE) * sizeof(double);
+  static constexpr int TAB = CW + 2 * 8 * 8 * 34;     // [ExpS::DOUBLES]
+  static constexpr size_t BYTES = (size_t)(TAB + ExpS::DOUBLES) * sizeof(double);
 };
 
 template <int KTYPE, int DIM>
@@ -420,8 +433,9 @@ __global__ void __launch_bounds__(MMA_NT, 2)
   const int jb1 = min(nT, b * tps + tps);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  for (int i = threadIdx.x; i < HX_TANG_TABLE_SIZE; i += blockDim.x) tab[i] = c_tang[i];
-  const double cs = hx_point_scale<KTYPE>(L.src.kp.a);
+  ExpS::fill(tab);
+  const ExpS ex(tab);
+  const double cs = hx_point_scale<KTYPE>(L.src.kp.a, ExpS::UNIT);
   const int64_t slice = (int64_t)L.nrhs * n;
   double* __restrict__ wsA = L.ws + (int64_t)a * slice;
   double* __restrict__ wsB = L.ws + (int64_t)b * slice;
@@ -477,8 +491,8 @@ __global__ void __launch_bounds__(MMA_NT, 2)
             s0 = fma(d0, d0, s0);
             s1 = fma(d1, d1, s1);
           }
-          e0[rc] = hx_kernel_unit_t<KTYPE>(s0, tab);
-          e1[rc] = hx_kernel_unit_t<KTYPE>(s1, tab);
+          e0[rc] = hx_kernel_unit<KTYPE>(s0, ex);
+          e1[rc] = hx_kernel_unit<KTYPE>(s1, ex);
           dmma_884(accR[rc], e0[rc], xb.x);
           dmma_884(accR[rc], e1[rc], xb.y);
         }
@@ -507,6 +521,14 @@ __global__ void __launch_bounds__(MMA_NT, 2)
         colw[(cc >> 2) & 1][w][2 * t][8 * (cc & 3) + g] = accC[0];
         colw[(cc >> 2) & 1][w][2 * t + 1][8 * (cc & 3) + g] = accC[1];
       };
+      // the workspace value that a group's sum is added to, read a group ahead
+      // (this thread wrote it)
+      double before = 0.0;
+      auto read_group = [&](int grp) {
+        const int col = threadIdx.x & 31, c = threadIdx.x >> 5;
+        const int j = J * ST + grp * 32 + col;
+        if (I != ia0 && c < L.nrhs && j < n) before = wsA[(int64_t)c * n + j];
+      };
       auto reduce_group = [&](int grp) {
         const int col = threadIdx.x & 31, c = threadIdx.x >> 5;
         const int j = J * ST + grp * 32 + col;
@@ -514,8 +536,7 @@ __global__ void __launch_bounds__(MMA_NT, 2)
           double sum = colw[grp & 1][0][c][col];
 #pragma unroll
           for (int ww = 1; ww < 8; ++ww) sum += colw[grp & 1][ww][c][col];
-          double* dst = wsA + (int64_t)c * n + j;
-          *dst = I == ia0 ? sum : *dst + sum;
+          wsA[(int64_t)c * n + j] = I == ia0 ? sum : before + sum;
         }
       };
       if (J == I) {  // diagonal tile pair: all entries, row sums only
@@ -526,32 +547,23 @@ __global__ void __launch_bounds__(MMA_NT, 2)
         }
         continue;
       }
-      // software pipeline: the column sums of chunk cc - 1 (entries already
-      // transposed) run beside the entries of chunk cc
-      {
-        double e0[4], e1[4];
-        chunk(0, e0, e1);
-        put_tr(0, e0, e1);
-        __syncwarp();
-      }
+      read_group(0);
 #pragma unroll 1
-      for (int cc = 1; cc < ST / 8; ++cc) {
-        double2 v[4];
-        get_tr((cc - 1) & 1, v);
-        double e0[4], e1[4];
-        chunk(cc, e0, e1);
-        col_sums(cc - 1, v);
-        put_tr(cc & 1, e0, e1);
-        __syncwarp();
-        if ((cc & 3) == 0) {
-          __syncthreads();
-          reduce_group((cc >> 2) - 1);
+      for (int cc = 0; cc < ST / 8; ++cc) {
+        {
+          double e0[4], e1[4];
+          chunk(cc, e0, e1);
+          put_tr(cc & 1, e0, e1);
         }
-      }
-      {
+        __syncwarp();
         double2 v[4];
-        get_tr(1, v);
-        col_sums(ST / 8 - 1, v);
+        get_tr(cc & 1, v);
+        col_sums(cc, v);
+        if ((cc & 3) == 3 && cc != ST / 8 - 1) {
+          __syncthreads();
+          reduce_group(cc >> 2);
+          read_group((cc >> 2) + 1);
+        }
       }
       __syncthreads();
       reduce_group(ST / 32 - 1);
@@ -606,15 +618,27 @@ void launch_sym_mma_type(const KmatvecLaunch& L, int S, int tps, cudaStream_t s)
   }
 }
 
+template <int NR, int ROWS, int KTYPE>
+void launch_sym_rows(const KmatvecLaunch& L, int S, int tps, cudaStream_t s) {
+  const int grid = S * (S + 1) / 2;
+  constexpr int NT = SymCfg<NR, ROWS>::NT;
+  if (L.src.kp.dim == 1)
+    kmatvec_sym_kernel<NR, ROWS, KTYPE, 1><<<grid, NT, 0, s>>>(L, S, tps);
+  else if (L.src.kp.dim == 2)
+    kmatvec_sym_kernel<NR, ROWS, KTYPE, 2><<<grid, NT, 0, s>>>(L, S, tps);
+  else
+    kmatvec_sym_kernel<NR, ROWS, KTYPE, 3><<<grid, NT, 0, s>>>(L, S, tps);
+}
+
+// 4 rows a thread where the CTAs (64 threads then) fill the chip about six deep,
+// 2 below.  One vector, Matern-3/2 2D, 2 rows | 4 rows, us: N = 3000 (78 CTAs)
+// 52 | 62, 9000 (666) 115 | 126, 12000 (1128) 160 | 152, 24000 (4465) 506 | 484.
 template <int NR, int KTYPE>
 void launch_sym_dim(const KmatvecLaunch& L, int S, int tps, cudaStream_t s) {
-  const int grid = S * (S + 1) / 2;
-  if (L.src.kp.dim == 1)
-    kmatvec_sym_kernel<NR, KTYPE, 1><<<grid, SymCfg<NR>::NT, 0, s>>>(L, S, tps);
-  else if (L.src.kp.dim == 2)
-    kmatvec_sym_kernel<NR, KTYPE, 2><<<grid, SymCfg<NR>::NT, 0, s>>>(L, S, tps);
-  else
-    kmatvec_sym_kernel<NR, KTYPE, 3><<<grid, SymCfg<NR>::NT, 0, s>>>(L, S, tps);
+  if constexpr (NR == 1) {
+    if (S * (S + 1) / 2 >= 900) return launch_sym_rows<1, 4, KTYPE>(L, S, tps, s);
+  }
+  launch_sym_rows<NR, 2, KTYPE>(L, S, tps, s);
 }
 
 template <int NR>
@@ -645,11 +669,13 @@ __global__ void __launch_bounds__(KT) kmatvec_forest_kernel(KmatvecLaunch L,
                                                             const int4* __restrict__ items) {
   __shared__ double xs[DIM][KT];
   __shared__ double vs[NR][KT];
-  __shared__ double tab[HX_TANG_TABLE_SIZE];
+  __shared__ double tab[ExpG::DOUBLES];
   const int4 it = items[blockIdx.x];
   if (L.skip && L.skip[it.w]) return;  // a converged system of a refinement
   const hx_kparams kp = L.src.kps[it.w];
-  for (int i = threadIdx.x; i < HX_TANG_TABLE_SIZE; i += blockDim.x) tab[i] = c_tang[i];
+  ExpG::fill(tab);
+  const ExpG ex(tab);
+  const double cs = hx_point_scale<KTYPE>(kp.a, ExpG::UNIT);
   int row[RPT];
   bool live[RPT];
   double xi[RPT][DIM];
@@ -659,7 +685,7 @@ __global__ void __launch_bounds__(KT) kmatvec_forest_kernel(KmatvecLaunch L,
     row[q] = it.x + q * KT + threadIdx.x;
     live[q] = row[q] < it.z;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) xi[q][d] = live[q] ? L.src.pts[d * L.src.ld + row[q]] : 0.0;
+    for (int d = 0; d < DIM; ++d) xi[q][d] = live[q] ? cs * L.src.pts[d * L.src.ld + row[q]] : 0.0;
 #pragma unroll
     for (int c = 0; c < NR; ++c) acc[q][c] = 0.0;
   }
@@ -669,7 +695,7 @@ __global__ void __launch_bounds__(KT) kmatvec_forest_kernel(KmatvecLaunch L,
     if (threadIdx.x < jn) {
       const int j = j0 + threadIdx.x;
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) xs[d][threadIdx.x] = L.src.pts[d * L.src.ld + j];
+      for (int d = 0; d < DIM; ++d) xs[d][threadIdx.x] = cs * L.src.pts[d * L.src.ld + j];
 #pragma unroll
       for (int c = 0; c < NR; ++c)
         vs[c][threadIdx.x] = c < L.nrhs ? L.X[(int64_t)c * L.ldx + j] : 0.0;
@@ -679,13 +705,13 @@ __global__ void __launch_bounds__(KT) kmatvec_forest_kernel(KmatvecLaunch L,
     for (int t = 0; t < jn; ++t) {
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
-        double r2 = 0.0;
+        double r2 = HX_R2_FLOOR;
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
           const double dd = xi[q][d] - xs[d][t];
           r2 = fma(dd, dd, r2);
         }
-        const double kij = hx_kernel_r2_fast_t<KTYPE>(kp.a, r2, tab);
+        const double kij = hx_kernel_unit<KTYPE>(r2, ex);
 #pragma unroll
         for (int c = 0; c < NR; ++c) acc[q][c] = fma(kij, vs[c][t], acc[q][c]);
       }

@@ -40,7 +40,7 @@
 #include <vector>
 
 #include "../dense_hodlr_b200/csrc/kfun.h"
-#include "../dense_hodlr_b200/csrc/kfast.cuh"
+#include "exp_tang.h"
 
 namespace {
 
