@@ -14,11 +14,15 @@
 //  schur_solve_kernel y = S^-1 Z by the stored LU (src/HODLR_Matrix.cpp:682).
 // The right-hand sides of a solve go through skinny.cu.
 // Pivoting takes the first maximum |a| of the column, as PartialPivLU does.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <vector>
 
 #include "common.cuh"
 #include "lu.h"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -239,18 +243,16 @@ __global__ void schur_form_kernel(SchurLaunch L) {
 
 // ------------------------------------------------------ dense batched LU
 // Blocked right-looking LU with row partial pivoting, S in global memory (L2
-// resident).  Panels of PNB columns are factored in shared memory; the
-// trailing matrix is updated with 4x4 register tiles.  The row interchanges
-// of a panel are applied to the whole row, so the packed result and `piv`
-// are those of an unblocked partial-pivot LU with the same pivot choices
-// (LAPACK getrf convention).
+// resident).  The row interchanges of a panel are applied to the whole row, so the
+// packed result and `piv` are those of an unblocked partial-pivot LU with the same
+// pivot choices (LAPACK getrf convention).
 constexpr int SNT = 512;
 
 // One CTA factors columns [jlo, jhi) of the n x n matrix a (columns < jlo
-// final, their interchanges already applied to columns >= jlo): the pivots of
-// those columns go to piv, their interchanges are applied to the columns of
-// [jlo, jhi) only, and the columns >= jhi are not touched.  jlo = 0,
-// jhi = n is the whole LU.
+// final, their interchanges already applied to columns >= jlo) in inner panels of
+// pnb columns in shared memory: the pivots of those columns go to piv, their
+// interchanges are applied to the columns of [jlo, jhi) only, and the columns
+// >= jhi are not touched.  For panels of too many rows to be held in registers.
 __device__ bool lu_columns(double* a, int n, int* piv, int jlo, int jhi, int pnb, double* pan,
                            double* red_v, int* red_i, int* lpiv) {
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -376,18 +378,289 @@ __device__ bool lu_columns(double* a, int n, int* piv, int jlo, int jhi, int pnb
   return singular;
 }
 
+// ------------------------------------------------- panels in registers
+// Columns [j0, j0 + nb), nb <= PW, of an n x n matrix, rows j0..: a row in each
+// thread's registers, one CTA or a cluster (CL) of up to 8 for more than SNT rows.
+// A column costs one barrier (and one of the cluster): every warp finds its first
+// maximum with warp reductions on the bits of |a|, its owner puts the value, its
+// position and the whole row into shared memory, and after the barrier all threads
+// pick the best of the warps' candidates and read that row.  Rows do not move:
+// each thread tracks the position its row would have after the interchanges and
+// writes it back there.  The same pivots, interchanges and eliminations as with
+// moved rows.
+//
+// Bound by that chain of PW reductions.  The panel in shared memory (three barriers
+// more, divisions and the rank-1 update through shared memory) took about 3 us a
+// column, in registers about 0.4 us:
+// factorization of N = 20011 2D 18.5 -> 13.1 ms, of 16384 points on a sphere
+// 62.8 -> 45.2 ms, of a forest of 40 systems 26.3 -> 21.9 ms.
+constexpr int PW = 32;
+struct PanelSmem {
+  unsigned hi[2][SNT / 32], lo[2][SNT / 32];
+  int pos[2][SNT / 32];
+  double inv[2][SNT / 32];
+  double row[2][SNT / 32][PW];
+  unsigned chi[2][8], clo[2][8];  // the cluster's candidates
+  int cpos[2][8];
+  double cinv[2][8];
+  double crow[2][8][PW];
+};
+
+// Index of the best candidate (largest |a| bits, then smallest position) among
+// `count` slots, in every lane.
+__device__ __forceinline__ int best_slot(const unsigned* hi, const unsigned* lo, const int* pos,
+                                         int count, int* q) {
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned h = lane < count ? hi[lane] : 0u, l = lane < count ? lo[lane] : 0u;
+  const int p = lane < count ? pos[lane] : INT_MAX;
+  const unsigned mh = __reduce_max_sync(all, h);
+  const unsigned ml = __reduce_max_sync(all, h == mh ? l : 0u);
+  const bool c = lane < count && h == mh && l == ml;
+  *q = __reduce_min_sync(all, c ? p : INT_MAX);
+  return __ffs(__ballot_sync(all, c && p == *q)) - 1;
+}
+
+template <bool CL>
+__device__ bool panel_in_registers(double* a, int n, int* piv, int j0, int nb, PanelSmem& sm) {
+  const unsigned all = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  int rank = 0, size = 1;
+  if (CL) {
+    rank = (int)cg::this_cluster().block_rank();
+    size = (int)cg::this_cluster().num_blocks();
+  }
+  const int r = rank * SNT + tid;
+  const bool live = r < n - j0;
+  int pos = r;
+  bool done = !live, singular = false;
+  double x[PW];
+#pragma unroll
+  for (int c = 0; c < PW; ++c) x[c] = live && c < nb ? a[(int64_t)(j0 + c) * n + j0 + r] : 0.0;
+#pragma unroll
+  for (int c = 0; c < PW; ++c) {
+    if (c < nb) {  // uniform
+      const int buf = c & 1;  // read until the next column's barrier
+      // a NaN is never larger than another value; rows in play have the top bit
+      const double v = fabs(x[c]);
+      const unsigned hi = done ? 0u : (v == v ? (unsigned)__double2hiint(v) : 0u) | 0x80000000u;
+      const unsigned lo = !done && v == v ? (unsigned)__double2loint(v) : 0u;
+      const double inv = 1.0 / x[c];
+      const unsigned mh = __reduce_max_sync(all, hi);
+      const unsigned ml = __reduce_max_sync(all, hi == mh ? lo : 0u);
+      const bool cand = !done && hi == mh && lo == ml;
+      const int mp = __reduce_min_sync(all, cand ? pos : INT_MAX);
+      if (mh == 0u) {
+        if (lane == 0) {
+          sm.hi[buf][w] = sm.lo[buf][w] = 0u;
+          sm.pos[buf][w] = INT_MAX;
+        }
+      } else if (cand && pos == mp) {
+        sm.hi[buf][w] = mh;
+        sm.lo[buf][w] = ml;
+        sm.pos[buf][w] = pos;
+        sm.inv[buf][w] = inv;
+#pragma unroll
+        for (int k = c & ~1; k < PW; k += 2)
+          *reinterpret_cast<double2*>(&sm.row[buf][w][k]) = make_double2(x[k], x[k + 1]);
+      }
+      __syncthreads();
+      int q;
+      int b = best_slot(sm.hi[buf], sm.lo[buf], sm.pos[buf], SNT / 32, &q);
+      const double* pr = sm.row[buf][b];
+      double di = sm.inv[buf][b];
+      if (CL) {
+        if (w == 0)
+          for (int o = 0; o < size; ++o) {
+            PanelSmem* to = cg::this_cluster().map_shared_rank(&sm, o);
+            to->crow[buf][rank][lane] = pr[lane];
+            if (lane == 0) {
+              to->chi[buf][rank] = sm.hi[buf][b];
+              to->clo[buf][rank] = sm.lo[buf][b];
+              to->cpos[buf][rank] = q;
+              to->cinv[buf][rank] = di;
+            }
+          }
+        cg::this_cluster().sync();
+        b = best_slot(sm.chi[buf], sm.clo[buf], sm.cpos[buf], size, &q);
+        pr = sm.crow[buf][b];
+        di = sm.cinv[buf][b];
+      }
+      if (r == 0) piv[j0 + c] = j0 + q;
+      if (pos == q) {
+        pos = c;
+        done = true;
+      } else if (pos == c) {
+        pos = q;
+      }
+      const double d = pr[c];
+      if (d == 0.0) {
+        singular = true;
+      } else if (!done) {
+        double l;
+        if (fabs(d) > 0x1p-1000 && fabs(d) < 0x1p1000) {  // x / d from 1 / d, one correction
+          l = x[c] * di;
+          l = fma(fma(-l, d, x[c]), di, l);
+        } else {
+          l = x[c] / d;
+        }
+        x[c] = l;
+#pragma unroll
+        for (int k = c + 1; k < PW; ++k) x[k] = fma(-l, pr[k], x[k]);
+      }
+    }
+  }
+  if (live) {
+#pragma unroll
+    for (int c = 0; c < PW; ++c)
+      if (c < nb) a[(int64_t)(j0 + c) * n + j0 + pos] = x[c];
+  }
+  return singular;
+}
+
+// The interchanges piv[0..nb) (relative positions p <-> piv[p], p = 0, 1, ..) as
+// moves: position i < nb receives row from[i], and position to[i] >= nb (or
+// to[i] < nb: none) row i.  Run by one warp; false: not LU interchanges.
+__device__ bool panel_moves(const int* piv, int j0, int nb, int rows, int* from, int* to) {
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int q = lane < nb ? piv[j0 + lane] - j0 : lane;
+  const bool ok = __all_sync(all, q >= lane && (lane >= nb || q < rows));
+  int t = lane, f = lane;
+  for (int c = 0; c < nb; ++c) {
+    const int qc = __shfl_sync(all, q, c);
+    t = t == c ? qc : t == qc ? c : t;
+  }
+  for (int c = nb - 1; c >= 0; --c) {
+    const int qc = __shfl_sync(all, q, c);
+    f = f == c ? qc : f == qc ? c : f;
+  }
+  from[lane] = ok ? f : lane;
+  to[lane] = ok ? t : lane;
+  return ok;
+}
+
+// A column's part of a panel's interchanges: u[i] <- its rows at positions < nb,
+// the displaced rows written below.  The caller writes u back.
+__device__ __forceinline__ void gather_moved(double* ac, int nb, const int* from, const int* to,
+                                             double (&u)[PW]) {
+#pragma unroll
+  for (int i = 0; i < PW; ++i) u[i] = i < nb ? ac[from[i]] : 0.0;
+#pragma unroll 8
+  for (int i = 0; i < nb; ++i)
+    if (to[i] >= nb) ac[to[i]] = ac[i];
+}
+
+// u <- L11^-1 u, unit lower, rows in order
+__device__ __forceinline__ void unit_lower_solve(const double (*l11)[PW], double (&u)[PW]) {
+#pragma unroll
+  for (int p = 0; p < PW - 1; ++p)
+#pragma unroll
+    for (int i = p + 1; i < PW; ++i) u[i] = fma(-l11[p][i], u[p], u[i]);
+}
+
+// D = A B for a warp: A 32 x 32 at as[p * lda + row], B 32 x 16 at bs[p * ldb + col],
+// leading dimensions 4 mod 16 (no bank conflicts).  D[m][v] of lane (g, t): rows
+// 8 m + g, columns 8 v + 2 t, + 1.
+__device__ __forceinline__ void warp_tile(const double* as, int lda, const double* bs, int ldb,
+                                          double (&acc)[4][2][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) acc[m][v][0] = acc[m][v][1] = 0.0;
+#pragma unroll
+  for (int k = 0; k < PW; k += 4) {
+    double av[4], bv[2];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) av[m] = as[(k + t) * lda + 8 * m + g];
+#pragma unroll
+    for (int v = 0; v < 2; ++v) bv[v] = bs[(k + t) * ldb + 8 * v + g];
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int v = 0; v < 2; ++v)
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+            : "+d"(acc[m][v][0]), "+d"(acc[m][v][1])
+            : "d"(av[m]), "d"(bv[v]));
+  }
+}
+
+// rows or columns of a trailing block, padded for warp_tile
+__host__ __device__ constexpr int tile_pitch(int m) { return (m + 31) / 32 * 32 + 4; }
+
 // Whole LU of every node with sd < big_sd, one CTA per node (larger nodes are
-// left to the multi-CTA path below).
-__global__ void __launch_bounds__(SNT) schur_lu_kernel(SchurLaunch L, int pnb, int big_sd) {
-  extern __shared__ double pan[];  // rows x pnb panel, leading dimension rows
-  __shared__ double red_v[SNT / 32];
-  __shared__ int red_i[SNT / 32];
-  __shared__ int lpiv[64];
+// left to the multi-CTA path below): panels in registers, a column a thread for
+// the interchanges and U12 = L11^-1 A12, A22 -= L21 U12 on the matrix
+// instructions from shared memory.
+__global__ void __launch_bounds__(SNT) schur_lu_kernel(SchurLaunch L, int big_sd) {
+  extern __shared__ __align__(16) double dyn[];
+  __shared__ __align__(16) PanelSmem sm;
+  __shared__ __align__(16) double l11[PW][PW];
+  __shared__ int from[PW], to[PW];
   const SchurNode N = L.nodes[blockIdx.x];
   const int n = N.kb + N.kt;
   if (n >= big_sd) return;
-  const bool singular =
-      lu_columns(L.S + N.s_off, n, L.piv + N.p_off, 0, n, pnb, pan, red_v, red_i, lpiv);
+  double* a = L.S + N.s_off;
+  int* piv = L.piv + N.p_off;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+  bool singular = false;
+  for (int j0 = 0; j0 < n; j0 += PW) {
+    const int nb = min(PW, n - j0), rest = n - j0 - nb;
+    singular |= panel_in_registers<false>(a, n, piv, j0, nb, sm);
+    __syncthreads();  // the panel and its pivots, by this CTA
+    if (w == 0) panel_moves(piv, j0, nb, n - j0, from, to);
+    const int ld = tile_pitch(rest);
+    double* ls = dyn;            // [PW][ld] L21
+    double* us = dyn + PW * ld;  // [PW][ld] U12
+    for (int e = tid; e < PW * PW; e += SNT) {
+      const int i = e % PW, p = e / PW;
+      l11[p][i] = i < nb && p < nb ? a[(int64_t)(j0 + p) * n + j0 + i] : 0.0;
+    }
+    if (rest > 0)
+      for (int e = tid; e < PW * (ld - 4); e += SNT) {
+        const int i = e % (ld - 4), p = e / (ld - 4);
+        ls[p * ld + i] = i < rest && p < nb ? a[(int64_t)(j0 + p) * n + j0 + nb + i] : 0.0;
+      }
+    __syncthreads();
+    for (int col = tid; col < n + (ld - 4 - rest); col += SNT) {
+      if (col >= j0 && col < j0 + nb) continue;
+      const int right = col - j0 - nb;  // column of U12; from n on: padding
+      double u[PW];
+      if (col < n) {
+        double* ac = a + (int64_t)col * n + j0;
+        gather_moved(ac, nb, from, to, u);
+        if (right >= 0) unit_lower_solve(l11, u);
+#pragma unroll
+        for (int i = 0; i < PW; ++i)
+          if (i < nb) ac[i] = u[i];
+      }
+      if (right >= 0 && rest > 0)
+#pragma unroll
+        for (int i = 0; i < PW; ++i) us[i * ld + right] = col < n ? u[i] : 0.0;
+    }
+    __syncthreads();
+    if (rest <= 0) break;
+    const int tr = (rest + 31) / 32, tc = (rest + 15) / 16;
+    for (int tt = w; tt < tr * tc; tt += SNT / 32) {
+      const int r0 = 32 * (tt % tr), c0 = 16 * (tt / tr);
+      double acc[4][2][2];
+      warp_tile(ls + r0, ld, us + c0, ld, acc);
+#pragma unroll
+      for (int v = 0; v < 2; ++v)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int c = c0 + 8 * v + 2 * t + e;
+          double* ac = a + (int64_t)(j0 + nb + c) * n + j0 + nb;
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            const int rr = r0 + 8 * m + g;
+            if (c < rest && rr < rest) ac[rr] -= acc[m][v][e];
+          }
+        }
+    }
+    __syncthreads();
+  }
   if (threadIdx.x == 0 && singular) atomicOr(L.err, DEV_ERR_SINGULAR);
 }
 
@@ -398,13 +671,25 @@ __global__ void __launch_bounds__(SNT) schur_lu_kernel(SchurLaunch L, int pnb, i
 // to every other column and form U12 = L11^-1 A12 right of the panel; (3)
 // A22 -= L21 U12 in 64 x 64 tiles over all SMs.  The pivot choices are the
 // column-wise first maxima, as in the one-CTA kernel.
-constexpr int BNB = 32;
+constexpr int BNB = PW;
 constexpr int BIG_MAX = 1024;  // nodes per launch (kernel parameter: 4 KB)
 struct BigNodes {
   int idx[BIG_MAX];
   int count;
 };
 
+template <bool CL>
+__global__ void __launch_bounds__(SNT) panel_kernel(SchurLaunch L, BigNodes B, int j0) {
+  __shared__ __align__(16) PanelSmem sm;
+  const SchurNode N = L.nodes[B.idx[blockIdx.y]];
+  const int n = N.kb + N.kt;
+  if (j0 >= n) return;  // the whole cluster
+  const bool singular = panel_in_registers<CL>(L.S + N.s_off, n, L.piv + N.p_off, j0,
+                                               min(BNB, n - j0), sm);
+  if (threadIdx.x == 0 && singular) atomicOr(L.err, DEV_ERR_SINGULAR);
+}
+
+// Panels of more rows than 8 CTAs' threads: through shared memory, one CTA.
 __global__ void __launch_bounds__(SNT) big_panel_kernel(SchurLaunch L, BigNodes B, int j0, int pnb) {
   extern __shared__ double pan[];
   __shared__ double red_v[SNT / 32];
@@ -418,49 +703,34 @@ __global__ void __launch_bounds__(SNT) big_panel_kernel(SchurLaunch L, BigNodes 
   if (threadIdx.x == 0 && singular) atomicOr(L.err, DEV_ERR_SINGULAR);
 }
 
-// One thread per column outside the panel: the panel's interchanges, then
-// (right of the panel) the unit-lower solve with L11.
-__global__ void __launch_bounds__(256) big_swap_trsm_kernel(SchurLaunch L, BigNodes B, int j0) {
-  __shared__ double l11[BNB][BNB + 1];
-  __shared__ int sp[BNB];
+// One thread per column outside the panel: the panel's interchanges as moves (32
+// independent loads instead of a chain of swaps), then (right of the panel) the
+// unit-lower solve with L11.
+__global__ void __launch_bounds__(128) big_swap_trsm_kernel(SchurLaunch L, BigNodes B, int j0) {
+  __shared__ __align__(16) double l11[PW][PW];
+  __shared__ int from[PW], to[PW];
   const SchurNode N = L.nodes[B.idx[blockIdx.y]];
   const int n = N.kb + N.kt;
   if (j0 >= n) return;
   const int nb = min(BNB, n - j0);
   double* a = L.S + N.s_off;
-  const int* piv = L.piv + N.p_off;
-  for (int e = threadIdx.x; e < BNB * BNB; e += blockDim.x) {
-    const int i = e % BNB, p = e / BNB;
-    l11[i][p] = (i < nb && p < nb) ? a[(int64_t)(j0 + p) * n + j0 + i] : 0.0;
+  if (threadIdx.x < 32 && !panel_moves(L.piv + N.p_off, j0, nb, n - j0, from, to) &&
+      threadIdx.x == 0)  // not LU interchanges: skipped and reported
+    atomicOr(L.err, DEV_ERR_INDEX | DEV_ERR_AT_LU_SWAP);
+  for (int e = threadIdx.x; e < PW * PW; e += blockDim.x) {
+    const int i = e % PW, p = e / PW;
+    l11[p][i] = (i < nb && p < nb) ? a[(int64_t)(j0 + p) * n + j0 + i] : 0.0;
   }
-  if (threadIdx.x < BNB) sp[threadIdx.x] = threadIdx.x < nb ? piv[j0 + threadIdx.x] : 0;
   __syncthreads();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= n || (col >= j0 && col < j0 + nb)) return;
-  double* ac = a + (int64_t)col * n;
-  for (int c = 0; c < nb; ++c) {
-    const int q = sp[c];
-    if (q < j0 + c || q >= n) {  // not an LU interchange: skip and report
-      atomicOr(L.err, DEV_ERR_INDEX | DEV_ERR_AT_LU_SWAP);
-      continue;
-    }
-    if (q != j0 + c) {
-      const double t = ac[j0 + c];
-      ac[j0 + c] = ac[q];
-      ac[q] = t;
-    }
-  }
-  if (col < j0) return;
-  double u[BNB];
+  double* ac = a + (int64_t)col * n + j0;
+  double u[PW];
+  gather_moved(ac, nb, from, to, u);
+  if (col > j0) unit_lower_solve(l11, u);
 #pragma unroll
-  for (int i = 0; i < BNB; ++i) u[i] = i < nb ? ac[j0 + i] : 0.0;
-#pragma unroll
-  for (int i = 1; i < BNB; ++i)
-#pragma unroll
-    for (int p = 0; p < i; ++p) u[i] = fma(-l11[i][p], u[p], u[i]);
-#pragma unroll
-  for (int i = 0; i < BNB; ++i)
-    if (i < nb) ac[j0 + i] = u[i];
+  for (int i = 0; i < PW; ++i)
+    if (i < nb) ac[i] = u[i];
 }
 
 // A22 -= L21 U12: CTA (ti, tj, node) owns a 64 x 64 tile, 256 threads with
@@ -731,10 +1001,10 @@ int schur_factor_launch(const SchurLaunch& L, int nnodes, const int* sd, cudaStr
     }
   }
   if (small_max > 0) {
-    const int pnb = panel_width(small_max);
-    size_t smem = (size_t)small_max * pnb * sizeof(double);
+    // L21 and U12 of the first panel
+    const size_t smem = sizeof(double) * 2 * PW * tile_pitch(std::max(0, small_max - PW));
     LCK(smem_opt_in((const void*)schur_lu_kernel, smem));
-    schur_lu_kernel<<<nnodes, SNT, smem, s>>>(L, pnb, SCHUR_BIG_SD);
+    schur_lu_kernel<<<nnodes, SNT, smem, s>>>(L, SCHUR_BIG_SD);
     LCK(cudaGetLastError());
   }
   for (size_t b0 = 0; b0 < big.size(); b0 += BIG_MAX) {
@@ -749,9 +1019,26 @@ int schur_factor_launch(const SchurLaunch& L, int nnodes, const int* sd, cudaStr
     const size_t smem = (size_t)mx * pnb * sizeof(double);
     LCK(smem_opt_in((const void*)big_panel_kernel, smem));
     for (int j0 = 0; j0 < mx; j0 += BNB) {
-      big_panel_kernel<<<B.count, SNT, smem, s>>>(L, B, j0, pnb);
+      const int ctas = (mx - j0 + SNT - 1) / SNT;  // of a cluster, SNT rows each
+      if (ctas == 1) {
+        panel_kernel<false><<<dim3(1, B.count), SNT, 0, s>>>(L, B, j0);
+      } else if (ctas <= 8) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ctas, B.count);
+        cfg.blockDim = dim3(SNT);
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = ctas;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        LCK(cudaLaunchKernelEx(&cfg, panel_kernel<true>, L, B, j0));
+      } else {
+        big_panel_kernel<<<B.count, SNT, smem, s>>>(L, B, j0, pnb);
+      }
       LCK(cudaGetLastError());
-      big_swap_trsm_kernel<<<dim3((mx + 255) / 256, B.count), 256, 0, s>>>(L, B, j0);
+      big_swap_trsm_kernel<<<dim3((mx + 127) / 128, B.count), 128, 0, s>>>(L, B, j0);
       LCK(cudaGetLastError());
       const int rest = mx - j0 - BNB;
       if (rest > 0) {

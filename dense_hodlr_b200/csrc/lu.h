@@ -58,8 +58,10 @@ int leaf_lu_launch(const LeafLULaunch& L, int nleaves, int smax, cudaStream_t s)
 int leaf_solve_launch(const LeafSolveLaunch& L, int nleaves, int smax, cudaStream_t s);
 // Capacitance matrices of at least this size are factored by the multi-CTA
 // blocked LU (panel, swap + triangular solve, tiled trailing update per 32
-// columns); smaller ones by one CTA each.
-constexpr int SCHUR_BIG_SD = 384;
+// columns); smaller ones by one CTA each.  Factorization with the line at 192,
+// 256, 384 and 416: N = 20011 2D 13.1, 13.1, 13.7, 13.7 ms, forest of 40 systems
+// 21.5, 21.9, 22.0, 22.0 ms; more nodes than SMs favour one CTA each.
+constexpr int SCHUR_BIG_SD = 256;
 // The factorization's solves of the ancestor columns go blocked from this
 // size (one 32-row diagonal block): the blocked solve reads each 32-row block
 // of the LU once per 64 columns and keeps every SM busy, where one CTA per 16
