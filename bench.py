@@ -371,9 +371,7 @@ def run_ours(args, rank, world, local_rank):
     aca_launch = float(np.mean(phase["aca_launches"]))
     hbm, peak_kind = peaks()
     achieved = aca_bytes / aca_s / 1e9
-    ratio = profiled_figure("aca_kernel_matern2d_n131072.md", "traffic_to_algorithmic")
     aca_per_launch = aca_bytes / max(aca_launch, 1.0)
-    traffic = ratio * aca_per_launch if ratio else None
     # full-kernel product: FP64 FLOPs per launch over its event-timed duration
     sm_mhz = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))).get("sm_max_mhz", 1965.0) \
         if os.path.exists(os.path.join(ROOT, "MEASURED_PEAKS.json")) else 1965.0
@@ -427,14 +425,13 @@ def run_ours(args, rank, world, local_rank):
                                       "(the workspace writes); the kernel is compute-bound"),
                      "algorithmic_flops_per_launch": kmv_flops,
                      "avg_launch_s": t_kmatvec},
-        "roofline_aca": {"kernel": "aca_kernel (batched partial-pivot ACA, one launch per level "
-                                   "group)",
+        "roofline_aca": {"kernel": "aca_group_kernel and aca_kernel (batched partial-pivot ACA; "
+                                   "sets of upper levels, pooled deep levels)",
                          "bound": "hbm", "achieved": achieved, "peak": hbm,
                          "peak_kind": f"{peak_kind} hbm_gbs (burst)", "unit": "GB/s",
                          "frac": achieved / hbm,
-                         "traffic": traffic,
-                         "traffic_note": ("DRAM/algorithmic ratio of the N=131072 capture "
-                                          "applied to this launch's algorithmic bytes"),
+                         "traffic": None,
+                         "traffic_note": "DRAM bytes of the current kernels not captured",
                          "algorithmic_bytes_per_launch": aca_per_launch,
                          "avg_launch_s": aca_s / max(aca_launch, 1.0),
                          "launches_per_step": aca_launch},
@@ -597,7 +594,7 @@ def run_profile_case(case):
     elif case.startswith("factor-profile"):
         # the FP64-at-scale workload (or its first N points' cloud at a smaller
         # N, 'factor-profile:N'): one compression, then one factorization (the
-        # launches after the aca_kernel ones) and one 8-RHS direct solve
+        # launches after the ACA ones) and one 8-RHS direct solve
         import torch
         from dense_hodlr_b200.points import uniform_cube
         parts = case.split(":")

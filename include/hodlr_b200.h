@@ -360,7 +360,8 @@ int hodlr_set_aca_streaming(hodlr_t h, int on);
 /* Bounded device waits (no counterpart in the reference).  The CTAs of one
  * ACA block group meet at a barrier in global memory; a barrier that is not
  * complete after `polls` polls (0: the default, 2^26) gives up, the launch
- * ends and the call returns HODLR_ERR_TIMEOUT, leaving the handle usable.
+ * ends and the call returns HODLR_ERR_TIMEOUT, leaving the handle usable (the
+ * streaming form's exchanges count 2^22 polls by default).
  * unreachable = 1 makes every such barrier wait for one arrival more than
  * its group has -- a wait nothing completes -- so that this path can be
  * tested; set it back to 0 for normal work. */
