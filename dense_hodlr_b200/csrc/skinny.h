@@ -41,12 +41,12 @@ struct CapNode {
 };
 
 struct CapLaunch {
-  const CapNode* nodes;
-  const double* S;
-  const int* perm;
-  const double* part;
-  double* z;
-  double* big;  // cap_big_elems doubles, or null when that is 0
+  const CapNode* nodes = nullptr;
+  const double* S = nullptr;
+  const int* perm = nullptr;
+  const double* part = nullptr;
+  double* z = nullptr;
+  double* big = nullptr;  // cap_big_elems doubles, or null when that is 0
 };
 
 // Column tiles of 8 a launch carries per CTA: 1 or 2.
