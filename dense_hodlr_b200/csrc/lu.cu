@@ -11,7 +11,7 @@
 //                     (src/HODLR_Matrix.cpp:663-673) from the level product Z.
 //  schur_lu_kernel    blocked partial-pivot LU of each node's S in place
 //                     (SchurLU = PartialPivLU(S), src/HODLR_Matrix.cpp:675).
-//  schur_solve_kernel y = S^-1 Z by the stored LU (src/HODLR_Matrix.cpp:682).
+//  big_rhs_* kernels  y = S^-1 Z by the stored LU (src/HODLR_Matrix.cpp:682).
 // The right-hand sides of a solve go through skinny.cu.
 // Pivoting takes the first maximum |a| of the column, as PartialPivLU does.
 #include <cooperative_groups.h>
@@ -121,14 +121,8 @@ struct SmemLU {
   int lda;
   __device__ double operator()(int i, int j) const { return a[j * lda + i]; }
 };
-struct GlobalLU {
-  const double* a;
-  int n;
-  __device__ double operator()(int i, int j) const { return __ldg(a + (int64_t)j * n + i); }
-};
 
-template <class LU>
-__device__ void lu_solve_tile(const LU& A, int n, double* x, int ldx, int ncol) {
+__device__ void lu_solve_tile(const SmemLU& A, int n, double* x, int ldx, int ncol) {
   const int tid = threadIdx.x, NT = blockDim.x;
   for (int b0 = 0; b0 < n; b0 += BS) {  // forward, unit lower
     const int be = min(n, b0 + BS);
@@ -781,14 +775,13 @@ __global__ void __launch_bounds__(256) big_update_kernel(SchurLaunch L, BigNodes
   }
 }
 
-// ---------------------------------- blocked solve of large nodes' ancestor columns
-// y = S^-1 Z for the N.coff ancestor columns of a node with sd >= SCHUR_BIG_SOLVE_SD
-// (the factorization's schur solve, src/HODLR_Matrix.cpp:682): the LU's row
-// interchanges, then the unit-lower and the upper solves by 32-row diagonal
-// blocks, each a register-resident triangular solve (one thread per column)
-// followed by a 64 x 64-tiled update of the remaining rows over all SMs.  The
-// one-CTA-per-column-tile kernel would read the whole LU again for every 16
-// columns; here each block of the LU is read once per 64 columns.
+// ---------------------------------- blocked solve of the nodes' ancestor columns
+// y = S^-1 Z for the N.coff ancestor columns of a node (the factorization's
+// schur solve, src/HODLR_Matrix.cpp:682): the LU's row interchanges, then the
+// unit-lower and the upper solves by 32-row diagonal blocks, each a
+// register-resident triangular solve (one thread per column) followed by a
+// 64 x 64-tiled update of the remaining rows over all SMs: each block of the LU is
+// read once per 64 columns.
 __global__ void __launch_bounds__(256) big_rhs_perm_kernel(SchurLaunch L, BigNodes B) {
   const SchurNode N = L.nodes[B.idx[blockIdx.y]];
   const int n = N.kb + N.kt;
@@ -895,52 +888,6 @@ __global__ void __launch_bounds__(256) big_rhs_update_kernel(SchurLaunch L, BigN
       const int r = r0 + tx + 16 * q;
       if (r < rhi) x[(int64_t)c * n + r] -= acc[q][y];
     }
-  }
-}
-
-// y = S^-1 Z for the ancestor columns (N.coff, at r_off, ld sd) of the nodes
-// with sd < skip_sd; one CTA per (node, tile of tc columns).
-constexpr int STC = 16;
-
-__global__ void __launch_bounds__(256) schur_solve_kernel(SchurLaunch L, int tc, int skip_sd) {
-  extern __shared__ double xs[];
-  const int node = blockIdx.y;
-  const SchurNode N = L.nodes[node];
-  const int n = N.kb + N.kt;
-  if (n >= skip_sd) return;  // left to the blocked solve
-  const int cols = N.coff;
-  const int c0 = blockIdx.x * tc;
-  if (c0 >= cols) return;
-  const int nc = min(tc, cols - c0);
-  const double* a = L.S + N.s_off;
-  const int* piv = L.piv + N.p_off;
-  double* R = L.R + N.r_off;
-  const int ldx = n | 1;
-  for (int e = threadIdx.x; e < n * nc; e += blockDim.x) {
-    int i = e % n, c = e / n;
-    xs[c * ldx + i] = R[(int64_t)(c0 + c) * n + i];
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-    double* xc = xs + c * ldx;
-    for (int p = 0; p < n; ++p) {
-      int q = piv[p];
-      if (q < p || q >= n) {  // not an LU interchange: skip and report
-        atomicOr(L.err, DEV_ERR_INDEX | DEV_ERR_AT_SOLVE_PIV);
-        continue;
-      }
-      if (q != p) {
-        double t = xc[p];
-        xc[p] = xc[q];
-        xc[q] = t;
-      }
-    }
-  }
-  __syncthreads();
-  lu_solve_tile(GlobalLU{a, n}, n, xs, ldx, nc);
-  for (int e = threadIdx.x; e < n * nc; e += blockDim.x) {
-    int i = e % n, c = e / n;
-    R[(int64_t)(c0 + c) * n + i] = xs[c * ldx + i];
   }
 }
 
@@ -1074,23 +1021,8 @@ int schur_solve_factor_launch(const SchurLaunch& L, int nnodes, const int* sd, i
   *launches = 0;
   if (nnodes == 0 || coff <= 0) return 0;
   std::vector<int> big;
-  int small_max = 0;
-  for (int i = 0; i < nnodes; ++i) {
-    if (sd[i] >= SCHUR_BIG_SOLVE_SD)
-      big.push_back(i);
-    else
-      small_max = std::max(small_max, sd[i]);
-  }
-  if (small_max > 0) {
-    const size_t col_bytes = sizeof(double) * (size_t)(small_max | 1);
-    const int tc = (int)std::max<size_t>(1, std::min<size_t>(STC, 200 * 1024 / col_bytes));
-    const size_t smem = col_bytes * tc;
-    LCK(smem_opt_in((const void*)schur_solve_kernel, smem));
-    schur_solve_kernel<<<dim3((coff + tc - 1) / tc, nnodes), 256, smem, s>>>(L, tc,
-                                                                             SCHUR_BIG_SOLVE_SD);
-    LCK(cudaGetLastError());
-    ++*launches;
-  }
+  for (int i = 0; i < nnodes; ++i)
+    if (sd[i] > 0) big.push_back(i);
   const int ctiles = (coff + BT - 1) / BT, cblocks = (coff + 255) / 256;
   for (size_t b0 = 0; b0 < big.size(); b0 += BIG_MAX) {
     BigNodes B;

@@ -62,19 +62,15 @@ int leaf_solve_launch(const LeafSolveLaunch& L, int nleaves, int smax, cudaStrea
 // 256, 384 and 416: N = 20011 2D 13.1, 13.1, 13.7, 13.7 ms, forest of 40 systems
 // 21.5, 21.9, 22.0, 22.0 ms; more nodes than SMs favour one CTA each.
 constexpr int SCHUR_BIG_SD = 256;
-// The factorization's solves of the ancestor columns go blocked from this
-// size (one 32-row diagonal block): the blocked solve reads each 32-row block
-// of the LU once per 64 columns and keeps every SM busy, where one CTA per 16
-// columns runs a latency-bound substitution per tile (measured on the 2D
-// Matern workload at N = 262144: factorization 0.146 s with the blocked solve
-// from 128 rows, 0.141 from 64, 0.128 from 32).
-constexpr int SCHUR_BIG_SOLVE_SD = 32;
 // sd: host array of the nodes' capacitance sizes (kb + kt), in node order.
 int schur_factor_launch(const SchurLaunch& L, int nnodes, const int* sd, cudaStream_t s);
 // Kernel launches schur_factor_launch makes for these sizes.
 int schur_factor_launches(const int* sd, int nnodes);
 // The factorization's solves y = S^-1 Z of the `coff` ancestor columns of every
-// node (R at r_off, ld sd); nodes with sd >= SCHUR_BIG_SOLVE_SD by the
-// blocked solve.  sd: host array of the nodes' sizes.  *launches: kernels launched.
+// node (R at r_off, ld sd), in 32-row diagonal blocks: the LU is read once per 64
+// columns and every SM is busy.  Nodes of less than 32 rows too: one register
+// substitution each way instead of 16-column tiles in shared memory (factorization
+// of 1D N = 1024 1.00 -> 0.89 ms, N = 4096 1.40 -> 1.35).  sd: host array of the nodes' sizes.  *launches:
+// kernels launched.
 int schur_solve_factor_launch(const SchurLaunch& L, int nnodes, const int* sd, int coff,
                               cudaStream_t s, int* launches);
