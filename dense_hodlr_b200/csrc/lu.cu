@@ -423,6 +423,9 @@ __device__ bool panel_in_registers(double* a, int n, int* piv, int j0, int nb, P
   if (CL) {
     rank = (int)cg::this_cluster().block_rank();
     size = (int)cg::this_cluster().num_blocks();
+    // a CTA's shared memory may be written once it has started: waited for
+    // before the first column's stores, behind the panel's loads
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   }
   const int r = rank * SNT + tid;
   const bool live = r < n - j0;
@@ -464,6 +467,7 @@ __device__ bool panel_in_registers(double* a, int n, int* piv, int j0, int nb, P
       const double* pr = sm.row[buf][b];
       double di = sm.inv[buf][b];
       if (CL) {
+        if (c == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (w == 0)
           for (int o = 0; o < size; ++o) {
             PanelSmem* to = cg::this_cluster().map_shared_rank(&sm, o);
