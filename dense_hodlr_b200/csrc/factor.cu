@@ -69,8 +69,7 @@ __global__ void y_init_kernel(double* Y, const double* W, int64_t ld, int kmax, 
 
 // log|det| pieces of the factorization: per leaf LU (column-major s x s,
 // final row permutation perm) and per capacitance LU (sd x sd, LAPACK-style
-// swaps piv): out = (sum_i log|u_ii|, #u_ii < 0, permutation parity).  The
-// stored diagonal is that of the inverted triangles, 1 / u_ii.
+// swaps piv): out = (sum_i log|u_ii|, #u_ii < 0, permutation parity).
 __global__ void leaf_logdet_kernel(const double* lu, const int64_t* lu_off, const int* leaf_min,
                                    const int* leaf_size, const int* perm, double* out) {
   if (threadIdx.x != 0) return;
@@ -81,7 +80,7 @@ __global__ void leaf_logdet_kernel(const double* lu, const int64_t* lu_off, cons
   int neg = 0;
   for (int i = 0; i < s; ++i) {
     const double d = g[(int64_t)i * s + i];
-    sum -= log(fabs(d));
+    sum += log(fabs(d));
     neg += d < 0.0;
   }
   unsigned char seen[160];
@@ -108,7 +107,7 @@ __global__ void schur_logdet_kernel(const SchurNode* nodes, const double* S, con
   int neg = 0, swaps = 0;
   for (int i = 0; i < n; ++i) {
     const double d = a[(int64_t)i * n + i];
-    sum -= log(fabs(d));
+    sum += log(fabs(d));
     neg += d < 0.0;
     swaps += p[i] != i;
   }
@@ -138,7 +137,7 @@ int do_factorize(hodlr_t h) {
   int64_t tot = 0;
   for (int p = 0; p < nl; ++p) {
     lu_off[p] = tot;
-    tot += (int64_t)h->leaf_size[p] * h->leaf_size[p];
+    tot += (int64_t)h->leaf_size[p] * h->leaf_size[p] + tri_elems(h->leaf_size[p]);
   }
   CK(dalloc(h, &h->d_lu, (size_t)tot));
   CK(dalloc(h, &h->d_lu_off, (size_t)nl));
@@ -352,7 +351,7 @@ int do_factorize(hodlr_t h) {
       const int sd = sn.kb + sn.kt;
       L.max_sd = std::max(L.max_sd, sd);
       sn.s_off = s_tot;
-      s_tot += (int64_t)sd * sd;
+      s_tot += (int64_t)sd * sd + tri_elems(sd);
       sn.z_off = z_tot;
       sn.r_off = z_tot;
       z_tot += (int64_t)sd * (L.coff + std::max(sn.kb, sn.kt));

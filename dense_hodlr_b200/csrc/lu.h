@@ -9,7 +9,7 @@
 struct LeafLULaunch {
   const int* leaf_min;
   const int* leaf_size;
-  const int64_t* lu_off;  // offset of each leaf's s x s LU in `lu`
+  const int64_t* lu_off;  // offset of each leaf's s x s LU (and tri_elems) in `lu`
   double* lu;
   int* perm;              // length N: row permutation of each leaf, local indices
   EntrySrc src;

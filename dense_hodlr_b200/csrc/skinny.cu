@@ -9,19 +9,21 @@
 // 32-step chain of shuffles per 32 rows in one CTA.
 //
 //  * Triangular solves multiply by inverted 64 x 64 diagonal triangles (formed
-//    once per factorization, in place), so a block step is two small products
-//    instead of a substitution: n / 64 steps each way.
+//    once per factorization, behind the LU), so a block step is two small products
+//    instead of a substitution: n / 64 steps each way.  A product with an inverse
+//    alone is not backward stable; blocks that need it are refined (tri_mode).
 //  * Large capacitance systems run on a cluster of up to 8 CTAs: block rows
 //    dealt out cyclically, a solved block written to every CTA's shared memory.
 //  * V^T X is split over rows into items; their sums are added by the
 //    capacitance solve that reads them, in a fixed order.
 //
 // Measured on B200, a repeated direct solve end to end, 64-wide tiles and
-// one-CTA substitutions -> these kernels: N = 262144 2D, 8 columns 7.59 -> 2.44
+// one-CTA substitutions -> these kernels: N = 262144 2D, 8 columns 7.59 -> 2.31
 // ms (its panels' 3.2 GB at the copy rate: 0.49 ms); N = 30001 2D, 1 column 1.81
-// -> 0.90; sphere 16384 5.4 -> 1.2 ms; 40000-point cube 10.4 -> 3.6 ms; 1D 4096
-// 0.35 -> 0.09 ms.  What is left is the chain of the top capacitance solves
-// (2 n / 64 cluster steps of about 2 us) and, at 262144, the panels' reads.
+// -> 0.68.  Unrefined, and with the sums of V^T X that a capacitance solve starts
+// with read one at a time, they took 2.48 and 0.88; unrefined, 1.99 and 0.59.
+// What is left of 0.68 is the capacitance solves' 0.43 (the top one, 704 rows: 0.03
+// for its sums, 22 block steps of 4 us), the panel kernels' 0.19 and 25 launches.
 #include "skinny.h"
 
 #include <cooperative_groups.h>
@@ -34,6 +36,7 @@ namespace cg = cooperative_groups;
 
 constexpr int NB = TRI_NB;
 constexpr int SK_NT = 256;  // 8 warps
+constexpr int TRI_BUFS = 5;  // block buffers of tri_solve; the triangle behind them
 
 __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -42,20 +45,65 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 }
 
 // ------------------------------------------- inverted diagonal triangles
-// One CTA per diagonal block: threads 0..63 invert the unit lower triangle (a
-// column each), threads 64..127 the upper one, both by substitution in
-// registers over a copy in shared memory.  `m` rows of the block exist; the
-// rest is the identity.
-__device__ void invert_block(double* a, int ld, int m, double (*t)[NB + 2]) {
-  const int tid = threadIdx.x;
+// How a block step uses an inverse D of a triangle T.  The residual of y = D x is at
+// most u |T| |D| |T| |y|, a substitution's u |T| |y|: in the norm of the weights
+// w = |T| z, z_j = 1 / max_i |T_ij| (rows and columns of a capacitance matrix differ
+// by up to 1e43, so the measure must not depend on their scales), an excess of
+// c = max_i (|T| |D| w)_i / w_i, and each y += D (x - T y) multiplies the excess by
+// c u.  So k of them while c (c u)^k is below 0.01, k <= 3, none up to c = 4, and a
+// substitution beyond (or where D overflows).  numpy, leaves of 64 and 128 points,
+// five kernels in 1D to 3D, shifts 1 to 1e-8, residuals over a substitution's: at
+// most 1.37, mean 1.04, as with a refinement everywhere; with none up to c = 8 2.1,
+// 64 3.7, 512 22; with none at all 1e1 (shift 1e-2) to 1e6 (1e-8).
+constexpr int TRI_SUBST = 4;
+__device__ __forceinline__ int tri_mode(double c) {
+  return c <= 4.0 ? 0 : c <= 1e7 ? 1 : c <= 1e10 ? 2 : c <= 3e11 ? 3 : TRI_SUBST;  // NaN: the last
+}
+
+// sum of at(p) over lo <= p < hi, eight loads in flight
+template <class F>
+__device__ __forceinline__ double sum_in_row(int lo, int hi, const F& at) {
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int p0 = lo & ~7; p0 < hi; p0 += 8) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = p0 + u >= lo && p0 + u < hi ? at(p0 + u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s[u & 3] += v[u];
+  }
+  return (s[0] + s[1]) + (s[2] + s[3]);
+}
+
+// One CTA per diagonal block T of `m` rows (the rest of 64 is the identity):
+// threads 0..63 invert the unit lower triangle (a column each), threads 64..127 the
+// upper one, both by substitution in registers over a copy in shared memory.
+__device__ void invert_block(const double* a, int ld, int m, double* inv, int2* mode,
+                             double (*t)[NB + 1]) {
+  __shared__ double z[2][NB], wt[2][NB];
+  __shared__ int worst[2];
+  const int tid = threadIdx.x, h = tid >= NB, j = tid & (NB - 1);
+  const int lo = h ? j : 0, hi = h ? NB : j;  // stored columns of row j
   for (int e = tid; e < NB * NB; e += blockDim.x) {
-    const int i = e % NB, j = e / NB;
-    t[i][j] = i < m && j < m ? a[(int64_t)j * ld + i] : i == j ? 1.0 : 0.0;
+    const int i = e % NB, q = e / NB;
+    t[i][q] = i < m && q < m ? a[(int64_t)q * ld + i] : i == q ? 1.0 : 0.0;
+  }
+  if (tid < 2) worst[tid] = 0;
+  __syncthreads();
+  bool range = true;  // no inverse of a pivot is subnormal, or overflows
+  double big = h ? 0.0 : 1.0;
+#pragma unroll 16
+  for (int i = 0; i < NB; ++i)
+    if (h ? i <= j : i > j) big = fmax(big, fabs(t[i][j]));
+  z[h][j] = 1.0 / big;
+  if (tid < NB) {
+    const double r = 1.0 / t[tid][tid];
+    t[tid][NB] = r;
+    range = fabs(r) > 0x1p-1000 && fabs(r) < 0x1p1000;
   }
   __syncthreads();
-  const int j = tid & (NB - 1);
-  if (tid < NB) t[tid][NB] = 1.0 / t[tid][tid];
-  __syncthreads();
+  const double w = (h ? 0.0 : z[0][j]) +
+                   sum_in_row(lo, hi, [&](int p) { return fabs(t[j][p]) * z[h][p]; });
+  wt[h][j] = w;
   double x[NB];
   if (tid < NB) {
 #pragma unroll
@@ -79,22 +127,45 @@ __device__ void invert_block(double* a, int ld, int m, double (*t)[NB + 2]) {
   for (int i = 0; i < NB; ++i)
     if (tid < NB ? i > j : i <= j) t[i][j] = x[i];
   __syncthreads();
+  const double v = (h ? 0.0 : wt[0][j]) +  // |D| w
+                   sum_in_row(lo, hi, [&](int p) { return fabs(t[j][p]) * wt[h][p]; });
+  z[h][j] = v;
+  __syncthreads();
+  const double c =  // |T| |D| w
+      j >= m ? w : (h ? 0.0 : v) + sum_in_row(lo, min(hi, m), [&](int p) {
+        return fabs(a[(int64_t)p * ld + j]) * z[h][p];
+      });
+  atomicMax(&worst[h], tri_mode(c / w));
+  if (!range) atomicMax(&worst[1], TRI_SUBST);
   for (int e = tid; e < NB * NB; e += blockDim.x) {
     const int i = e % NB, q = e / NB;
-    if (i < m && q < m) a[(int64_t)q * ld + i] = t[i][q];
+    if (i < m && q < m) inv[q * m + i] = t[i][q];
   }
+  __syncthreads();
+  if (tid == 0) *mode = make_int2(worst[0], worst[1]);
+}
+
+// Where block b of a packed n x n LU has its inverse, and the modes of its
+// lower and upper triangle (tri_elems doubles behind the LU).
+__device__ __forceinline__ const double* tri_inverse(const double* a, int n, int b) {
+  return a + (int64_t)n * n + (int64_t)b * NB * NB;
+}
+__device__ __forceinline__ const int2* tri_modes(const double* a, int n) {
+  return reinterpret_cast<const int2*>(a + (int64_t)n * n + tri_elems(n)) - (n + NB - 1) / NB;
 }
 
 __global__ void __launch_bounds__(2 * NB) invert_leaves_kernel(LeafSolveLaunch L) {
-  __shared__ double t[NB][NB + 2];
+  __shared__ double t[NB][NB + 1];
   const int s = L.leaf_size[blockIdx.x], b0 = blockIdx.y * NB;
   if (b0 >= s) return;
   double* a = const_cast<double*>(L.lu) + L.lu_off[blockIdx.x];
-  invert_block(a + (int64_t)b0 * s + b0, s, min(NB, s - b0), t);
+  invert_block(a + (int64_t)b0 * s + b0, s, min(NB, s - b0),
+               const_cast<double*>(tri_inverse(a, s, blockIdx.y)),
+               const_cast<int2*>(tri_modes(a, s)) + blockIdx.y, t);
 }
 
 __global__ void __launch_bounds__(2 * NB) invert_nodes_kernel(SchurLaunch L, int* perm) {
-  __shared__ double t[NB][NB + 2];
+  __shared__ double t[NB][NB + 1];
   const SchurNode N = L.nodes[blockIdx.x];
   const int n = N.kb + N.kt, b0 = (int)(blockIdx.y - 1) * NB;
   if (blockIdx.y == 0) {  // the interchanges, in order, as a permutation
@@ -127,7 +198,10 @@ __global__ void __launch_bounds__(2 * NB) invert_nodes_kernel(SchurLaunch L, int
     return;
   }
   if (b0 >= n) return;
-  invert_block(L.S + N.s_off + (int64_t)b0 * n + b0, n, min(NB, n - b0), t);
+  double* a = L.S + N.s_off;
+  invert_block(a + (int64_t)b0 * n + b0, n, min(NB, n - b0),
+               const_cast<double*>(tri_inverse(a, n, blockIdx.y - 1)),
+               const_cast<int2*>(tri_modes(a, n)) + blockIdx.y - 1, t);
 }
 
 // --------------------------------------------------- blocked triangular solve
@@ -157,12 +231,95 @@ __device__ __forceinline__ void block_product(const double (&av)[NB / 4],
   }
 }
 
-// x <- U^-1 L^-1 x with the packed LU `a` (n x n, inverted diagonal triangles)
+// A triangle itself, for blocks that are refined or substituted: element (i, j) at
+// ts[j * TRI_PITCH + i], no bank conflicts between the lanes of a fragment.
+constexpr int TRI_PITCH = NB + 4;
+
+// The 8 rows of a triangular block that a warp multiplies: a scheduler's two warps
+// (w and w + 4) together have 9 of the 16 8 x 8 tiles that are not zero.
+__device__ __forceinline__ int tri_rows(int w) { return 8 * (w < 4 ? w : 11 - w); }
+
+// A triangle's (dir 0: unit lower, 1: upper) element in that warp's fragment k:
+// stored(col, row), or what the format implies.
+template <class F>
+__device__ __forceinline__ void load_tri(int dir, int m, const F& stored, double (&v)[NB / 4]) {
+  const int lane = threadIdx.x & 31, row = tri_rows(threadIdx.x >> 5) + (lane >> 2), t = lane & 3;
+#pragma unroll
+  for (int k = 0; k < NB / 4; ++k) {
+    const int col = 4 * k + t;
+    const bool in = (dir == 0 ? col < row : col >= row) && row < m && col < m;
+    v[k] = in ? stored(col, row) : dir == 0 && col == row ? 1.0 : 0.0;
+  }
+}
+
+// block_product for a triangle's fragments, without its zero tiles.
+template <int NT>
+__device__ __forceinline__ void tri_product(int dir, const double (&av)[NB / 4],
+                                            const double* const (&x)[NT], double (&out)[NT][2]) {
+  const int lane = threadIdx.x & 31, r8 = tri_rows(threadIdx.x >> 5) / 8, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int u = 0; u < NT; ++u) {
+    double acc[4][2];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[c][0] = acc[c][1] = 0.0;
+#pragma unroll
+    for (int k = 0; k < NB / 4; ++k)
+      if (dir == 0 ? k / 2 <= r8 : k / 2 >= r8)  // the same for the warp
+        dmma(acc[k & 3], av[k], x[u][(4 * k + t) * 8 + g]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) out[u][e] = (acc[0][e] + acc[1][e]) + (acc[2][e] + acc[3][e]);
+  }
+}
+
+// Columns of a 64-row block (row i, column c at x[u][i * 8 + c]) by substitution:
+// a warp takes column w of each tile, lane l rows l and l + 32.
+template <int NT>
+__device__ __noinline__ void substitute_block(const double* ts, int dir, int m,
+                                              double* const (&x)[NT]) {
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r1 = lane + 32;
+  // the reciprocal pivots, before the chain (a division inside it: 8 us a block)
+  const double q0 = 1.0 / (lane < m ? ts[lane * TRI_PITCH + lane] : 1.0);
+  const double q1 = 1.0 / (r1 < m ? ts[r1 * TRI_PITCH + r1] : 1.0);
+  for (int u = 0; u < NT; ++u) {
+    double v0 = x[u][lane * 8 + w], v1 = x[u][r1 * 8 + w];
+    // the next column is on its way while this one's chain runs
+    auto column = [&](int s, double& t0, double& t1) {
+      const double* tp = ts + (dir == 0 ? s : m - 1 - s) * TRI_PITCH;
+      t0 = tp[lane];
+      t1 = tp[r1];
+    };
+    double t0, t1, n0 = 0.0, n1 = 0.0;
+    column(0, t0, t1);
+    for (int s = 0; s < m; ++s) {
+      const int p = dir == 0 ? s : m - 1 - s;
+      if (s + 1 < m) column(s + 1, n0, n1);
+      double xp = p < 32 ? v0 : v1;
+      if (dir == 1 && lane == (p & 31)) {
+        const double r = p < 32 ? q0 : q1;
+        xp = fabs(r) > 0x1p-1000 && fabs(r) < 0x1p1000 ? xp * r : xp / ts[p * TRI_PITCH + p];
+        (p < 32 ? v0 : v1) = xp;
+      }
+      xp = __shfl_sync(all, xp, p & 31);
+      if (dir == 0 ? lane > p && lane < m : lane < p) v0 = fma(-t0, xp, v0);
+      if (dir == 0 ? r1 > p && r1 < m : r1 < p) v1 = fma(-t1, xp, v1);
+      t0 = n0;
+      t1 = n1;
+    }
+    x[u][lane * 8 + w] = v0;
+    x[u][r1 * 8 + w] = v1;
+  }
+}
+
+// x <- U^-1 L^-1 x with the packed LU `a` (n x n, its triangles' inverses behind it)
 // in global memory.  The CTAs of a cluster (CL; otherwise one CTA) own block
 // rows rank, rank + size, ...: own[u][q][r][c] is column c of column tile u,
 // row r of owned block q.  Step b: its owner forms D_b x_b, one 8-row tile a
-// warp, and writes it to every CTA's xb[b mod 3]; all subtract A(b', b) x_b from
-// their blocks still to be solved.
+// warp, refines it where the triangle asks for that, and writes it to every CTA's
+// xb[b mod 3]; all subtract A(b', b) x_b from their blocks still to be solved.
+// xb[3], xb[4] and the triangle at `ts` are the refinement's: in shared memory, copied
+// a step ahead (from L2 or memory inside the chain a refined step took 4 us, not
+// 2), and not in registers, which doubled (120 -> 255).
 //
 // The chain is wait, update of the next block, its product, write: the owner
 // of the next step does those first and everybody else's updates overlap it.
@@ -172,6 +329,7 @@ __device__ __forceinline__ void block_product(const double (&av)[NB / 4],
 template <int NT, bool CL>
 __device__ void tri_solve(const double* __restrict__ a, int n, double* own, int own_blocks,
                           double (*xb)[NT][NB][8]) {
+  double* ts = &xb[TRI_BUFS][0][0][0];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   int rank = 0, size = 1;
   if (CL) {
@@ -181,15 +339,23 @@ __device__ void tri_solve(const double* __restrict__ a, int n, double* own, int 
   const int nb = (n + NB - 1) / NB;
   auto ox = [&](int u, int q) { return own + ((int64_t)u * own_blocks + q) * NB * 8; };
   double dv[NB / 4];
+  int mode = 0;
   auto load_diag = [&](int dir, int b) {
-    const int row = 8 * w + g, gr = b * NB + row;
-#pragma unroll
-    for (int k = 0; k < NB / 4; ++k) {
-      const int col = 4 * k + t;
-      double v = dir == 0 && col == row ? 1.0 : 0.0;
-      if ((dir == 0 ? col < row : col >= row) && gr < n && b * NB + col < n)
-        v = __ldg(a + (int64_t)(b * NB + col) * n + gr);
-      dv[k] = v;
+    const int m = min(NB, n - b * NB);
+    const int2 md = __ldg(tri_modes(a, n) + b);
+    mode = dir == 0 ? md.x : md.y;
+    const double* inv = tri_inverse(a, n, b);
+    load_tri(dir, m, [&](int c, int r) { return __ldg(inv + c * m + r); }, dv);
+    if (mode > 0) {
+      const double* tri = a + (int64_t)b * NB * n + b * NB;
+      for (int e = threadIdx.x; e < NB * m; e += SK_NT) {
+        const int i = e % NB, j = e / NB;
+        if (i < m)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                           (unsigned)__cvta_generic_to_shared(ts + j * TRI_PITCH + i)),
+                       "l"(tri + (int64_t)j * n + i)
+                       : "memory");
+      }
     }
   };
   double av[NB / 4];
@@ -202,20 +368,65 @@ __device__ void tri_solve(const double* __restrict__ a, int n, double* own, int 
     }
   };
   // x_b = D_b x_b of this CTA's block b, to all CTAs' buffers
-  auto solve_block = [&](int b, int buf) {
+  auto solve_block = [&](int dir, int b, int buf) {
     const int q = CL ? b / size : b;
-    __syncthreads();  // the block's updates, by all warps
+    const int m = min(NB, n - b * NB), at = (tri_rows(w) + g) * 8 + 2 * t;  // this lane's
+    if (mode > 0) asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // the block's updates, by all warps; its triangle
     const double* x[NT];
     double y[NT][2];
 #pragma unroll
     for (int u = 0; u < NT; ++u) x[u] = ox(u, q);
-    block_product<NT>(dv, x, y);
-    __syncthreads();
+    if (mode == TRI_SUBST) {
+      double* xs[NT];
+#pragma unroll
+      for (int u = 0; u < NT; ++u) xs[u] = ox(u, q);
+      substitute_block<NT>(ts, dir, m, xs);
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < NT; ++u) {
+        y[u][0] = x[u][at];
+        y[u][1] = x[u][at + 1];
+      }
+    } else {
+      tri_product<NT>(dir, dv, x, y);
+    }
+    const double *yp[NT], *rp[NT];
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+      yp[u] = &xb[3][u][0][0];
+      rp[u] = &xb[4][u][0][0];
+    }
+#pragma unroll 1
+    for (int it = 0; it < (mode == TRI_SUBST ? 0 : mode); ++it) {  // y += D (x - T y)
+      double v[NT][2];
+#pragma unroll
+      for (int u = 0; u < NT; ++u)
+        *reinterpret_cast<double2*>(&xb[3][u][0][0] + at) = make_double2(y[u][0], y[u][1]);
+      __syncthreads();
+      double tv[NB / 4];
+      load_tri(dir, m, [&](int c, int r) { return ts[c * TRI_PITCH + r]; }, tv);
+      tri_product<NT>(dir, tv, yp, v);
+#pragma unroll
+      for (int u = 0; u < NT; ++u) {
+        const double2 r = *reinterpret_cast<const double2*>(x[u] + at);
+        *reinterpret_cast<double2*>(&xb[4][u][0][0] + at) =
+            make_double2(r.x - v[u][0], r.y - v[u][1]);
+      }
+      __syncthreads();
+      tri_product<NT>(dir, dv, rp, v);
+#pragma unroll
+      for (int u = 0; u < NT; ++u) {
+        y[u][0] += v[u][0];
+        y[u][1] += v[u][1];
+      }
+    }
+    if (mode == 0) __syncthreads();  // everybody has read x
 #pragma unroll
     for (int u = 0; u < NT; ++u) {
       const double2 v = make_double2(y[u][0], y[u][1]);
-      *reinterpret_cast<double2*>(ox(u, q) + (8 * w + g) * 8 + 2 * t) = v;
-      double* to = &xb[buf][u][8 * w + g][2 * t];
+      *reinterpret_cast<double2*>(ox(u, q) + at) = v;
+      double* to = &xb[buf][u][0][0] + at;
       if (CL)
         for (int r = 0; r < size; ++r)
           *reinterpret_cast<double2*>(cg::this_cluster().map_shared_rank(to, r)) = v;
@@ -229,7 +440,7 @@ __device__ void tri_solve(const double* __restrict__ a, int n, double* own, int 
     auto mine = [&](int step) { return step < nb && (!CL || block_of(step) % size == rank); };
     if (mine(0)) {
       load_diag(dir, block_of(0));
-      solve_block(block_of(0), 0);
+      solve_block(dir, block_of(0), 0);
     }
     if (CL) cluster_arrive();
 #pragma unroll 1
@@ -272,7 +483,7 @@ __device__ void tri_solve(const double* __restrict__ a, int n, double* own, int 
           *x = v;
         }
         if (i == 0 && next) {
-          solve_block(block_of(step + 1), (step + 1) % 3);
+          solve_block(dir, block_of(step + 1), (step + 1) % 3);
           if (CL) cluster_arrive();
         }
       }
@@ -288,12 +499,12 @@ __device__ void tri_solve(const double* __restrict__ a, int n, double* own, int 
 // ------------------------------------------------------------------ leaves
 // One CTA per leaf and 8 NT columns, the leaf's rows in shared memory.
 template <int NT>
-__global__ void __launch_bounds__(SK_NT) leaf_apply_kernel(LeafSolveLaunch L) {
+__global__ void __launch_bounds__(SK_NT, 2) leaf_apply_kernel(LeafSolveLaunch L) {
   extern __shared__ __align__(16) double dyn[];
   const int leaf = blockIdx.x, c0 = blockIdx.y * 8 * NT;
   const int r0 = L.leaf_min[leaf], s = L.leaf_size[leaf], nb = (s + NB - 1) / NB;
   double* own = dyn;
-  auto xb = reinterpret_cast<double(*)[NT][NB][8]>(dyn + (size_t)NT * nb * NB * 8);  // 3 buffers
+  auto xb = reinterpret_cast<double(*)[NT][NB][8]>(dyn + (size_t)NT * nb * NB * 8);  // TRI_BUFS
   const int* perm = L.perm + r0;
   for (int e = threadIdx.x; e < 8 * NT * nb * NB; e += SK_NT) {
     const int i = e % (nb * NB), c = e / (nb * NB);
@@ -322,7 +533,7 @@ __global__ void __launch_bounds__(SK_NT) leaf_apply_kernel(LeafSolveLaunch L) {
 // column-major (n x nrhs at the node's z).  Cluster `size` CTAs per (node,
 // column tile); grid.x = node * size + rank.
 template <int NT, bool PARTS, bool CL>
-__global__ void __launch_bounds__(SK_NT) cap_solve_kernel(CapLaunch L, int nrhs, int own_max,
+__global__ void __launch_bounds__(SK_NT, 2) cap_solve_kernel(CapLaunch L, int nrhs, int own_max,
                                                           unsigned* err) {
   extern __shared__ __align__(16) double dyn[];
   int rank = 0, size = 1;
@@ -348,11 +559,20 @@ __global__ void __launch_bounds__(SK_NT) cap_solve_kernel(CapLaunch L, int nrhs,
       if (q < 0 || q >= n) {
         atomicOr(err, DEV_ERR_INDEX | DEV_ERR_AT_SOLVE_PIV);
       } else if (PARTS) {
-        const int h = q >= N.off[0] && q < N.off[0] + N.m[0] ? 0 : 1;
-        const double* p = L.part + N.part[h] + (int64_t)(q - N.off[h]) * NCP + c;
-        const int64_t st = (int64_t)N.m[h] * NCP;
-#pragma unroll 16
-        for (int k = 0; k < N.chunks[h]; ++k) v += __ldg(p + k * st);
+        const bool h = !(q >= N.off[0] && q < N.off[0] + N.m[0]);
+        const double* p = L.part + (h ? N.part[1] : N.part[0]) +
+                          (int64_t)(q - (h ? N.off[1] : N.off[0])) * NCP + c;
+        const int64_t st = (int64_t)(h ? N.m[1] : N.m[0]) * NCP;
+        const int count = h ? N.chunks[1] : N.chunks[0];
+        constexpr int U = 16;  // loads in flight, added in order
+        for (int k = 0; k < count; k += U) {
+          double s[U];
+#pragma unroll
+          for (int i = 0; i < U; ++i) s[i] = k + i < count ? __ldg(p + (k + i) * st) : 0.0;
+#pragma unroll
+          for (int i = 0; i < U; ++i)
+            if (k + i < count) v += s[i];
+        }
       } else if (c0 + c < nrhs) {
         v = L.z[N.z + (int64_t)(c0 + c) * n + q];
       }
@@ -561,20 +781,24 @@ __global__ void __launch_bounds__(SK_NT) skinny_nn_kernel(const NnItem* __restri
   } while (0)
 
 constexpr size_t kCapSmem = 200 * 1024;
+// Shared memory of tri_solve beside the owned rows.
+constexpr size_t tri_smem(int nt) {
+  return sizeof(double) * (size_t)(TRI_BUFS * nt * NB * 8 + NB * TRI_PITCH);
+}
 
 template <int NT, bool PARTS>
 int cap_launch(const CapLaunch& L, int nnodes, int nrhs, int max_sd, unsigned* err,
                cudaStream_t s) {
   const int nb = (max_sd + NB - 1) / NB;
   auto smem_of = [&](int c) {
-    return sizeof(double) * 8 * NB * NT * (size_t)((nb + c - 1) / c + 3);
+    return sizeof(double) * 8 * NB * NT * (size_t)((nb + c - 1) / c) + tri_smem(NT);
   };
   // CTAs of a cluster: at least two block rows each, and as few nodes as leave
   // SMs over; more where the rows would not fit
   int size = 1;
   while (size < 8 && (smem_of(size) > kCapSmem || (nb >= 4 * size && nnodes * size < 148))) size *= 2;
   if (L.big) size = 1;
-  const size_t smem = L.big ? sizeof(double) * 8 * NB * NT * 3 : smem_of(size);
+  const size_t smem = L.big ? tri_smem(NT) : smem_of(size);
   if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
   const dim3 grid(nnodes * size, (nrhs + 8 * NT - 1) / (8 * NT));
   const int own = (nb + size - 1) / size;
@@ -603,7 +827,7 @@ int cap_launch(const CapLaunch& L, int nnodes, int nrhs, int max_sd, unsigned* e
 
 int64_t cap_big_elems(int nnodes, int nrhs, int max_sd) {
   const int nt = skinny_tiles(nrhs), nb = (max_sd + NB - 1) / NB;
-  if (sizeof(double) * 8 * NB * nt * (size_t)((nb + 7) / 8 + 3) <= kCapSmem) return 0;
+  if (sizeof(double) * 8 * NB * nt * (size_t)((nb + 7) / 8) + tri_smem(nt) <= kCapSmem) return 0;
   return (int64_t)nnodes * ((nrhs + 8 * nt - 1) / (8 * nt)) * nt * nb * NB * 8;
 }
 
@@ -623,7 +847,7 @@ int tri_invert_nodes_launch(const SchurLaunch& L, int* perm, int nnodes, int max
 int leaf_apply_launch(const LeafSolveLaunch& L, int nleaves, int smax, cudaStream_t s) {
   if (L.ncols <= 0 || nleaves == 0) return 0;
   const int nt = skinny_tiles(L.ncols), nb = (smax + NB - 1) / NB;
-  const size_t smem = sizeof(double) * 8 * NB * nt * (size_t)(nb + 3);
+  const size_t smem = sizeof(double) * 8 * NB * nt * (size_t)nb + tri_smem(nt);
   const dim3 grid(nleaves, (L.ncols + 8 * nt - 1) / (8 * nt));
   if (nt == 1) {
     LCK(smem_opt_in((const void*)leaf_apply_kernel<1>, smem));

@@ -6,8 +6,15 @@
 
 #include "lu.h"
 
-// Rows of the diagonal blocks whose triangles are stored inverted.
+// Rows of the diagonal blocks whose triangles' inverses are kept.
 constexpr int TRI_NB = 64;
+// Doubles behind an n x n packed LU for them: the inverses of block after block
+// (column-major, leading dimension the block's rows), then an int2 a block, how
+// its lower and its upper triangle are solved.
+__host__ __device__ inline int64_t tri_elems(int n) {
+  const int nb = (n + TRI_NB - 1) / TRI_NB, last = n - (nb - 1) * TRI_NB;
+  return n > 0 ? (int64_t)(nb - 1) * TRI_NB * TRI_NB + last * last + nb : 0;
+}
 // Right-hand sides the row-major path takes (two tiles of 8).
 constexpr int SKINNY_MAX = 16;
 // Rows of V^T X that go through shared memory at a time; a panel's start may be
@@ -34,7 +41,7 @@ struct NnItem {
 // solution goes.
 struct CapNode {
   int n, pad;
-  int64_t s_off, p_off;  // LU (triangles of the diagonal blocks inverted), permutation
+  int64_t s_off, p_off;  // LU (and tri_elems), permutation
   int off[2], m[2], chunks[2];
   int64_t part[2];
   int64_t z;  // row-major result / column-major right-hand sides and result
@@ -56,8 +63,8 @@ inline int skinny_tiles(int nrhs) { return nrhs <= 8 ? 1 : 2; }
 // a cluster (doubles; 0: they fit).
 int64_t cap_big_elems(int nnodes, int nrhs, int max_sd);
 
-// In place: the triangles of every TRI_NB diagonal block of the packed LUs
-// (n x n at off, column-major) become their inverses.
+// The inverses of the triangles of every TRI_NB diagonal block of the packed LUs
+// (n x n at off, column-major, tri_elems(n) doubles behind each).
 int tri_invert_leaves_launch(const LeafSolveLaunch& L, int nleaves, int smax, cudaStream_t s);
 // The same for the nodes' capacitance LUs, and their interchanges as
 // permutations: perm[i] = row of the right-hand side that becomes row i.

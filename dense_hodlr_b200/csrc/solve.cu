@@ -228,7 +228,8 @@ int solve_in_place(hodlr_t h, int nrhs) {
     if (!rc && h->checked)
       for (const auto& sn : L.nodes) {
         const int64_t sd = sn.kb + sn.kt;
-        rc = check_extent(h, L.S + sn.s_off, sizeof(double) * sd * sd, "capacitance LU", "solve");
+        rc = check_extent(h, L.S + sn.s_off, sizeof(double) * (sd * sd + tri_elems((int)sd)),
+                          "capacitance LU", "solve");
         if (!rc) rc = check_extent(h, L.perm + sn.p_off, sizeof(int) * sd, "permutation", "solve");
         if (rc) break;
       }
