@@ -1,14 +1,18 @@
 // Fast FP64 kernel entries for the full-kernel product K x.
 //
-// The product needs FP64-accurate entries (a few ulp), not entries that are
-// bit-identical to the ones ACA used, so it may contract into FMAs and use a
-// cheaper exponential.  exp here follows Tang's table-driven method (P. T. P.
+// The product needs FP64-accurate entries (a few ulp of a kernel of the distances
+// that it forms), not entries that are bit-identical to the ones ACA used, so it
+// may contract into FMAs and use a cheaper exponential.  exp here follows Tang's table-driven method (P. T. P.
 // Tang, "Table-driven implementation of the exponential function in IEEE
 // floating-point arithmetic", ACM TOMS 15(2), 1989), in units of ln2 / T: with
 // z = x T / ln2 = n + f, e^-x = 2^-(n / T) 2^(-f / T), the first factor from a
 // table of correctly rounded 2^(-j/T) and an exponent shift, the second from a
-// polynomial.  The unit is folded into the point coordinates, so f = z - n is
-// exact and no second multiplication by a split ln2 / T is left.
+// polynomial.  The unit is folded into the scale of the distances, so f = z - n is
+// exact and no second multiplication by a split ln2 / T is left.  The symmetric
+// forms scale the coordinates: a distance then carries an error of 2^-53 times the
+// coordinates, in length scales.  The row-by-row and forest forms scale the distance
+// (one more multiplication per entry): nearby coordinates subtract exactly, wherever
+// the cloud lies.
 //
 // The product is bound by issue: an FP64 instruction takes a scheduler two cycles
 // (64 lanes a cycle and SM), every other one takes one and hides behind nothing.
@@ -72,7 +76,8 @@ struct ExpTab {
 
   // t = 2^-(n / T) and f of z >= 0, n = rint(z): the low word of z + 1.5 * 2^52.
   // z is clamped at 1020 T by its high word, so that 2^-n/T stays normal: from
-  // x = 707 on the factor is about 1e-307, and a NaN goes on in z itself.
+  // x = 707 on the factor is about 1e-307.  A NaN is clamped with it: (1 + x) e^-x
+  // returns the NaN of its own x, a plain e^-x the clamped value.
   __device__ __forceinline__ void split(double z, double& t, double& f) const {
     constexpr int ZMAX = (1023 + 9 + LOGT) << 20 | 0xfe000;  // high word of 1020 T
     const double zc = __hiloint2double(min(__double2hiint(z), ZMAX), __double2loint(z));
@@ -145,17 +150,37 @@ __device__ __forceinline__ double hx_point_scale(double a, double unit) {
   if (KTYPE == HX_KERNEL_MATERN32 || KTYPE == HX_KERNEL_EXPONENTIAL) return a * unit;
   return sqrt(a);  // inverse multiquadric, quadratic
 }
+// (1 + x) e^-x, z = x T / ln2
+template <class E>
+__device__ __forceinline__ double hx_matern32(double z, const E& e) {
+  double t, f;
+  e.split(z, t, f);
+  return e.scaled(t, f, fma(z, e.l, 1.0));
+}
 template <int KTYPE, class E>
 __device__ __forceinline__ double hx_kernel_unit(double r2, const E& e) {
   if (KTYPE == HX_KERNEL_GAUSSIAN) return e.neg_exp(r2);
-  if (KTYPE == HX_KERNEL_MATERN32) {
-    const double z = hx_sqrt_nr(r2, e.k375);
-    double t, f;
-    e.split(z, t, f);
-    return e.scaled(t, f, fma(z, e.l, 1.0));  // (1 + x) e^-x
-  }
+  if (KTYPE == HX_KERNEL_MATERN32) return hx_matern32(hx_sqrt_nr(r2, e.k375), e);
   if (KTYPE == HX_KERNEL_INV_MULTIQUADRIC) return hx_rsqrt_nr(1.0 + r2, e.k375);
   if (KTYPE == HX_KERNEL_QUADRATIC) return 1.0 + r2;
   return e.neg_exp(hx_sqrt_nr(r2, e.k375));
+}
+
+// The same from an unscaled squared distance r2 >= HX_R2_RAW_FLOOR and c =
+// hx_distance_scale<KTYPE>(a, E::UNIT): one more multiplication per entry.
+#define HX_R2_RAW_FLOOR 1e-300
+template <int KTYPE>
+__device__ __forceinline__ double hx_distance_scale(double a, double unit) {
+  if (KTYPE == HX_KERNEL_GAUSSIAN) return -a * unit;
+  if (KTYPE == HX_KERNEL_MATERN32 || KTYPE == HX_KERNEL_EXPONENTIAL) return a * unit;
+  return a;  // inverse multiquadric, quadratic
+}
+template <int KTYPE, class E>
+__device__ __forceinline__ double hx_kernel_raw(double r2, double c, const E& e) {
+  if (KTYPE == HX_KERNEL_GAUSSIAN) return e.neg_exp(r2 * c);
+  if (KTYPE == HX_KERNEL_MATERN32) return hx_matern32(hx_sqrt_nr(r2, e.k375) * c, e);
+  if (KTYPE == HX_KERNEL_INV_MULTIQUADRIC) return hx_rsqrt_nr(fma(r2, c, 1.0), e.k375);
+  if (KTYPE == HX_KERNEL_QUADRATIC) return fma(r2, c, 1.0);
+  return e.neg_exp(hx_sqrt_nr(r2, e.k375) * c);
 }
 #endif

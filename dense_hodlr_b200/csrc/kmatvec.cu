@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(KT) kmatvec_kernel(KmatvecLaunch L) {
   const int jb = blockIdx.y * per, je = min(n, jb + per);
   if (DIM > 0) ExpG::fill(tab);
   const ExpG ex(tab);
-  const double cs = hx_point_scale<KTYPE>(L.src.kp.a, ExpG::UNIT);
+  const double cs = hx_distance_scale<KTYPE>(L.src.kp.a, ExpG::UNIT);
   int row[RPT];
   bool live[RPT];
   double xi[RPT][DIM > 0 ? DIM : 1];
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(KT) kmatvec_kernel(KmatvecLaunch L) {
     row[q] = blockIdx.x * (KT * RPT) + q * KT + threadIdx.x;
     live[q] = row[q] < n;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) xi[q][d] = live[q] ? cs * L.src.pts[d * L.src.ld + row[q]] : 0.0;
+    for (int d = 0; d < DIM; ++d) xi[q][d] = live[q] ? L.src.pts[d * L.src.ld + row[q]] : 0.0;
 #pragma unroll
     for (int c = 0; c < NR; ++c) acc[q][c] = 0.0;
   }
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(KT) kmatvec_kernel(KmatvecLaunch L) {
     if (threadIdx.x < jn) {
       const int j = j0 + threadIdx.x;
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) xs[d][threadIdx.x] = cs * L.src.pts[d * L.src.ld + j];
+      for (int d = 0; d < DIM; ++d) xs[d][threadIdx.x] = L.src.pts[d * L.src.ld + j];
 #pragma unroll
       for (int c = 0; c < NR; ++c)
         vs[c][threadIdx.x] = c < L.nrhs ? L.X[(int64_t)c * L.ldx + j] : 0.0;
@@ -78,13 +78,13 @@ __global__ void __launch_bounds__(KT) kmatvec_kernel(KmatvecLaunch L) {
           kij = live[q] ? L.src.A[(int64_t)(j0 + t) * L.src.ld + row[q]] : 0.0;
         } else {
           // off-diagonal formula everywhere; the diagonal is corrected below
-          double r2 = HX_R2_FLOOR;
+          double r2 = HX_R2_RAW_FLOOR;
 #pragma unroll
           for (int d = 0; d < DIM; ++d) {
             double dd = xi[q][d] - xs[d][t];
             r2 = fma(dd, dd, r2);
           }
-          kij = hx_kernel_unit<KTYPE>(r2, ex);
+          kij = hx_kernel_raw<KTYPE>(r2, cs, ex);
         }
 #pragma unroll
         for (int c = 0; c < NR; ++c) acc[q][c] = fma(kij, vs[c][t], acc[q][c]);
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(KT) kmatvec_forest_kernel(KmatvecLaunch L,
   const hx_kparams kp = L.src.kps[it.w];
   ExpG::fill(tab);
   const ExpG ex(tab);
-  const double cs = hx_point_scale<KTYPE>(kp.a, ExpG::UNIT);
+  const double cs = hx_distance_scale<KTYPE>(kp.a, ExpG::UNIT);
   int row[RPT];
   bool live[RPT];
   double xi[RPT][DIM];
@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(KT) kmatvec_forest_kernel(KmatvecLaunch L,
     row[q] = it.x + q * KT + threadIdx.x;
     live[q] = row[q] < it.z;
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) xi[q][d] = live[q] ? cs * L.src.pts[d * L.src.ld + row[q]] : 0.0;
+    for (int d = 0; d < DIM; ++d) xi[q][d] = live[q] ? L.src.pts[d * L.src.ld + row[q]] : 0.0;
 #pragma unroll
     for (int c = 0; c < NR; ++c) acc[q][c] = 0.0;
   }
@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(KT) kmatvec_forest_kernel(KmatvecLaunch L,
     if (threadIdx.x < jn) {
       const int j = j0 + threadIdx.x;
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) xs[d][threadIdx.x] = cs * L.src.pts[d * L.src.ld + j];
+      for (int d = 0; d < DIM; ++d) xs[d][threadIdx.x] = L.src.pts[d * L.src.ld + j];
 #pragma unroll
       for (int c = 0; c < NR; ++c)
         vs[c][threadIdx.x] = c < L.nrhs ? L.X[(int64_t)c * L.ldx + j] : 0.0;
@@ -705,13 +705,13 @@ __global__ void __launch_bounds__(KT) kmatvec_forest_kernel(KmatvecLaunch L,
     for (int t = 0; t < jn; ++t) {
 #pragma unroll
       for (int q = 0; q < RPT; ++q) {
-        double r2 = HX_R2_FLOOR;
+        double r2 = HX_R2_RAW_FLOOR;
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
           const double dd = xi[q][d] - xs[d][t];
           r2 = fma(dd, dd, r2);
         }
-        const double kij = hx_kernel_unit<KTYPE>(r2, ex);
+        const double kij = hx_kernel_raw<KTYPE>(r2, cs, ex);
 #pragma unroll
         for (int c = 0; c < NR; ++c) acc[q][c] = fma(kij, vs[c][t], acc[q][c]);
       }
