@@ -62,6 +62,8 @@ SIGNATURES = {
     "hodlr_set_capacity_hint": (_I, [_H, _PI, _I]),
     "hodlr_set_factor_in_place": (_I, [_H, _I]),
     "hodlr_set_aca_streaming": (_I, [_H, _I]),
+    "hodlr_set_memory_limit": (_I, [_H, ctypes.c_longlong]),
+    "hodlr_get_memory_held": (_I, [_H, ctypes.POINTER(ctypes.c_longlong)]),
     "hodlr_set_wait_limit": (_I, [_H, ctypes.c_uint, _I]),
     "hodlr_set_checked": (_I, [_H, _I]),
     "hodlr_set_solver_form": (_I, [_H, _I]),

@@ -82,33 +82,16 @@ int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_ma
     std::vector<int> table((size_t)ncta);
     for (int i = 0; i < nb; ++i)
       for (int c = 0; c < blocks[i].G; ++c) table[(size_t)(blocks[i].g0 + c)] = i;
-    if (ncta > h->cta_cap) {
-      dfree(h, h->d_cta);
-      CK(dalloc(h, &h->d_cta, (size_t)ncta));
-      h->cta_cap = ncta;
-    }
+    CK(dgrow(h, h->d_cta, h->cta_cap, ncta));
     CK(cudaMemcpyAsync(h->d_cta, table.data(), sizeof(int) * ncta, cudaMemcpyHostToDevice,
                        h->stream));
   }
-  if (nb > h->blocks_cap) {
-    dfree(h, h->d_blocks);
-    CK(dalloc(h, &h->d_blocks, (size_t)nb));
-    h->blocks_cap = nb;
-  }
+  CK(dgrow(h, h->d_blocks, h->blocks_cap, nb));
   CK(cudaMemcpyAsync(h->d_blocks, blocks.data(), sizeof(AcaBlock) * nb, cudaMemcpyHostToDevice,
                      h->stream));
   int64_t stride = 12 + 4 * (int64_t)kcap_max;  // args + two banks of dots and norms
-  int64_t need = stride * ncta;
-  if (need > h->part_cap) {
-    dfree(h, h->part);
-    CK(dalloc(h, &h->part, (size_t)need));
-    h->part_cap = need;
-  }
-  if (nb > h->bar_cap) {
-    dfree(h, h->bar);
-    CK(dalloc(h, &h->bar, (size_t)nb));
-    h->bar_cap = nb;
-  }
+  CK(dgrow(h, h->part, h->part_cap, stride * ncta));
+  CK(dgrow(h, h->bar, h->bar_cap, nb));
   CK(cudaMemsetAsync(h->bar, 0, sizeof(unsigned) * nb, h->stream));
   AcaLaunch L;
   L.blocks = h->d_blocks;
@@ -142,11 +125,7 @@ int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_ma
     L.ring_stages = aca_group_ring(variant, rows, kcap_max, group_smem_budget(variant), &L.stage_elems,
                                    &smem);
     if (!L.ring_stages) return fail(h, HODLR_ERR_STATE, "ACA ring does not fit");
-    if (ncta > h->slots_cap) {
-      dfree(h, h->slots);
-      CK(dalloc(h, &h->slots, (size_t)ncta * 128 + 128));
-      h->slots_cap = ncta;
-    }
+    CK(dgrow(h, h->slots, h->slots_cap, (int64_t)ncta * 128 + 128));
     L.slots = h->slots;
     CK(cudaMemsetAsync(h->slots, 0, (size_t)ncta * 128 + 128, h->stream));
     L.idle = reinterpret_cast<unsigned*>(h->slots + (size_t)ncta * 128);
@@ -154,11 +133,8 @@ int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_ma
     L.pub_stride = 16 * ((int64_t)kcap_max + 1);
     const int64_t pneed = 2 * L.pub_stride * ncta;
     if (pneed > h->pub_cap) {
-      dfree(h, h->pub);
-      h->pub_cap = 0;
-      CK(dalloc(h, &h->pub, (size_t)pneed));
+      CK(dgrow(h, h->pub, h->pub_cap, pneed));
       CK(cudaMemsetAsync(h->pub, 0, (size_t)pneed, h->stream));
-      h->pub_cap = pneed;
     }
     L.pub = h->pub;
     L.launch_tag = ++h->aca_tag;
@@ -179,12 +155,7 @@ int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_ma
     if (aca_dots_global(nt, kcap_max)) L.dotg_stride = (int64_t)(nt / 32) * kcap_max;
   }
   if (L.dotg_stride > 0) {
-    const int64_t dneed = L.dotg_stride * ncta;
-    if (dneed > h->dotg_cap) {
-      dfree(h, h->dotg);
-      CK(dalloc(h, &h->dotg, (size_t)dneed));
-      h->dotg_cap = dneed;
-    }
+    CK(dgrow(h, h->dotg, h->dotg_cap, L.dotg_stride * ncta));
     L.dotg = h->dotg;
   }
   bool coop = G > 1;
@@ -337,7 +308,7 @@ int predict_ranks(hodlr_t h) {
 // The working layout's memory goes back to the device pool, not to the
 // handle's cache: the factorization's panels are cut from it next.
 void free_aca_work(hodlr_t h) {
-  if (h->aca_work) cudaFreeAsync(h->aca_work, h->stream);
+  if (h->aca_work) h->pool.raw_free(h->aca_work, sizeof(double) * (size_t)h->aca_work_cap, h->stream);
   h->aca_work = nullptr;
   h->aca_work_cap = 0;
 }

@@ -363,11 +363,7 @@ int do_factorize(hodlr_t h) {
     CK(dalloc(h, &L.perm, (size_t)p_tot));
     CK(dalloc(h, &L.d_nodes, (size_t)nn));
     CK(h2d_async(h, L.d_nodes, L.nodes.data(), sizeof(SchurNode) * nn));
-    if (z_tot > h->z_cap) {
-      dfree(h, h->Z);
-      CK(dalloc(h, &h->Z, (size_t)z_tot));
-      h->z_cap = z_tot;
-    }
+    CK(dgrow(h, h->Z, h->z_cap, z_tot));
     // Z_h = V_h^T [Y_0 .. Y_{l-1} | own U columns of Y_l] on the node's rows:
     // Z columns [coff_a, coff_a + kmax_a) from level a < l, then the own
     // rank(U_h) columns at coff_l, one grouped-GEMM problem per panel

@@ -102,10 +102,7 @@ void free_compress(hodlr_t h) {
 }
 
 int ensure_ws(hodlr_t h, int64_t elems) {
-  if (elems <= h->ws_cap) return HODLR_OK;
-  dfree(h, h->ws);
-  CK(dalloc(h, &h->ws, (size_t)elems));
-  h->ws_cap = elems;
+  CK(dgrow(h, h->ws, h->ws_cap, elems));
   return HODLR_OK;
 }
 

@@ -108,6 +108,7 @@ struct Level {
   TnItem* d_stn = nullptr;        // solve of few right-hand sides: V^T X, X -= Y y
   NnItem* d_snn = nullptr;
   int nstn = 0, nsnn = 0;
+  int64_t spart_need = 0;         // elements of h->spart that they use
 };
 
 inline void block_geom(const Level& L, int q, int& r0, int& c0, int& m, int& n) {
@@ -138,10 +139,17 @@ struct DevPool {
   cudaMemPool_t mp = nullptr;
   std::multimap<size_t, void*> freeb, pending;
   std::unordered_map<void*, size_t> size;
+  size_t held = 0, limit = 0;  // bytes from the device pool; most of them (0: no limit)
   cudaError_t raw_alloc(void** p, size_t bytes, cudaStream_t s) {
     if (!mp) mp = device_pool();
-    if (!mp) return cudaErrorMemoryAllocation;
-    return cudaMallocFromPoolAsync(p, bytes, mp, s);
+    if (!mp || (limit && held + bytes > limit)) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, mp, s);
+    if (e == cudaSuccess) held += bytes;
+    return e;
+  }
+  void raw_free(void* p, size_t bytes, cudaStream_t s) {
+    cudaFreeAsync(p, s);
+    held -= bytes;
   }
   cudaError_t alloc(void** p, size_t bytes, cudaStream_t s) {
     bytes = (bytes + 255) & ~(size_t)255;
@@ -164,7 +172,7 @@ struct DevPool {
       cudaGetLastError();
       release_free(s);
       for (auto& f : pending) {
-        cudaFreeAsync(f.second, s);
+        raw_free(f.second, f.first, s);
         size.erase(f.second);
       }
       pending.clear();
@@ -191,13 +199,13 @@ struct DevPool {
   }
   void release_free(cudaStream_t s) {
     for (auto& f : freeb) {
-      cudaFreeAsync(f.second, s);
+      raw_free(f.second, f.first, s);
       size.erase(f.second);
     }
     freeb.clear();
   }
   void release_all(cudaStream_t s) {
-    for (auto& f : size) cudaFreeAsync(f.first, s);
+    for (auto& f : size) raw_free(f.first, f.second, s);
     size.clear();
     freeb.clear();
     pending.clear();
@@ -352,6 +360,18 @@ template <class T>
 void dfree(hodlr_t h, T*& p) {
   if (p) h->pool.free((void*)p);
   p = nullptr;
+}
+
+// p with room for `need` elements, contents lost when it grows.  cap is 0 from the
+// moment that the old buffer is given up until there is a new one.
+template <class T, class C>
+cudaError_t dgrow(hodlr_t h, T*& p, C& cap, int64_t need) {
+  if (need <= cap) return cudaSuccess;
+  dfree(h, p);
+  cap = 0;
+  const cudaError_t e = dalloc(h, &p, (size_t)need);
+  if (e == cudaSuccess) cap = (C)need;
+  return e;
 }
 
 int fail(hodlr_t h, int code, const std::string& msg);

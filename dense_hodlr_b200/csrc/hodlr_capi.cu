@@ -466,6 +466,18 @@ int hodlr_trim_device_memory(void) {
   return cudaMemPoolTrimTo(mp, 0) == cudaSuccess ? HODLR_OK : HODLR_ERR_CUDA;
 }
 
+int hodlr_set_memory_limit(hodlr_t h, long long bytes) {
+  if (!h || bytes < 0) return HODLR_ERR_ARG;
+  h->pool.limit = (size_t)bytes;
+  return HODLR_OK;
+}
+
+int hodlr_get_memory_held(hodlr_t h, long long* bytes) {
+  if (!h || !bytes) return HODLR_ERR_ARG;
+  *bytes = (long long)h->pool.held;
+  return HODLR_OK;
+}
+
 int hodlr_set_capacity_hint(hodlr_t h, const int* caps, int nlevels) {
   if (!h || nlevels < 0 || (nlevels > 0 && !caps)) return HODLR_ERR_ARG;
   h->cap_hint.assign(caps, caps + nlevels);

@@ -89,30 +89,25 @@ int build_solve_plans(hodlr_t h, int nrhs) {
     big = std::max(big, cap_big_elems((int)L.nodes.size(), nrhs, L.max_sd));
   }
   if (zs_tot > h->zs_cap) {
-    dfree(h, h->zs);
-    CK(dalloc(h, &h->zs, (size_t)zs_tot));
-    h->zs_cap = zs_tot;
     for (auto& L : h->lv) L.solve_nrhs = -1;  // the GEMM plans point into it
+    CK(dgrow(h, h->zs, h->zs_cap, zs_tot));
   }
-  if (big > h->cap_big_cap) {
-    dfree(h, h->cap_big);
-    CK(dalloc(h, &h->cap_big, (size_t)big));
-    h->cap_big_cap = big;
-  }
+  CK(dgrow(h, h->cap_big, h->cap_big_cap, big));
   if (nrhs > h->x_cols) {
+    for (auto& L : h->lv) L.solve_nrhs = -1;  // the GEMM plans point into it
     dfree(h, h->X);
+    h->x_cols = 0;
     CK(dalloc(h, &h->X, (size_t)(N * nrhs)));
     h->x_cols = nrhs;
-    for (auto& L : h->lv) L.solve_nrhs = -1;  // the GEMM plans point into it
   }
-  int64_t part_tot = 0;
   for (auto& L : h->lv) {
     if (L.solve_nrhs == nrhs) continue;
+    L.solve_nrhs = -1;  // no plan until the whole new one is there
+    L.spart_need = 0;
     if (few) {
-      int64_t z = 0, part = 0;
-      int rc = build_few(h, L, nrhs, &z, &part);
+      int64_t z = 0;
+      int rc = build_few(h, L, nrhs, &z, &L.spart_need);
       if (rc) return rc;
-      part_tot = std::max(part_tot, part);
       L.solve_nrhs = nrhs;
       continue;
     }
@@ -187,11 +182,9 @@ int build_solve_plans(hodlr_t h, int nrhs) {
     if (rc) return rc;
     L.solve_nrhs = nrhs;
   }
-  if (part_tot > h->spart_cap) {
-    dfree(h, h->spart);
-    CK(dalloc(h, &h->spart, (size_t)part_tot));
-    h->spart_cap = part_tot;
-  }
+  int64_t part_tot = 0;  // of all levels, those planned by an earlier call too
+  for (auto& L : h->lv) part_tot = std::max(part_tot, L.spart_need);
+  CK(dgrow(h, h->spart, h->spart_cap, part_tot));
   return HODLR_OK;
 }
 
@@ -473,6 +466,7 @@ int refine_device(hodlr_t h, int nrhs, const double* d_b, int ldb, double* d_x, 
     dfree(h, h->ir_x);
     dfree(h, h->ir_y);
     dfree(h, h->ir_part);
+    h->ir_cols = 0;
     CK(dalloc(h, &h->ir_b, (size_t)(N * nrhs)));
     CK(dalloc(h, &h->ir_x, (size_t)(N * nrhs)));
     CK(dalloc(h, &h->ir_y, (size_t)(N * nrhs)));
@@ -544,6 +538,7 @@ int forest_refine_device(hodlr_t h, int nrhs, const double* d_b, int ldb, double
     dfree(h, h->ir_x);
     dfree(h, h->ir_y);
     dfree(h, h->ir_part);
+    h->ir_cols = 0;
     CK(dalloc(h, &h->ir_b, (size_t)(N * nrhs)));
     CK(dalloc(h, &h->ir_x, (size_t)(N * nrhs)));
     CK(dalloc(h, &h->ir_y, (size_t)(N * nrhs)));
@@ -788,6 +783,7 @@ int gmres_device(hodlr_t h, int nrhs, const double* d_b, int ldb, double* d_x, i
     dfree(h, h->ir_x);
     dfree(h, h->ir_y);
     dfree(h, h->ir_part);
+    h->ir_cols = 0;
     CK(dalloc(h, &h->ir_b, (size_t)(N * nrhs)));
     CK(dalloc(h, &h->ir_x, (size_t)(N * nrhs)));
     CK(dalloc(h, &h->ir_y, (size_t)(N * nrhs)));
@@ -800,6 +796,7 @@ int gmres_device(hodlr_t h, int nrhs, const double* d_b, int ldb, double* d_x, i
     dfree(h, h->gm_W);
     dfree(h, h->gm_h);
     dfree(h, h->gm_part);
+    h->gm_m = h->gm_cols = 0;
     CK(dalloc(h, &h->gm_V, (size_t)((m + 1) * N * nrhs)));
     CK(dalloc(h, &h->gm_Z, (size_t)(m * N * nrhs)));
     CK(dalloc(h, &h->gm_W, (size_t)(m * N * nrhs)));

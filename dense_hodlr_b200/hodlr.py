@@ -185,6 +185,17 @@ class HODLR_Matrix:
         on for every new handle."""
         _check(self._h, _L.lib().hodlr_set_checked(self._h, int(bool(on))))
 
+    def set_memory_limit(self, nbytes):
+        """Most device memory the handle may hold (0: no limit); calls that need
+        more raise HODLR_ERR_ALLOC and can be repeated with more room."""
+        _check(self._h, _L.lib().hodlr_set_memory_limit(self._h, int(nbytes)))
+
+    def memory_held(self):
+        """Device memory the handle holds, its cache included (bytes)."""
+        v = ctypes.c_longlong()
+        _check(self._h, _L.lib().hodlr_get_memory_held(self._h, ctypes.byref(v)))
+        return v.value
+
     def set_aca_streaming(self, on):
         """Top-level ACA panels through the CTAs' shared-memory rings (2, default,
         or 1), or loaded per thread (0).  Same results in every mode."""

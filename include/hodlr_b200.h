@@ -347,6 +347,13 @@ int hodlr_gemm_device(int precision, int mode, int m, int n, int k, const double
  * last factorization overwrote. */
 int hodlr_set_factor_in_place(hodlr_t h, int mode);
 
+/* Most device memory the handle may hold (0: no limit, the default), and what it
+ * holds now, its cache included (no counterpart in the reference).  A call that
+ * needs more returns HODLR_ERR_ALLOC, as on a device without free memory, and the
+ * handle stays usable: with more room, the same call succeeds. */
+int hodlr_set_memory_limit(hodlr_t h, long long bytes);
+int hodlr_get_memory_held(hodlr_t h, long long* bytes);
+
 /* How the ACA of the few-block top levels reads its W/V panel slices (no
  * counterpart in the reference): on = 2 (default) or 1 streams them through
  * a shared-memory ring per CTA, one bulk copy per panel column of a tile; 0
