@@ -102,7 +102,8 @@ int build_solve_plans(hodlr_t h, int nrhs) {
   }
   for (auto& L : h->lv) {
     if (L.solve_nrhs == nrhs) continue;
-    L.solve_nrhs = -1;  // no plan until the whole new one is there
+    drop_solve_graph(h);  // captured with the arrays of the plan that goes
+    L.solve_nrhs = -1;    // no plan until the whole new one is there
     L.spart_need = 0;
     if (few) {
       int64_t z = 0;
@@ -253,8 +254,9 @@ int solve_in_place(hodlr_t h, int nrhs) {
 }
 
 // solve_in_place through a CUDA graph: captured on first use, replayed while
-// the right-hand-side count, stream, buffers, precision and factorization
-// are the same (one launch instead of ~4 per level).
+// the right-hand-side count, stream, buffers, precision, factorization and
+// plans (build_solve_plans drops the graph) are the same: one launch instead of
+// ~4 per level.
 int solve_fast(hodlr_t h, int nrhs) {
   if (h->sg_off || h->checked) return solve_in_place(h, nrhs);
   const void* key[6] = {h->X, h->zs, h->ws, (const void*)(intptr_t)(h->gemm_prec + 1), h->spart,
