@@ -305,14 +305,6 @@ int predict_ranks(hodlr_t h) {
   return HODLR_OK;
 }
 
-// The working layout's memory goes back to the device pool, not to the
-// handle's cache: the factorization's panels are cut from it next.
-void free_aca_work(hodlr_t h) {
-  if (h->aca_work) h->pool.raw_free(h->aca_work, sizeof(double) * (size_t)h->aca_work_cap, h->stream);
-  h->aca_work = nullptr;
-  h->aca_work_cap = 0;
-}
-
 // ---- launches of the few-block levels
 //
 // Time of a block's ACA from k0 to k columns, in us: steps of two passes.  A pass is a fixed part
@@ -420,10 +412,11 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
   std::vector<GroupJob> jobs = group_jobs(h, set, rank_est);
   int ctas = h->num_sms, kcap_max = 1;
   for (int l : set) kcap_max = std::max(kcap_max, h->lv[l].kcap);
+  bool ring = h->aca_ring;
   for (;;) {  // a cooperative launch the driver refuses is retried with half the CTAs
     int variant = ACA_GROUP_NONE;
     const double t1 = share_ctas(jobs, ctas, ACA_GROUP_8x1);
-    if (h->aca_ring && t1 >= 0) {
+    if (ring && t1 >= 0) {
       int rows = 1, elems = 0, ps = 0;
       size_t bytes = 0;
       variant = ACA_GROUP_8x4;
@@ -436,8 +429,8 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
         variant = ACA_GROUP_NONE;  // too many columns beside a ring
       else if (aca_group_max_coresident(variant, bytes, &ps) || ps < 1)
         return fail(h, HODLR_ERR_CUDA, "occupancy query failed");
-      // the slices' working layout; without memory for it the panels are
-      // loaded from the arenas per thread
+      // the slices' working layout, in the pool's scratch; without memory for it
+      // the panels are loaded from the arenas per thread
       int64_t work = 0;
       for (auto& j : jobs) {
         int r0, c0, m, n;
@@ -448,16 +441,9 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
         j.strV = aca_group_slice(variant, (n + j.G - 1) / j.G, kcap);
         work += (j.strW + j.strV) * j.G;
       }
-      if (variant && work > h->aca_work_cap) {
-        free_aca_work(h);
-        if (h->pool.raw_alloc((void**)&h->aca_work, sizeof(double) * (size_t)work, h->stream) ==
-            cudaSuccess) {
-          h->aca_work_cap = work;
-        } else {
-          cudaGetLastError();
-          h->aca_work = nullptr;
-          variant = ACA_GROUP_NONE;
-        }
+      if (variant && h->pool.grow_scratch(sizeof(double) * (size_t)work, h->stream)) {
+        cudaGetLastError();
+        variant = ACA_GROUP_NONE;
       }
     }
     if (!variant) {
@@ -476,7 +462,7 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
       Level& L = h->lv[jobs[i].level];
       fill_block(h, L, jobs[i].q, bl[i]);
       if (variant) {
-        bl[i].sW = h->aca_work + jobs[i].work;
+        bl[i].sW = (double*)h->pool.scratch + jobs[i].work;
         bl[i].sV = bl[i].sW + jobs[i].strW * jobs[i].G;
         bl[i].strW = jobs[i].strW;
         bl[i].strV = jobs[i].strV;
@@ -495,7 +481,14 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
     // them are out of work, where a launch takes far longer than its overhead
     // (2D N = 262144: 107 ms against 133 with fixed shares)
     const int yield_at = jobs.size() > 1 && slowest > 2000.0 ? std::max(1, most / 3) : 0;
+    h->pool.scratch_busy = variant != ACA_GROUP_NONE;
     const int rc = run_aca(h, bl, 1, any ? 256 : 128, kcap_max, variant, &groups, yield_at);
+    h->pool.scratch_busy = false;
+    if (rc == HODLR_ERR_ALLOC && variant) {  // no room beside the working layout
+      h->pool.free_scratch(h->stream);
+      ring = false;
+      continue;
+    }
     if (rc != HODLR_ERR_RETRY_SMALLER) return rc;
     if (ctas == 1) return fail(h, HODLR_ERR_CUDA, "aca_launch: cooperative launch refused");
     ctas = std::max(1, ctas / 2);
@@ -616,7 +609,9 @@ int do_compress(hodlr_t h) {
     }
     for (auto it = set.rbegin(); it != set.rend(); ++it) note_rank(*it);
   }
-  free_aca_work(h);
+  // back to the device pool, not to the handle's cache: the factorization's
+  // panels are cut from it next
+  h->pool.free_scratch(h->stream);
   for (auto& L : h->lv)
     if (!level_done(L)) return fail(h, HODLR_ERR_STATE, "ACA did not converge in its launches");
   // ranks, level widths, column offsets, algorithmic bytes

@@ -167,6 +167,11 @@ struct DevPool {
         pending.clear();
       }
     }
+    const cudaError_t e = raw_alloc_or_trim(p, bytes, s);
+    if (e == cudaSuccess) size[*p] = bytes;
+    return e;
+  }
+  cudaError_t raw_alloc_or_trim(void** p, size_t bytes, cudaStream_t s) {
     cudaError_t e = raw_alloc(p, bytes, s);
     if (e == cudaErrorMemoryAllocation) {  // give back every cache, retry once
       cudaGetLastError();
@@ -176,11 +181,31 @@ struct DevPool {
         size.erase(f.second);
       }
       pending.clear();
+      if (!scratch_busy) free_scratch(s);
       cudaStreamSynchronize(s);
-      cudaMemPoolTrimTo(mp, 0);
+      if (mp) cudaMemPoolTrimTo(mp, 0);
       e = raw_alloc(p, bytes, s);
     }
-    if (e == cudaSuccess) size[*p] = bytes;
+    return e;
+  }
+  // One buffer whose contents nobody keeps: given back when anything else does
+  // not fit, except while a launch uses it (scratch_busy).
+  void* scratch = nullptr;
+  size_t scratch_bytes = 0;
+  bool scratch_busy = false;
+  void free_scratch(cudaStream_t s) {
+    if (scratch) raw_free(scratch, scratch_bytes, s);
+    scratch = nullptr;
+    scratch_bytes = 0;
+  }
+  cudaError_t grow_scratch(size_t bytes, cudaStream_t s) {
+    if (bytes <= scratch_bytes) return cudaSuccess;
+    free_scratch(s);
+    const cudaError_t e = raw_alloc_or_trim(&scratch, bytes, s);
+    if (e == cudaSuccess)
+      scratch_bytes = bytes;
+    else
+      scratch = nullptr;
     return e;
   }
   // the live allocation that holds [p, p + bytes), if any (checked mode)
@@ -205,6 +230,7 @@ struct DevPool {
     freeb.clear();
   }
   void release_all(cudaStream_t s) {
+    free_scratch(s);
     for (auto& f : size) raw_free(f.first, f.second, s);
     size.clear();
     freeb.clear();
@@ -319,8 +345,6 @@ struct hodlr_handle_s {
   int slots_cap = 0;
   unsigned char* pub = nullptr;    // its published rows, zeroed when allocated
   int64_t pub_cap = 0;
-  double* aca_work = nullptr;      // its blocks' slices while a compression runs
-  int64_t aca_work_cap = 0;
   unsigned aca_tag = 0;            // number of its last launch: no tag is used twice
   AcaBlock* d_blocks = nullptr;
   int blocks_cap = 0;
@@ -419,7 +443,6 @@ int level_kmax(const Level& L);
 std::vector<int4> block_geoms(hodlr_t h);
 int block_features_dev(hodlr_t h, const std::vector<int4>& geom, double l, float* d_F);
 int predict_ranks(hodlr_t h);
-void free_aca_work(hodlr_t h);
 int do_compress(hodlr_t h);
 int upload_plan(hodlr_t h, std::vector<GemmProblem>& probs, bool split, DevPlan& out,
                 const char* what = "grouped GEMM");

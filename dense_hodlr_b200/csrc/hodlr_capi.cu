@@ -282,7 +282,6 @@ void hodlr_destroy(hodlr_t h) {
   dfree(h, h->bar);
   dfree(h, h->slots);
   dfree(h, h->pub);
-  free_aca_work(h);
   dfree(h, h->d_blocks);
   dfree(h, h->d_cta);
   dfree(h, h->dotg);

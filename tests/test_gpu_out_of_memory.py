@@ -93,3 +93,29 @@ def test_whole_calls_that_do_not_fit():
         g.set_memory_limit(0)
         assert _close(g.recLU_Solve(b), x)
     assert failed
+
+
+@pytest.mark.parametrize("hint", [0, 8])
+def test_streamed_compression_fits_where_per_thread_loads_do(hint):
+    """The working layout of the group levels is a second copy of their panels: it
+    is given back when a level grows (hint: from 8 columns) or another one starts."""
+    n = 12001
+    pts = uniform_cube(n, 2, 6)
+
+    def compress(mode, limit):
+        g = HODLR_Matrix(n, n, KernelSpec("matern32", 0.2, 0.5), pts, 128)
+        g.set_LRTolerance(1e-8)
+        g.set_aca_streaming(mode)
+        if hint:
+            g.set_capacity_hint([hint] * 20)
+        g.set_memory_limit(limit)
+        g.storeLRinTree()
+        return g.ranks(), g.memory_held()
+
+    # what is held at the end, the cache included, is the most it ever was
+    ranks, low = compress(0, 0)
+    same, high = compress(2, 0)
+    assert np.array_equal(same, ranks)
+    # exchange slots and published rows of the group form: below 4 MB
+    for limit in np.linspace(low + (4 << 20), max(high, low) + (8 << 20), 20).astype(int):
+        assert np.array_equal(compress(2, limit)[0], ranks)
