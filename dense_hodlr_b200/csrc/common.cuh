@@ -10,12 +10,12 @@
 
 #define HODLR_INLINE __device__ __forceinline__
 
-// Dynamic shared memory of a launch: opted in at its exact size before every
-// launch.  The 48 KB a kernel gets without the opt-in counts its static
-// shared memory too, so a dynamic size just under 48 KB can still need it.
-inline cudaError_t smem_opt_in(const void* fn, size_t dyn_bytes) {
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_bytes);
-}
+// Dynamic shared memory of a launch, opted in before it.  The 48 KB a kernel gets
+// without the opt-in counts its static shared memory too, so a dynamic size just
+// under 48 KB can still need it.  The limit belongs to the kernel and the device, not
+// to the launch: it only ever rises, so that no thread lowers it between another
+// one's opt-in and launch (handle.cu).
+cudaError_t smem_opt_in(const void* fn, size_t dyn_bytes);
 
 // Status codes of the C ABI (mirrored in include/hodlr_b200.h).
 enum {

@@ -2,6 +2,22 @@
 // by the host orchestration units (handle.h).
 #include "handle.h"
 
+#include "common.cuh"
+
+cudaError_t smem_opt_in(const void* fn, size_t dyn_bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> granted;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  size_t& have = granted[{dev, fn}];
+  if (dyn_bytes <= have) return cudaSuccess;
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_bytes);
+  if (e == cudaSuccess) have = dyn_bytes;
+  return e;
+}
+
 namespace hodlr_impl {
 
 // Device memory of every handle on a device comes from one stream-ordered
