@@ -412,11 +412,10 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
   std::vector<GroupJob> jobs = group_jobs(h, set, rank_est);
   int ctas = h->num_sms, kcap_max = 1;
   for (int l : set) kcap_max = std::max(kcap_max, h->lv[l].kcap);
-  bool ring = h->aca_ring;
   for (;;) {  // a cooperative launch the driver refuses is retried with half the CTAs
     int variant = ACA_GROUP_NONE;
     const double t1 = share_ctas(jobs, ctas, ACA_GROUP_8x1);
-    if (ring && t1 >= 0) {
+    if (h->aca_ring && h->aca_ring_fits && t1 >= 0) {
       int rows = 1, elems = 0, ps = 0;
       size_t bytes = 0;
       variant = ACA_GROUP_8x4;
@@ -484,19 +483,13 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
     h->pool.scratch_busy = variant != ACA_GROUP_NONE;
     const int rc = run_aca(h, bl, 1, any ? 256 : 128, kcap_max, variant, &groups, yield_at);
     h->pool.scratch_busy = false;
-    if (rc == HODLR_ERR_ALLOC && variant) {  // no room beside the working layout
-      h->pool.free_scratch(h->stream);
-      ring = false;
-      continue;
-    }
     if (rc != HODLR_ERR_RETRY_SMALLER) return rc;
     if (ctas == 1) return fail(h, HODLR_ERR_CUDA, "aca_launch: cooperative launch refused");
     ctas = std::max(1, ctas / 2);
   }
 }
 
-int do_compress(hodlr_t h) {
-  if (h->compressed) return HODLR_OK;
+static int compress_levels(hodlr_t h) {
   free_compress(h);
   h->aca_launches = 0;
   h->aca_seconds = 0;
@@ -636,6 +629,26 @@ int do_compress(hodlr_t h) {
   h->aca_bytes = bytes;
   h->compressed = true;
   return HODLR_OK;
+}
+
+int do_compress(hodlr_t h) {
+  if (h->compressed) return HODLR_OK;
+  h->aca_ring_fits = true;
+  int rc = compress_levels(h);
+  if (rc == HODLR_ERR_ALLOC && h->aca_ring) {
+    // not with the group form's working layout, slots, published rows and dots:
+    // once more with the panels loaded per thread, which needs none of them
+    h->pool.free_scratch(h->stream);
+    dfree(h, h->slots);
+    dfree(h, h->pub);
+    dfree(h, h->dotg);
+    dfree(h, h->part);
+    h->slots_cap = 0;
+    h->pub_cap = h->dotg_cap = h->part_cap = 0;
+    h->aca_ring_fits = false;
+    rc = compress_levels(h);
+  }
+  return rc;
 }
 
 }  // namespace hodlr_impl

@@ -287,6 +287,7 @@ struct hodlr_handle_s {
   // group levels in aca_group_kernel (panels through the CTAs' rings); false:
   // aca_kernel (panels loaded per thread), the same bits
   bool aca_ring = true;
+  bool aca_ring_fits = true;  // in memory, as far as this compression knows
   // factorization form (hodlr_set_solver_form): false recLU's Schur systems
   // [bottom; top], true recSM's perturbI systems [top; bottom]
   bool sm_form = false;

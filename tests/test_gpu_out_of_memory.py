@@ -112,10 +112,16 @@ def test_streamed_compression_fits_where_per_thread_loads_do(hint):
         g.storeLRinTree()
         return g.ranks(), g.memory_held()
 
-    # what is held at the end, the cache included, is the most it ever was
-    ranks, low = compress(0, 0)
-    same, high = compress(2, 0)
-    assert np.array_equal(same, ranks)
+    ranks, most = compress(0, 0)
+    too_little, enough = most // 8, most  # what per-thread loads need, by bisection
+    while enough - too_little > 1 << 18:
+        limit = (too_little + enough) // 2
+        try:
+            assert np.array_equal(compress(0, limit)[0], ranks)
+            enough = limit
+        except HODLRError as e:
+            assert e.status == _lib.ERR_ALLOC
+            too_little = limit
     # exchange slots and published rows of the group form: below 4 MB
-    for limit in np.linspace(low + (4 << 20), max(high, low) + (8 << 20), 20).astype(int):
+    for limit in np.linspace(enough + (4 << 20), 2 * most, 40).astype(int):
         assert np.array_equal(compress(2, limit)[0], ranks)
