@@ -392,11 +392,9 @@ constexpr int PW = 32;
 struct PanelSmem {
   unsigned hi[2][SNT / 32], lo[2][SNT / 32];
   int pos[2][SNT / 32];
-  double inv[2][SNT / 32];
   double row[2][SNT / 32][PW];
   unsigned chi[2][8], clo[2][8];  // the cluster's candidates
   int cpos[2][8];
-  double cinv[2][8];
   double crow[2][8][PW];
 };
 
@@ -442,7 +440,6 @@ __device__ bool panel_in_registers(double* a, int n, int* piv, int j0, int nb, P
       const double v = fabs(x[c]);
       const unsigned hi = done ? 0u : (v == v ? (unsigned)__double2hiint(v) : 0u) | 0x80000000u;
       const unsigned lo = !done && v == v ? (unsigned)__double2loint(v) : 0u;
-      const double inv = 1.0 / x[c];
       const unsigned mh = __reduce_max_sync(all, hi);
       const unsigned ml = __reduce_max_sync(all, hi == mh ? lo : 0u);
       const bool cand = !done && hi == mh && lo == ml;
@@ -456,7 +453,6 @@ __device__ bool panel_in_registers(double* a, int n, int* piv, int j0, int nb, P
         sm.hi[buf][w] = mh;
         sm.lo[buf][w] = ml;
         sm.pos[buf][w] = pos;
-        sm.inv[buf][w] = inv;
 #pragma unroll
         for (int k = c & ~1; k < PW; k += 2)
           *reinterpret_cast<double2*>(&sm.row[buf][w][k]) = make_double2(x[k], x[k + 1]);
@@ -465,7 +461,6 @@ __device__ bool panel_in_registers(double* a, int n, int* piv, int j0, int nb, P
       int q;
       int b = best_slot(sm.hi[buf], sm.lo[buf], sm.pos[buf], SNT / 32, &q);
       const double* pr = sm.row[buf][b];
-      double di = sm.inv[buf][b];
       if (CL) {
         if (c == 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (w == 0)
@@ -476,13 +471,11 @@ __device__ bool panel_in_registers(double* a, int n, int* piv, int j0, int nb, P
               to->chi[buf][rank] = sm.hi[buf][b];
               to->clo[buf][rank] = sm.lo[buf][b];
               to->cpos[buf][rank] = q;
-              to->cinv[buf][rank] = di;
             }
           }
         cg::this_cluster().sync();
         b = best_slot(sm.chi[buf], sm.clo[buf], sm.cpos[buf], size, &q);
         pr = sm.crow[buf][b];
-        di = sm.cinv[buf][b];
       }
       if (r == 0) piv[j0 + c] = j0 + q;
       if (pos == q) {
@@ -495,13 +488,7 @@ __device__ bool panel_in_registers(double* a, int n, int* piv, int j0, int nb, P
       if (d == 0.0) {
         singular = true;
       } else if (!done) {
-        double l;
-        if (fabs(d) > 0x1p-1000 && fabs(d) < 0x1p1000) {  // x / d from 1 / d, one correction
-          l = x[c] * di;
-          l = fma(fma(-l, d, x[c]), di, l);
-        } else {
-          l = x[c] / d;
-        }
+        const double l = x[c] / d;
         x[c] = l;
 #pragma unroll
         for (int k = c + 1; k < PW; ++k) x[k] = fma(-l, pr[k], x[k]);
