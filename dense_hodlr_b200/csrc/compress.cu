@@ -414,22 +414,26 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
     int variant = ACA_GROUP_NONE;
     const double t1 = share_ctas(jobs, ctas, ACA_GROUP_8x1);
     if (h->aca_ring && h->aca_ring_fits && t1 >= 0) {
-      int rows = 1, elems = 0, ps = 0;
-      size_t bytes = 0;
-      variant = ACA_GROUP_8x4;
-      if (t1 <= share_ctas(jobs, ctas, variant)) {
-        variant = ACA_GROUP_8x1;
-        share_ctas(jobs, ctas, variant);
+      // the faster form, or the other one where only that has room for a ring
+      // beside the coefficients of so many columns; neither: per thread
+      const double t4 = share_ctas(jobs, ctas, ACA_GROUP_8x4);
+      const int first = t1 <= t4 ? ACA_GROUP_8x1 : ACA_GROUP_8x4;
+      for (int v : {first, ACA_GROUP_8x1 + ACA_GROUP_8x4 - first}) {
+        int rows = 1, elems = 0, ps = 0;
+        size_t bytes = 0;
+        share_ctas(jobs, ctas, v);
+        for (auto& j : jobs) rows = std::max(rows, (j.rows + j.G - 1) / j.G);
+        if (!aca_group_ring(v, rows, kcap_max, group_smem_budget(v), &elems, &bytes)) continue;
+        if (aca_group_max_coresident(v, bytes, &ps) || ps < 1)
+          return fail(h, HODLR_ERR_CUDA, "occupancy query failed");
+        variant = v;
+        break;
       }
-      for (auto& j : jobs) rows = std::max(rows, (j.rows + j.G - 1) / j.G);
-      if (!aca_group_ring(variant, rows, kcap_max, group_smem_budget(variant), &elems, &bytes))
-        variant = ACA_GROUP_NONE;  // too many columns beside a ring
-      else if (aca_group_max_coresident(variant, bytes, &ps) || ps < 1)
-        return fail(h, HODLR_ERR_CUDA, "occupancy query failed");
       // the slices' working layout, in the pool's scratch; without memory for it
       // the panels are loaded from the arenas per thread
       int64_t work = 0;
       for (auto& j : jobs) {
+        if (!variant) break;
         int r0, c0, m, n;
         block_geom(h->lv[j.level], j.q, r0, c0, m, n);
         const int kcap = h->lv[j.level].kcap;
