@@ -354,6 +354,10 @@ int init_common(hodlr_t h) {
   if (acs && acs[0] >= '0' && acs[0] <= '2' && acs[1] == 0) {
     h->aca_ring = acs[0] != '0';
   }
+  // HODLR_CAPACITANCE_SMEM=bytes: shared memory a CTA of a capacitance solve may
+  // use in new handles; systems beyond it run from device memory
+  const char* cap = getenv("HODLR_CAPACITANCE_SMEM");
+  if (cap && atoll(cap) > 0) h->cap_smem = (size_t)std::min<long long>(atoll(cap), CAP_SMEM);
   CK(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
   h->stream = h->own_stream;
   CK(cudaEventCreate(&h->ev0));

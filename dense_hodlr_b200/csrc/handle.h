@@ -338,6 +338,7 @@ struct hodlr_handle_s {
   int64_t spart_cap = 0;
   double* cap_big = nullptr;  // solve: capacitance systems beyond shared memory
   int64_t cap_big_cap = 0;
+  size_t cap_smem = CAP_SMEM;  // HODLR_CAPACITANCE_SMEM: less, so that small systems take that form
   double* part = nullptr;
   int64_t part_cap = 0;
   unsigned* bar = nullptr;

@@ -28,6 +28,8 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace {
@@ -36,7 +38,7 @@ namespace cg = cooperative_groups;
 
 constexpr int NB = TRI_NB;
 constexpr int SK_NT = 256;  // 8 warps
-constexpr int TRI_BUFS = 5;  // block buffers of tri_solve; the triangle behind them
+constexpr int TRI_BUFS = 4;  // block buffers of tri_solve; the triangle behind them
 
 __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -317,8 +319,8 @@ __device__ __noinline__ void substitute_block(const double* ts, int dir, int m,
 // row r of owned block q.  Step b: its owner forms D_b x_b, one 8-row tile a
 // warp, refines it where the triangle asks for that, and writes it to every CTA's
 // xb[b mod 3]; all subtract A(b', b) x_b from their blocks still to be solved.
-// xb[3], xb[4] and the triangle at `ts` are the refinement's: in shared memory, copied
-// a step ahead (from L2 or memory inside the chain a refined step took 4 us, not
+// xb[3] and the triangle at `ts` are the refinement's, and xb[b mod 3] before x_b is
+// there; the triangle is copied a step ahead (from L2 or memory inside the chain a refined step took 4 us, not
 // 2), and not in registers, which doubled (120 -> 255).
 //
 // The chain is wait, update of the next block, its product, write: the owner
@@ -394,15 +396,15 @@ __device__ void tri_solve(const double* __restrict__ a, int n, double* own, int 
     const double *yp[NT], *rp[NT];
 #pragma unroll
     for (int u = 0; u < NT; ++u) {
-      yp[u] = &xb[3][u][0][0];
-      rp[u] = &xb[4][u][0][0];
+      yp[u] = &xb[buf][u][0][0];
+      rp[u] = &xb[3][u][0][0];
     }
 #pragma unroll 1
     for (int it = 0; it < (mode == TRI_SUBST ? 0 : mode); ++it) {  // y += D (x - T y)
       double v[NT][2];
 #pragma unroll
       for (int u = 0; u < NT; ++u)
-        *reinterpret_cast<double2*>(&xb[3][u][0][0] + at) = make_double2(y[u][0], y[u][1]);
+        *reinterpret_cast<double2*>(&xb[buf][u][0][0] + at) = make_double2(y[u][0], y[u][1]);
       __syncthreads();
       double tv[NB / 4];
       load_tri(dir, m, [&](int c, int r) { return ts[c * TRI_PITCH + r]; }, tv);
@@ -410,7 +412,7 @@ __device__ void tri_solve(const double* __restrict__ a, int n, double* own, int 
 #pragma unroll
       for (int u = 0; u < NT; ++u) {
         const double2 r = *reinterpret_cast<const double2*>(x[u] + at);
-        *reinterpret_cast<double2*>(&xb[4][u][0][0] + at) =
+        *reinterpret_cast<double2*>(&xb[3][u][0][0] + at) =
             make_double2(r.x - v[u][0], r.y - v[u][1]);
       }
       __syncthreads();
@@ -534,7 +536,7 @@ __global__ void __launch_bounds__(SK_NT, 2) leaf_apply_kernel(LeafSolveLaunch L)
 // column tile); grid.x = node * size + rank.
 template <int NT, bool PARTS, bool CL>
 __global__ void __launch_bounds__(SK_NT, 2) cap_solve_kernel(CapLaunch L, int nrhs, int own_max,
-                                                          unsigned* err) {
+                                                          int ncp, unsigned* err) {
   extern __shared__ __align__(16) double dyn[];
   int rank = 0, size = 1;
   if (CL) {
@@ -561,8 +563,8 @@ __global__ void __launch_bounds__(SK_NT, 2) cap_solve_kernel(CapLaunch L, int nr
       } else if (PARTS) {
         const bool h = !(q >= N.off[0] && q < N.off[0] + N.m[0]);
         const double* p = L.part + (h ? N.part[1] : N.part[0]) +
-                          (int64_t)(q - (h ? N.off[1] : N.off[0])) * NCP + c;
-        const int64_t st = (int64_t)(h ? N.m[1] : N.m[0]) * NCP;
+                          (int64_t)(q - (h ? N.off[1] : N.off[0])) * ncp + c0 + c;
+        const int64_t st = (int64_t)(h ? N.m[1] : N.m[0]) * ncp;
         const int count = h ? N.chunks[1] : N.chunks[0];
         constexpr int U = 16;  // loads in flight, added in order
         for (int k = 0; k < count; k += U) {
@@ -591,7 +593,7 @@ __global__ void __launch_bounds__(SK_NT, 2) cap_solve_kernel(CapLaunch L, int nr
     if (i >= n) continue;
     const double v = own[((int64_t)(c >> 3) * own_max * NB + lr) * 8 + (c & 7)];
     if (PARTS)
-      L.z[N.z + (int64_t)i * NCP + c] = v;
+      L.z[N.z + (int64_t)i * ncp + c0 + c] = v;
     else if (c0 + c < nrhs)
       L.z[N.z + (int64_t)(c0 + c) * n + i] = v;
   }
@@ -780,31 +782,39 @@ __global__ void __launch_bounds__(SK_NT) skinny_nn_kernel(const NnItem* __restri
     if (e__ != cudaSuccess) return (int)e__;  \
   } while (0)
 
-constexpr size_t kCapSmem = 200 * 1024;
 // Shared memory of tri_solve beside the owned rows.
 constexpr size_t tri_smem(int nt) {
   return sizeof(double) * (size_t)(TRI_BUFS * nt * NB * 8 + NB * TRI_PITCH);
+}
+// ... and with them, of the largest of the CTAs that share nb block rows.
+size_t cap_smem(int nt, int nb, int ctas) {
+  return sizeof(double) * 8 * NB * nt * (size_t)((nb + ctas - 1) / ctas) + tri_smem(nt);
+}
+// Column tiles a CTA takes: both of 9 to 16 columns where a cluster holds them
+// (7000 rows), else one (22528 rows; beyond, L.big).
+int cap_tiles(int nrhs, int max_sd, size_t limit) {
+  const int nt = skinny_tiles(nrhs);
+  return nt == 2 && cap_smem(2, (max_sd + NB - 1) / NB, 8) > limit ? 1 : nt;
 }
 
 template <int NT, bool PARTS>
 int cap_launch(const CapLaunch& L, int nnodes, int nrhs, int max_sd, unsigned* err,
                cudaStream_t s) {
   const int nb = (max_sd + NB - 1) / NB;
-  auto smem_of = [&](int c) {
-    return sizeof(double) * 8 * NB * NT * (size_t)((nb + c - 1) / c) + tri_smem(NT);
-  };
   // CTAs of a cluster: at least two block rows each, and as few nodes as leave
   // SMs over; more where the rows would not fit
   int size = 1;
-  while (size < 8 && (smem_of(size) > kCapSmem || (nb >= 4 * size && nnodes * size < 148))) size *= 2;
+  while (size < 8 && (cap_smem(NT, nb, size) > std::min<size_t>(200 * 1024, L.smem_limit) ||
+                      (nb >= 4 * size && nnodes * size < 148)))
+    size *= 2;
   if (L.big) size = 1;
-  const size_t smem = L.big ? tri_smem(NT) : smem_of(size);
-  if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
+  const size_t smem = L.big ? tri_smem(NT) : cap_smem(NT, nb, size);
+  if (smem > CAP_SMEM) return (int)cudaErrorInvalidValue;
   const dim3 grid(nnodes * size, (nrhs + 8 * NT - 1) / (8 * NT));
-  const int own = (nb + size - 1) / size;
+  const int own = (nb + size - 1) / size, ncp = 8 * skinny_tiles(nrhs);
   if (size == 1) {
     LCK(smem_opt_in((const void*)cap_solve_kernel<NT, PARTS, false>, smem));
-    cap_solve_kernel<NT, PARTS, false><<<grid, SK_NT, smem, s>>>(L, nrhs, own, err);
+    cap_solve_kernel<NT, PARTS, false><<<grid, SK_NT, smem, s>>>(L, nrhs, own, ncp, err);
     return (int)cudaGetLastError();
   }
   LCK(smem_opt_in((const void*)cap_solve_kernel<NT, PARTS, true>, smem));
@@ -820,14 +830,14 @@ int cap_launch(const CapLaunch& L, int nnodes, int nrhs, int max_sd, unsigned* e
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, cap_solve_kernel<NT, PARTS, true>, L, nrhs, own, err);
+  return (int)cudaLaunchKernelEx(&cfg, cap_solve_kernel<NT, PARTS, true>, L, nrhs, own, ncp, err);
 }
 
 }  // namespace
 
-int64_t cap_big_elems(int nnodes, int nrhs, int max_sd) {
-  const int nt = skinny_tiles(nrhs), nb = (max_sd + NB - 1) / NB;
-  if (sizeof(double) * 8 * NB * nt * (size_t)((nb + 7) / 8) + tri_smem(nt) <= kCapSmem) return 0;
+int64_t cap_big_elems(int nnodes, int nrhs, int max_sd, size_t limit) {
+  const int nt = cap_tiles(nrhs, max_sd, limit), nb = (max_sd + NB - 1) / NB;
+  if (cap_smem(nt, nb, 8) <= limit) return 0;
   return (int64_t)nnodes * ((nrhs + 8 * nt - 1) / (8 * nt)) * nt * nb * NB * 8;
 }
 
@@ -887,7 +897,7 @@ int skinny_nn_launch(const NnItem* items, int count, double* X, int64_t ldx, int
 int cap_solve_launch(const CapLaunch& L, int nnodes, int nrhs, int max_sd, bool parts,
                      unsigned* err, cudaStream_t s) {
   if (nnodes == 0 || nrhs <= 0) return 0;
-  if (skinny_tiles(nrhs) == 1)
+  if (cap_tiles(nrhs, max_sd, L.smem_limit) == 1)
     return parts ? cap_launch<1, true>(L, nnodes, nrhs, max_sd, err, s)
                  : cap_launch<1, false>(L, nnodes, nrhs, max_sd, err, s);
   return parts ? cap_launch<2, true>(L, nnodes, nrhs, max_sd, err, s)

@@ -47,6 +47,10 @@ struct CapNode {
   int64_t z;  // row-major result / column-major right-hand sides and result
 };
 
+// Most shared memory of a CTA: rows that a cluster of 8 cannot hold in so much of
+// it are kept in device memory.
+constexpr size_t CAP_SMEM = 227 * 1024;
+
 struct CapLaunch {
   const CapNode* nodes = nullptr;
   const double* S = nullptr;
@@ -54,6 +58,7 @@ struct CapLaunch {
   const double* part = nullptr;
   double* z = nullptr;
   double* big = nullptr;  // cap_big_elems doubles, or null when that is 0
+  size_t smem_limit = CAP_SMEM;
 };
 
 // Column tiles of 8 a launch carries per CTA: 1 or 2.
@@ -61,7 +66,7 @@ inline int skinny_tiles(int nrhs) { return nrhs <= 8 ? 1 : 2; }
 
 // Memory a launch needs for systems whose rows do not fit the shared memory of
 // a cluster (doubles; 0: they fit).
-int64_t cap_big_elems(int nnodes, int nrhs, int max_sd);
+int64_t cap_big_elems(int nnodes, int nrhs, int max_sd, size_t limit);
 
 // The inverses of the triangles of every TRI_NB diagonal block of the packed LUs
 // (n x n at off, column-major, tri_elems(n) doubles behind each).

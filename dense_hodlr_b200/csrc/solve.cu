@@ -86,7 +86,7 @@ int build_solve_plans(hodlr_t h, int nrhs) {
     for (auto& sn : L.nodes)
       t += (int64_t)(sn.kb + sn.kt) * (few ? 8 * skinny_tiles(nrhs) : nrhs);
     zs_tot = std::max(zs_tot, t);
-    big = std::max(big, cap_big_elems((int)L.nodes.size(), nrhs, L.max_sd));
+    big = std::max(big, cap_big_elems((int)L.nodes.size(), nrhs, L.max_sd, h->cap_smem));
   }
   if (zs_tot > h->zs_cap) {
     for (auto& L : h->lv) L.solve_nrhs = -1;  // the GEMM plans point into it
@@ -234,7 +234,8 @@ int solve_in_place(hodlr_t h, int nrhs) {
     CL.perm = L.perm;
     CL.part = h->spart;
     CL.z = h->zs;
-    CL.big = cap_big_elems(nn, nrhs, L.max_sd) ? h->cap_big : nullptr;
+    CL.big = cap_big_elems(nn, nrhs, L.max_sd, h->cap_smem) ? h->cap_big : nullptr;
+    CL.smem_limit = h->cap_smem;
     e = cap_solve_launch(CL, nn, nrhs, L.max_sd, few, h->d_err, h->stream);
     if (e) return cuda_fail(h, (cudaError_t)e, "solve capacitance");
     h->nlaunch += 1;
