@@ -77,6 +77,31 @@ static int build_few(hodlr_t h, Level& L, int nrhs, int64_t* z, int64_t* part) {
   return HODLR_OK;
 }
 
+// Checked mode: what a level's V^T X and X updates read and write, as check_gemm
+// verifies the plans of the grouped GEMMs.  Rows are read in aligned pairs.
+static int check_few(hodlr_t h, const Level& L) {
+  if (!h->checked) return HODLR_OK;
+  const size_t e = sizeof(double);
+  const int64_t ldp = h->ldp();
+  int rc = check_extent(h, L.d_stn, sizeof(TnItem) * L.nstn, "V^T X items", "solve");
+  if (!rc) rc = check_extent(h, L.d_snn, sizeof(NnItem) * L.nsnn, "X update items", "solve");
+  if (!rc) rc = check_extent(h, L.d_caps, sizeof(CapNode) * L.nodes.size(), "capacitance nodes", "solve");
+  if (!rc) rc = check_extent(h, h->spart, e * L.spart_need, "V^T X sums", "solve");
+  for (size_t p = 0; p < L.nodes.size() && !rc; ++p) {
+    const SchurNode& sn = L.nodes[p];
+    const int lo[2] = {L.nmin[p], L.nsplit[p] + 1}, hi[2] = {L.nsplit[p] + 1, L.nmax[p] + 1};
+    const int m[2] = {sn.kb, sn.kt}, k[2] = {sn.kt, sn.kb};
+    for (int q = 0; q < 2 && !rc; ++q) {
+      const int64_t first = lo[q] & ~1, rows = ((hi[q] + 1) & ~1) - first;
+      if (m[q] > 0)
+        rc = check_extent(h, L.V + first, e * ((m[q] - 1) * ldp + rows), "V panel", "solve");
+      if (!rc && k[q] > 0)
+        rc = check_extent(h, L.Yl + first, e * ((k[q] - 1) * ldp + rows), "K^-1 U panel", "solve");
+    }
+  }
+  return rc;
+}
+
 int build_solve_plans(hodlr_t h, int nrhs) {
   const int64_t N = h->n, ldp = h->ldp();
   const bool few = few_rhs(h, nrhs);
@@ -211,6 +236,8 @@ int solve_in_place(hodlr_t h, int nrhs) {
   for (int l = (int)h->lv.size() - 1; l >= 0; --l) {
     Level& L = h->lv[l];
     const int nn = (int)L.nmin.size();
+    if (few) rc = check_few(h, L);
+    if (rc) return rc;
     if (few) {
       e = skinny_tn_launch(L.d_stn, L.nstn, h->X, N, nrhs, h->ldp(), h->spart, h->stream);
       h->nlaunch += 1;
