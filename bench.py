@@ -67,20 +67,6 @@ def peaks():
     return 6650.0, "fallback"
 
 
-def profiled_figure(name, key):
-    """A figure from a committed ncu summary under profiles/ (a 'key: value' line)."""
-    p = os.path.join(ROOT, "profiles", name)
-    if not os.path.exists(p):
-        return None
-    for line in open(p):
-        if line.strip().startswith(key + ":"):
-            try:
-                return float(line.split(":", 1)[1].strip().split()[0])
-            except (ValueError, IndexError):
-                return None
-    return None
-
-
 # FP64 FLOPs of the symmetric full-kernel product (kmatvec.cu / kfast.cuh),
 # FMA counted as 2, as the kernel executes them: one Matern-3/2 entry in 2D is
 # the distance (2 sub + 2 fma from the floor), the square root from the
@@ -92,12 +78,6 @@ def profiled_figure(name, key):
 KMV_EVAL_FLOPS = 27
 
 
-def sym_slices(n):
-    """Workspace slices of the symmetric product (kmatvec.cu: 256-point tiles,
-    about 96 splits)."""
-    nt = -(-n // 256)
-    tps = 1 if nt <= 96 else -(-nt // 96)
-    return -(-nt // tps)
 FP64_LANES_PER_SM = 64
 
 
@@ -380,7 +360,6 @@ def run_ours(args, rank, world, local_rank):
     evaluated = N_PTS * (N_PTS + 256) / 2.0
     kmv_flops = evaluated * (KMV_EVAL_FLOPS + 4 * NRHS)
     kmv_tf = kmv_flops / t_kmatvec / 1e12
-    kmv_dram_ref = profiled_figure("kmatvec_sym_mma_matern2d_n65536.md", "dram_bytes_per_launch")
     out = {
         "metric": METRIC,
         "value": job_rate(ms_max, world),
@@ -419,10 +398,9 @@ def run_ours(args, rank, world, local_rank):
                                    f"{sm_mhz:.0f} MHz), shared by FP64 FMAs and FP64 MMAs; "
                                    "no measured FP64 figure exists"),
                      "unit": "TFLOP/s", "frac": kmv_tf / fp64_peak,
-                     "traffic": (kmv_dram_ref * (N_PTS * sym_slices(N_PTS))
-                                 / (65536.0 * sym_slices(65536)) if kmv_dram_ref else None),
-                     "traffic_note": ("DRAM bytes of the n=65536 capture scaled by slices x n "
-                                      "(the workspace writes); the kernel is compute-bound"),
+                     "traffic": None,
+                     "traffic_note": ("DRAM bytes of the current kernel not captured; it is bound "
+                                      "by instruction issue"),
                      "algorithmic_flops_per_launch": kmv_flops,
                      "avg_launch_s": t_kmatvec},
         "roofline_aca": {"kernel": "aca_group_kernel and aca_kernel (batched partial-pivot ACA; "

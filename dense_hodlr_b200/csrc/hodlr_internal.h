@@ -84,7 +84,7 @@ struct AcaLaunch {
   unsigned spin_limit;   // polls of a group barrier before it gives up (DEV_ERR_TIMEOUT)
   unsigned bar_extra;    // arrivals a group barrier waits for beyond its G CTAs (0; 1 makes
                          // every barrier unreachable, to exercise the timeout path)
-  // aca_group_kernel: ring stages, doubles of a stage (GR_TC columns of the
+  // aca_group_kernel: ring stages, doubles of a stage (a tile's columns of the
   // largest chunk), and the exchange slots (128 bytes a CTA, zeroed before launch)
   int ring_stages, stage_elems;
   unsigned char* slots;

@@ -651,10 +651,11 @@ __global__ void __launch_bounds__(SNT) schur_lu_kernel(SchurLaunch L, int big_sd
 
 // ------------------------------------------- multi-CTA LU of large nodes
 // Right-looking, outer panels of BNB columns.  Per panel j0, for every large
-// node (its index in BigNodes): (1) one CTA factors the panel columns
-// [j0, j0+BNB) with lu_columns; (2) many CTAs apply the panel's interchanges
-// to every other column and form U12 = L11^-1 A12 right of the panel; (3)
-// A22 -= L21 U12 in 64 x 64 tiles over all SMs.  The pivot choices are the
+// node (its index in BigNodes): (1) the panel columns [j0, j0+BNB), in the
+// registers of one CTA or of a cluster of up to 8 (512 rows each), above 4096 rows
+// by one CTA through shared memory (lu_columns); (2) many CTAs apply the panel's
+// interchanges to every other column and form U12 = L11^-1 A12 right of the panel;
+// (3) A22 -= L21 U12 in 64 x 64 tiles over all SMs.  The pivot choices are the
 // column-wise first maxima, as in the one-CTA kernel.
 constexpr int BNB = PW;
 constexpr int BIG_MAX = 1024;  // nodes per launch (kernel parameter: 4 KB)

@@ -534,8 +534,11 @@ __global__ void __launch_bounds__(SK_NT, 2) leaf_apply_kernel(LeafSolveLaunch L)
 // PARTS: r row-summed from the V^T X chunks, y row-major; otherwise r and y
 // column-major (n x nrhs at the node's z).  Cluster `size` CTAs per (node,
 // column tile); grid.x = node * size + rank.
+// Two CTAs an SM for one column tile (128 registers; N = 262144, 8 columns 2.24 ms
+// against 2.38 unbounded); two tiles spill inside the chain then (40000-point cube, 16
+// columns, the capacitance solves of 5 passes 6.3 ms against 3.9).
 template <int NT, bool PARTS, bool CL>
-__global__ void __launch_bounds__(SK_NT, 2) cap_solve_kernel(CapLaunch L, int nrhs, int own_max,
+__global__ void __launch_bounds__(SK_NT, NT == 1 ? 2 : 1) cap_solve_kernel(CapLaunch L, int nrhs, int own_max,
                                                           int ncp, unsigned* err) {
   extern __shared__ __align__(16) double dyn[];
   int rank = 0, size = 1;

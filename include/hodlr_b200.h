@@ -356,10 +356,10 @@ int hodlr_get_memory_held(hodlr_t h, long long* bytes);
 
 /* How the ACA of the few-block top levels reads its W/V panel slices (no
  * counterpart in the reference): on = 2 (default) or 1 streams them through
- * a shared-memory ring per CTA, one bulk copy per panel column of a tile; 0
- * loads the panels per thread.  Measured ACA time, streamed / per thread:
- * 0.015 / 0.090 s (2D Matern cloud, N = 20011, tol 1e-8), 0.133 / 0.260 s
- * (N = 262144).  Pivots, ranks and W/V are the same in every mode; the
+ * a shared-memory ring per CTA, one bulk copy per tile; 0 loads the panels per
+ * thread, and so does a compression that does not fit beside the rings' buffers.
+ * Measured ACA time, streamed / per thread: 0.015 / 0.090 s (2D Matern cloud,
+ * N = 20011, tol 1e-8), 0.117 / 0.260 s (N = 262144).  Pivots, ranks and W/V are the same in every mode; the
  * setting applies from the next compression.  HODLR_ACA_STREAMING=0, 1 or 2
  * in the environment sets the mode of every new handle. */
 int hodlr_set_aca_streaming(hodlr_t h, int on);
