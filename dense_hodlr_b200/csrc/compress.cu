@@ -479,15 +479,12 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
     // would depend on the clock.  ACA in ms of 2D N = 262144, sphere 16384, cube
     // 40000: fixed shares 131, 107.8, 92.7; pauses at 0.8 of that rank 114.6, 109.1,
     // 94.1; at the rank 117.1, 108.7, 88.6; with a third of the CTAs idle 111.0, 107.3,
-    // 87.8 and other last bits of epsilon every time.  In a forest a level's expected
-    // rank is its largest system's, so a first pause at a fifth of it lets the
-    // systems of low rank go (40 systems: 57.1 -> 53.8 ms, 54.1 by the clock).
+    // 87.8 and other last bits of epsilon every time.
     double slowest = 0.0;
     for (auto& j : jobs) slowest = std::max(slowest, j.t);
     if (variant && jobs.size() > 1 && slowest > 2000.0)
       for (size_t i = 0; i < jobs.size(); ++i)
-        bl[i].kstop = (int)std::max(jobs[i].k0 + 24.0,
-                                    h->nsys && jobs[i].k0 == 0.0 ? 0.2 * jobs[i].k : jobs[i].k);
+        bl[i].kstop = (int)std::max(jobs[i].k0 + 24.0, jobs[i].k);
     h->pool.scratch_busy = variant != ACA_GROUP_NONE;
     const int rc = run_aca(h, bl, 1, any ? 256 : 128, kcap_max, variant, &groups);
     h->pool.scratch_busy = false;
