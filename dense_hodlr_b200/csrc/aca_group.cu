@@ -48,7 +48,7 @@
 // barrier, a sum of all CTAs' dots in every CTA, and one launch a level:
 // N = 20011 2D Matern-3/2 tol 1e-8 15 ms (90), sphere N = 16384 tol 1e-10 113
 // ms (796), 3D Gaussian N = 40000 89 ms (288), 1D N = 4096 0.3 ms (1.7),
-// 2D N = 262144 117 ms (142).
+// 2D N = 262144 111 ms (142).
 #include "aca_post.cuh"
 #include "common.cuh"
 #include "hodlr_internal.h"
@@ -84,7 +84,7 @@ struct GroupShared {
   double lag[4];         // the reduce warps' shares of the lagging norm update
   // the group's result of an exchange
   double mv;
-  int mi, mflag, mcand, fail, imin, stop;
+  int mi, mflag, mcand, fail, imin, stop, yield;
   // the stopping test, kept by thread 0: squared norms of column k-1 (its
   // epsilon pending) and of column k-2 (its epsilon lagging), and of the row
   // residual of this step
@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
     sh.swl = sh.svl = sh.svt = 0.0;
     sh.near = st->near;
     sh.stop = !(st->eps > L.tol) && st->k >= B.minRank;
-    sh.fail = 0;
+    sh.fail = sh.yield = 0;
   }
   __syncthreads();
   if (E == 1)
@@ -723,6 +723,8 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
   // to the tolerance is not noted yet; the product of the lagging norms
   int settled = 0;
   double rl = 0.0;
+  bool idle = false;
+  const int iters0 = st->iters;
   const int maxR = B.maxRank;  // -1: none (src/lowRank.cpp:149,244-247)
   if (status == ACA_RUNNING && k == 0 && maxR == 0) status = ACA_POST;
   auto bank = [&](int kc) { return (int64_t)(kc & 1) * 2 * L.kcap_max; };
@@ -739,7 +741,7 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
     if (op == OP_TOP) {  // a new step
       if (k == 1) pending = 0;  // settled with the column itself: no earlier columns
       if (!pending && !lag && sh.stop) { status = ACA_POST; break; }
-      if (k >= ub || k >= min(B.kcap, B.kstop)) {
+      if (k >= ub || k >= B.kcap || sh.yield) {
         if (lag) {
           op = OP_FENCE;
           next = OP_LAG;
@@ -851,7 +853,13 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
           if (gap < 1e-10) ++sh.near;
         }
         settled = 0;
-        if (op == OP_ROW) rl = sqrt(sh.swl) * sqrt(sh.svl);
+        if (op == OP_ROW) {
+          rl = sqrt(sh.swl) * sqrt(sh.svl);
+          // enough of the launch's CTAs have run out of work: let the host
+          // share them among the blocks that still run
+          idle = g == 0 && L.yield_at > 0 && iters - iters0 >= 24 &&
+                 *(volatile unsigned*)L.idle >= (unsigned)L.yield_at;
+        }
       }
       if (E > 1 && add_n > 0) {  // the last pass's dots, chunks and warps in order
         const double* dw = L.dotg + (int64_t)blockIdx.x * L.dotg_stride +
@@ -888,6 +896,7 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
     {
       double bv = -1.0, sq = 0.0, dot = 0.0;
       int bi = INT_MAX, cand = INT_MAX;
+      unsigned yield = 0;
       if (pass && lane < C::SW) {
         bv = sh.red_v[lane];
         bi = sh.red_i[lane];
@@ -900,12 +909,13 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
         cand = __reduce_min_sync(0xffffffffu, cand);
         sq = warp_sum_all(sq);
         for (int r = 0; r < C::RW; ++r) dot += sh.lag[r];
+        yield = __shfl_sync(0xffffffffu, (unsigned)idle, 0);
         if (G > 1) {
           if (!pass) fence_gpu();
           unsigned char* slots = L.slots + (size_t)B.g0 * 128 + (gen & 1) * 64;
           if (lane < 3) {
             const double v = lane == 0 ? bv : lane == 1 ? sq : dot;
-            const uint32_t x = lane == 0 ? (uint32_t)bi : (uint32_t)cand;  // the third has none
+            const uint32_t x = lane == 0 ? (uint32_t)bi : lane == 1 ? (uint32_t)cand : yield;
             st_b128(slots + (size_t)g * 128 + 16 * lane, (uint64_t)__double_as_longlong(v),
                     (uint64_t)x | ((uint64_t)gen << 32));
           }
@@ -933,6 +943,7 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
             cand = min(cand, (int)(uint32_t)b1);
             sq += __longlong_as_double((long long)b0);
             dot += __longlong_as_double((long long)e0);
+            yield |= (unsigned)e1;
           }
           if (!pass) fence_gpu();
           warp_argmax_all(bv, bi);
@@ -940,6 +951,7 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
           sq = warp_sum_all(sq);
           dot = warp_sum_all(dot);
           fail = __any_sync(0xffffffffu, fail);
+          yield = __reduce_or_sync(0xffffffffu, yield);
         } else if (L.bar_extra) {  // a group of one waits for nobody, unless it is told to
           fail = true;
         }
@@ -952,7 +964,10 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
             sh.mflag = bi == INT_MAX ? 0 : bi & 1;
             sh.mcand = cand;
           }
-          if (row) sh.svt = sq;
+          if (row) {
+            sh.svt = sq;
+            sh.yield = (int)yield;
+          }
           // epsilon after kce columns (src/lowRank.cpp:234-241), from the norms
           // of the lagging or the pending column and the dots just summed
           int kce = kc;
@@ -1150,6 +1165,7 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
     if (sh.fail) status = ACA_ERROR;
   }
   __syncthreads();
+  if (tid == 0 && L.yield_at > 0) atomicAdd(L.idle, 1u);
   if (g == 0 && tid == 0) {
     st->k = k;
     st->cur = cur;

@@ -47,7 +47,6 @@ void fill_block(hodlr_t h, Level& L, int q, AcaBlock& B) {
   B.g0 = 0;
   B.G = 1;
   const int p = q >> 1;
-  B.kstop = INT_MAX;
   B.sW = B.sV = nullptr;
   B.strW = B.strV = 0;
   B.minRank = (q & 1) ? L.bmin[p] : L.tmin[p];
@@ -67,8 +66,9 @@ size_t group_smem_budget(int v) { return v == ACA_GROUP_8x1 ? 212 * 1024 : 224 *
 // One ACA launch over `blocks`: groups of G CTAs each, or, with `groups`,
 // groups[i] CTAs for block i (a CTA table maps CTAs to blocks).  variant:
 // ACA_GROUP_NONE for aca_kernel with nt threads, else of aca_group_kernel.
+// yield_at: with so many CTAs out of work the others' blocks pause (0: never).
 int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_max, int variant,
-            const std::vector<int>* groups) {
+            const std::vector<int>* groups, int yield_at) {
   const int nb = (int)blocks.size();
   if (nb == 0) return HODLR_OK;
   int ncta = nb * G;
@@ -125,9 +125,11 @@ int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_ma
     L.ring_stages = aca_group_ring(variant, rows, kcap_max, group_smem_budget(variant), &L.stage_elems,
                                    &smem);
     if (!L.ring_stages) return fail(h, HODLR_ERR_STATE, "ACA ring does not fit");
-    CK(dgrow(h, h->slots, h->slots_cap, (int64_t)ncta * 128));
+    CK(dgrow(h, h->slots, h->slots_cap, (int64_t)ncta * 128 + 128));
     L.slots = h->slots;
-    CK(cudaMemsetAsync(h->slots, 0, (size_t)ncta * 128, h->stream));
+    CK(cudaMemsetAsync(h->slots, 0, (size_t)ncta * 128 + 128, h->stream));
+    L.idle = reinterpret_cast<unsigned*>(h->slots + (size_t)ncta * 128);
+    L.yield_at = yield_at;
     L.pub_stride = 16 * ((int64_t)kcap_max + 1);
     const int64_t pneed = 2 * L.pub_stride * ncta;
     if (pneed > h->pub_cap) {
@@ -472,21 +474,18 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
       L.G = jobs[i].G;
       any |= jobs[i].G > 1;
     }
-    // ranks differ from block to block: where a launch takes far longer than its
-    // overhead, a block pauses at the rank that was expected of it, and the CTAs are
-    // shared anew among those that go on.  At a column count, not when CTAs run out
-    // of work: the sums of the stopping test depend on a block's groups, so they
-    // would depend on the clock.  ACA in ms of 2D N = 262144, sphere 16384, cube
-    // 40000: fixed shares 131, 107.8, 92.7; pauses at 0.8 of that rank 114.6, 109.1,
-    // 94.1; at the rank 117.1, 108.7, 88.6; with a third of the CTAs idle 111.0, 107.3,
-    // 87.8 and other last bits of epsilon every time.
+    int most = 0;
     double slowest = 0.0;
-    for (auto& j : jobs) slowest = std::max(slowest, j.t);
-    if (variant && jobs.size() > 1 && slowest > 2000.0)
-      for (size_t i = 0; i < jobs.size(); ++i)
-        bl[i].kstop = (int)std::max(jobs[i].k0 + 24.0, jobs[i].k);
+    for (auto& j : jobs) {
+      most += j.G;
+      slowest = std::max(slowest, j.t);
+    }
+    // ranks differ from block to block: share the CTAs anew when a third of
+    // them are out of work, where a launch takes far longer than its overhead
+    // (2D N = 262144: 107 ms against 133 with fixed shares)
+    const int yield_at = jobs.size() > 1 && slowest > 2000.0 ? std::max(1, most / 3) : 0;
     h->pool.scratch_busy = variant != ACA_GROUP_NONE;
-    const int rc = run_aca(h, bl, 1, any ? 256 : 128, kcap_max, variant, &groups);
+    const int rc = run_aca(h, bl, 1, any ? 256 : 128, kcap_max, variant, &groups, yield_at);
     h->pool.scratch_busy = false;
     if (rc != HODLR_ERR_RETRY_SMALLER) return rc;
     if (ctas == 1) return fail(h, HODLR_ERR_CUDA, "aca_launch: cooperative launch refused");
@@ -567,7 +566,7 @@ static int compress_levels(hodlr_t h) {
     if (all) break;
   }
   // 2. the few-block levels, in sets of neighbouring levels, deepest first:
-  // the blocks of a set run in one launch (group_set_top)
+  // the blocks of a set run in one launch (group_sets)
   std::vector<double> rank_est((size_t)nlev, 0.0);
   double growth = 1.0;  // of the rank from one level to the next above it
   int known = -1;       // the uppermost level compressed so far

@@ -438,7 +438,7 @@ int grow_level(hodlr_t h, Level& L, int cap);
 void fill_block(hodlr_t h, Level& L, int q, AcaBlock& B);
 bool level_done(const Level& L);
 int run_aca(hodlr_t h, std::vector<AcaBlock>& blocks, int G, int nt, int kcap_max, int variant = 0,
-            const std::vector<int>* groups = nullptr);
+            const std::vector<int>* groups = nullptr, int yield_at = 0);
 int init_level(hodlr_t h, Level& L, int cap);
 int sync_level(hodlr_t h, Level& L, bool* done);
 int level_kmax(const Level& L);

@@ -45,7 +45,6 @@ struct AcaBlock {
   int* pcol;          // pivot column of step t
   int r0, c0, m, n;
   int kcap;           // columns available in W and V
-  int kstop;          // aca_group_kernel: columns at which the block pauses
   int level;
   int g0, G;          // with a CTA table: first CTA of this block's group, group size
   // aca_group_kernel: the block's slices of W and V in the launch's working
@@ -93,4 +92,8 @@ struct AcaLaunch {
   unsigned char* pub;
   int64_t pub_stride;
   unsigned launch_tag;
+  // CTAs of the launch that ran out of work so far (zeroed before launch); once
+  // there are yield_at (0: never) the blocks still running pause
+  unsigned* idle;
+  int yield_at;
 };
