@@ -42,6 +42,13 @@
 //   pass's exchange: epsilon of a step is known one step later, and the work
 //   begun meanwhile is discarded if the loop had ended (the same ranks,
 //   pivots and iteration counts).
+// * Pauses.  Blocks of a long launch pause so that the host shares the CTAs anew:
+//   once a third of them are out of work, which depends on the clock, or (AcaBlock::
+//   kstop) at a column count.  A block goes on in a group of another size, which adds
+//   the norms and dots up in another order: with pauses by the clock the last bits of
+//   epsilon differ from run to run, and a rank can where epsilon is within rounding
+//   of the tolerance (counted: AcaState::near).  W, V and the pivots up to there are
+//   the same bits whatever the groups.
 //
 // Measured on B200, all group levels of one compression, against per-warp
 // rings of 128-row tiles (panels loaded per thread for an odd N), a counter
@@ -741,7 +748,7 @@ __global__ void __launch_bounds__(GroupCfg<SW, E>::NT, 1)
     if (op == OP_TOP) {  // a new step
       if (k == 1) pending = 0;  // settled with the column itself: no earlier columns
       if (!pending && !lag && sh.stop) { status = ACA_POST; break; }
-      if (k >= ub || k >= B.kcap || sh.yield) {
+      if (k >= ub || k >= min(B.kcap, B.kstop) || sh.yield) {
         if (lag) {
           op = OP_FENCE;
           next = OP_LAG;

@@ -47,6 +47,7 @@ void fill_block(hodlr_t h, Level& L, int q, AcaBlock& B) {
   B.g0 = 0;
   B.G = 1;
   const int p = q >> 1;
+  B.kstop = INT_MAX;
   B.sW = B.sV = nullptr;
   B.strW = B.strV = 0;
   B.minRank = (q & 1) ? L.bmin[p] : L.tmin[p];
@@ -480,10 +481,20 @@ int run_group_set(hodlr_t h, const std::vector<int>& set, const std::vector<doub
       most += j.G;
       slowest = std::max(slowest, j.t);
     }
-    // ranks differ from block to block: share the CTAs anew when a third of
-    // them are out of work, where a launch takes far longer than its overhead
-    // (2D N = 262144: 107 ms against 133 with fixed shares)
-    const int yield_at = jobs.size() > 1 && slowest > 2000.0 ? std::max(1, most / 3) : 0;
+    // ranks differ from block to block: share the CTAs anew when a third of them are
+    // out of work, where a launch takes far longer than its overhead, or
+    // (hodlr_set_aca_streaming(1), the same bits of epsilon every time) when a block
+    // has the rank that was expected of it; in a forest first at a fifth of that,
+    // which is the largest system's.  ACA in ms, fixed shares | by the clock | at column
+    // counts: 2D N = 262144 131 | 111 | 117, sphere 16384 107.8 | 107.3 | 109.6, sphere
+    // 65536 - | 373 | 400 (with a rank model 427), cube 40000 92.7 | 87.8 | 88.9, forest
+    // of 40 - | 54.1 | 53.8.
+    const bool share = variant && jobs.size() > 1 && slowest > 2000.0;
+    const int yield_at = share && !h->aca_by_count ? std::max(1, most / 3) : 0;
+    if (share && h->aca_by_count)
+      for (size_t i = 0; i < jobs.size(); ++i)
+        bl[i].kstop = (int)std::max(jobs[i].k0 + 24.0,
+                                    h->nsys && jobs[i].k0 == 0.0 ? 0.2 * jobs[i].k : jobs[i].k);
     h->pool.scratch_busy = variant != ACA_GROUP_NONE;
     const int rc = run_aca(h, bl, 1, any ? 256 : 128, kcap_max, variant, &groups, yield_at);
     h->pool.scratch_busy = false;
@@ -566,7 +577,7 @@ static int compress_levels(hodlr_t h) {
     if (all) break;
   }
   // 2. the few-block levels, in sets of neighbouring levels, deepest first:
-  // the blocks of a set run in one launch (group_sets)
+  // the blocks of a set run in one launch (group_set_top)
   std::vector<double> rank_est((size_t)nlev, 0.0);
   double growth = 1.0;  // of the rank from one level to the next above it
   int known = -1;       // the uppermost level compressed so far

@@ -353,6 +353,7 @@ int init_common(hodlr_t h) {
   const char* acs = getenv("HODLR_ACA_STREAMING");
   if (acs && acs[0] >= '0' && acs[0] <= '2' && acs[1] == 0) {
     h->aca_ring = acs[0] != '0';
+    h->aca_by_count = acs[0] == '1';
   }
   // HODLR_CAPACITANCE_SMEM=bytes: shared memory a CTA of a capacitance solve may
   // use in new handles; systems beyond it run from device memory

@@ -288,6 +288,7 @@ struct hodlr_handle_s {
   // aca_kernel (panels loaded per thread), the same bits
   bool aca_ring = true;
   bool aca_ring_fits = true;  // in memory, as far as this compression knows
+  bool aca_by_count = false;  // blocks pause at column counts, not by the clock
   // factorization form (hodlr_set_solver_form): false recLU's Schur systems
   // [bottom; top], true recSM's perturbI systems [top; bottom]
   bool sm_form = false;

@@ -517,6 +517,7 @@ int hodlr_set_checked(hodlr_t h, int on) {
 int hodlr_set_aca_streaming(hodlr_t h, int on) {
   if (!h || on < 0 || on > 2) return HODLR_ERR_ARG;
   h->aca_ring = on != 0;
+  h->aca_by_count = on == 1;
   return HODLR_OK;
 }
 

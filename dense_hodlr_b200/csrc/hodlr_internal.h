@@ -45,6 +45,7 @@ struct AcaBlock {
   int* pcol;          // pivot column of step t
   int r0, c0, m, n;
   int kcap;           // columns available in W and V
+  int kstop;          // aca_group_kernel: columns at which the block pauses
   int level;
   int g0, G;          // with a CTA table: first CTA of this block's group, group size
   // aca_group_kernel: the block's slices of W and V in the launch's working

@@ -198,7 +198,8 @@ class HODLR_Matrix:
 
     def set_aca_streaming(self, on):
         """Top-level ACA panels through the CTAs' shared-memory rings (2, default,
-        or 1), or loaded per thread (0).  Same results in every mode."""
+        or 1), or loaded per thread (0).  Same results in every mode; in mode 1 the
+        stopping test's epsilons have the same last bits in every run too."""
         _check(self._h, _L.lib().hodlr_set_aca_streaming(self._h, int(on)))
 
     def set_factor_in_place(self, mode):

@@ -359,8 +359,13 @@ int hodlr_get_memory_held(hodlr_t h, long long* bytes);
  * a shared-memory ring per CTA, one bulk copy per tile; 0 loads the panels per
  * thread, and so does a compression that does not fit beside the rings' buffers.
  * Measured ACA time, streamed / per thread: 0.015 / 0.090 s (2D Matern cloud,
- * N = 20011, tol 1e-8), 0.117 / 0.260 s (N = 262144).  Pivots, ranks and W/V are the same in every mode; the
- * setting applies from the next compression.  HODLR_ACA_STREAMING=0, 1 or 2
+ * N = 20011, tol 1e-8), 0.111 / 0.260 s (N = 262144).  Pivots, ranks and W/V are
+ * the same in every mode.  In long compressions blocks pause to have the CTAs
+ * shared anew, which regroups the sums of the stopping test: mode 2 pauses by the
+ * clock, so the last bits of an epsilon (hodlr_get_block_margin) differ from run
+ * to run, and a rank can where epsilon is within rounding of the tolerance; mode 1
+ * pauses at column counts and gives the same bits every time (0 to 14% slower).
+ * The setting applies from the next compression.  HODLR_ACA_STREAMING=0, 1 or 2
  * in the environment sets the mode of every new handle. */
 int hodlr_set_aca_streaming(hodlr_t h, int on);
 
