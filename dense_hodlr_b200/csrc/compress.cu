@@ -617,9 +617,6 @@ static int compress_levels(hodlr_t h) {
     }
     for (auto it = set.rbegin(); it != set.rend(); ++it) note_rank(*it);
   }
-  // back to the device pool, not to the handle's cache: the factorization's
-  // panels are cut from it next
-  h->pool.free_scratch(h->stream);
   for (auto& L : h->lv)
     if (!level_done(L)) return fail(h, HODLR_ERR_STATE, "ACA did not converge in its launches");
   // ranks, level widths, column offsets, algorithmic bytes

@@ -189,7 +189,10 @@ struct DevPool {
     return e;
   }
   // One buffer whose contents nobody keeps: given back when anything else does
-  // not fit, except while a launch uses it (scratch_busy).
+  // not fit, except while a launch uses it (scratch_busy).  It stays for the next
+  // compression: taken from the device pool and returned every time, gigabytes were
+  // mapped anew whenever the pool's free memory lay in pieces (3 ms for 3 GB, and up
+  // to a second beside a process that polls the device).
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
   bool scratch_busy = false;
