@@ -320,8 +320,8 @@ __device__ __noinline__ void substitute_block(const double* ts, int dir, int m,
 // warp, refines it where the triangle asks for that, and writes it to every CTA's
 // xb[b mod 3]; all subtract A(b', b) x_b from their blocks still to be solved.
 // xb[3] and the triangle at `ts` are the refinement's, and xb[b mod 3] before x_b is
-// there; the triangle is copied a step ahead (from L2 or memory inside the chain a refined step took 4 us, not
-// 2), and not in registers, which doubled (120 -> 255).
+// there; the triangle is copied into shared memory a step ahead, not held in
+// registers, which doubled (120 -> 255).
 //
 // The chain is wait, update of the next block, its product, write: the owner
 // of the next step does those first and everybody else's updates overlap it.

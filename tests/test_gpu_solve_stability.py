@@ -3,10 +3,10 @@
 The triangles of the stored LUs are applied as inverses, refined by their
 condition; the residual on the compressed operator is compared with that of the
 CPU oracle, which substitutes, both over the norms of their solutions (backward
-errors: at a shift of 1e-12 the solutions have few digits in common).  Unrefined inverses left 1e1 (shift 1e-2) to 1e6
-times the oracle's (shift 1e-8).  By the rule of the kernels a block step leaves
-1 to 2 times a substitution's residual; 3 allows for the scatter of residuals of
-24 random columns.
+errors: at a shift of 1e-12 the solutions have few digits in common).  Unrefined
+inverses left 1.3 to 112 times the oracle's.  By the rule of the kernels a block
+step leaves at most 1.4 times a substitution's residual; 3 allows for the scatter
+of residuals of 24 random columns.
 """
 import numpy as np
 import pytest
